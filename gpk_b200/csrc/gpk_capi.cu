@@ -586,6 +586,7 @@ int gpk_grid_graph_prepare(gpk_grid* G, double dt, double dt_cap) {
     const std::vector<uint64_t> sig = graph_signature(G, dt, dt_cap);
     if (G->step_graph && sig == G->graph_sig) return GPK_OK;
     gpk_grid_graph_release(G);
+    GPK_TRY(G->precision == GPK_PREC_F64 ? gpk_geometry_items_init<double>(G) : gpk_geometry_items_init<float>(G));
     GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
     const uint64_t step0 = G->step_id, launches0 = G->launches;
     GPK_CUDA_TRY(cudaStreamBeginCapture(G->stream, cudaStreamCaptureModeThreadLocal));

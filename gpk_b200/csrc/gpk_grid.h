@@ -99,6 +99,13 @@ struct gpk_grid {
     // remap screening: weight sums of the 128 patterns of a 7-tap row, for the
     // ten distinct dy^2 + dz^2 of a 7 x 7 row block (radius 3 only)
     double* d_remap_rtab = nullptr;
+    // direct geometry (gpk_geometry_items.cu): packed tap table, items of 64
+    // interface cells, bitmap pool
+    void* d_geom_packed = nullptr;
+    int32_t* item_word = nullptr; int32_t* item_cell = nullptr;
+    uint32_t* item_support = nullptr; uint32_t* item_words = nullptr;
+    unsigned item_pool = 0;
+    unsigned* item_counters = nullptr;
     gpk_dev::StepScalars* scal = nullptr;  // device scalars
     gpk_dev::StepScalars* h_scal = nullptr;  // pinned host mirror
     void* host_kernels = nullptr;          // HostKernels<real>*
@@ -107,11 +114,11 @@ struct gpk_grid {
     // waves of the crossing sweeps, waves of the remap exchange loops,
     // crossing candidates, remap proposals (summed since last read)
     uint64_t wave_stats[4] = {};
-    // rows of a 2-D geometry tile at kernel radius 8 divided by 1, 2 or 4
-    // (1024, 512 or 256 cells; gpk_grid_set_tile_rows)
+    // rows of a 2-D geometry tile at kernel radius 8: 32 divided by 1, 2 or 4
+    // (gpk_grid_set_tile_rows)
     int tile_rows_div = 1;
-    // geometry kernel choice: 0 = tiled (per-cell kernel where no tiled
-    // instantiation exists), 1 = per-cell kernel
+    // geometry kernel choice: 0 = items (per-cell kernel where no item
+    // instantiation exists), 1 = per-cell kernel (gpk_grid_set_geometry_kernel)
     int geometry_kernel = 0;
     // E_el supplied by the caller (gpk_grid_set_external_elastic)
     int external_elastic = 0;
@@ -152,7 +159,8 @@ template <typename real> int gpk_interface_mask(gpk_grid* G, const unsigned long
 template <typename real> int gpk_max_dt_impl(gpk_grid* G, double* out);
 template <typename real> int gpk_phase_volume_impl(gpk_grid* G, int32_t label, double* out);
 template <typename real>
-int gpk_geometry_tiled(gpk_grid* G, int R, real inv_dx, real inv_dx2, real dx, real kappa_limit);
+int gpk_geometry_items(gpk_grid* G, int R, real inv_dx, real inv_dx2, real dx, real kappa_limit);
+template <typename real> int gpk_geometry_items_init(gpk_grid* G);
 // FP64 separable tiles (throughput geometry); -1 when they do not apply
 int gpk_geometry_sep_tiles(gpk_grid* G, int R, const double* gauss, int gauss_radius, double dx,
                            double kappa_limit);

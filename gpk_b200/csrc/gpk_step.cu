@@ -30,12 +30,16 @@ static constexpr int MASK_TPB = 256;
 static constexpr int MASK_IPT = 8;
 static constexpr int MASK_TILE = MASK_TPB * MASK_IPT;
 
+// `item_counters` (may be null): the three counters of the geometry's items,
+// cleared here for the geometry that follows.
 // `gate` (may be null): when it points to zero the launch does nothing
 // (device-side skip of a stage inside a captured step)
 __global__ void __launch_bounds__(MASK_TPB) k_mask_tiles(Dims D, const int32_t* __restrict__ phi,
                                                          uint8_t* __restrict__ mask, int32_t* __restrict__ tile_cnt,
+                                                         unsigned* __restrict__ item_counters,
                                                          const unsigned long long* gate = nullptr) {
     if (gate && *gate == 0ull) return;
+    if (blockIdx.x == 0 && threadIdx.x < 3 && item_counters) item_counters[threadIdx.x] = 0u;
     typedef cub::BlockReduce<int, MASK_TPB> BR;
     __shared__ typename BR::TempStorage tmp;
     const int base = blockIdx.x * MASK_TILE;
@@ -62,8 +66,10 @@ __global__ void __launch_bounds__(MASK_TPB) k_mask_tiles(Dims D, const int32_t* 
 // loads for the x neighbours of the group's ends) and stores four flags at once.
 __global__ void __launch_bounds__(MASK_TPB) k_mask_tiles4(Dims D, const int32_t* __restrict__ phi,
                                                           uint8_t* __restrict__ mask, int32_t* __restrict__ tile_cnt,
-                                                          const unsigned long long* gate = nullptr) {
+                                                          unsigned* __restrict__ item_counters,
+                                                         const unsigned long long* gate = nullptr) {
     if (gate && *gate == 0ull) return;
+    if (blockIdx.x == 0 && threadIdx.x < 3 && item_counters) item_counters[threadIdx.x] = 0u;
     typedef cub::BlockReduce<int, MASK_TPB> BR;
     __shared__ typename BR::TempStorage tmp;
     const int nx4 = D.Nx >> 2, plane = D.Nx * D.Ny;
@@ -1480,9 +1486,9 @@ template <typename real>
 int gpk_interface_mask(gpk_grid* G, const unsigned long long* gate) {
     const int nt = (G->d.N + MASK_TILE - 1) / MASK_TILE;
     if (G->d.Nx % 4 == 0)
-        k_mask_tiles4<<<nt, MASK_TPB, 0, G->stream>>>(G->d, G->phi, G->mask, G->tile_off, gate);
+        k_mask_tiles4<<<nt, MASK_TPB, 0, G->stream>>>(G->d, G->phi, G->mask, G->tile_off, G->item_counters, gate);
     else
-        k_mask_tiles<<<nt, MASK_TPB, 0, G->stream>>>(G->d, G->phi, G->mask, G->tile_off, gate);
+        k_mask_tiles<<<nt, MASK_TPB, 0, G->stream>>>(G->d, G->phi, G->mask, G->tile_off, G->item_counters, gate);
     k_scan_tiles<<<1, 1024, 0, G->stream>>>(G->tile_off, nt, &G->scal->n_active, gate);
     k_compact_u8<<<nt, MASK_TPB, 0, G->stream>>>(G->d.N, G->mask, G->tile_off, G->active, gate);
     G->launches += 3;
@@ -1514,7 +1520,7 @@ static int geometry(gpk_grid* G) {
             }
         }
         if (G->geometry_kernel != 1) {
-            const int rc = gpk_geometry_tiled<real>(G, hk->geom_radius, inv_dx, inv_dx2, dx, kappa_limit);
+            const int rc = gpk_geometry_items<real>(G, hk->geom_radius, inv_dx, inv_dx2, dx, kappa_limit);
             if (rc != -1) return rc;
         }
         const int grid = G->num_sms * 16;

@@ -248,9 +248,9 @@ int gpk_grid_stage_times(gpk_grid* grid, double ms[GPK_NUM_STAGES], uint64_t cal
 int gpk_grid_wave_stats(gpk_grid* grid, uint64_t out[10]);
 /* Kernel selection (all give identical results): 0 = tiled shared-memory
  * kernels where an instantiation exists (default), 1 = the per-interface-
- * cell kernels, 2 = tiled kernels with one label per geometry bitmap batch
- * (exercises the many-label path of the tiled geometry kernel; the remap
- * scores then skip their bitmap screening), 3 = tiled kernels with every
+ * cell kernels, 2 = tiled kernels without label bitmaps in the geometry
+ * (exercises its path for tiles with more labels than the bitmap pool holds;
+ * the remap scores then skip their bitmap screening), 3 = tiled kernels with every
  * remap score summed tap by tap (no screening) and the pair-compare
  * projection tiles.  4 = separable tiles, FP64 grids only (the throughput
  * geometry): the reference's separable geometry (src/gpk_geometry.cpp:
@@ -308,8 +308,7 @@ int gpk_grid_set_solid_diffusivity_ratio(gpk_grid* grid, double ratio);
  * gpk_grid_step_graph returns GPK_ERR_UNSUPPORTED_MODEL otherwise.       */
 int gpk_grid_step_graph(gpk_grid* grid, int n, double dt, double dt_cap, double* time_out);
 /* Height of the 2-D geometry tiles at kernel radius 8 (sigma 1.5): the
- * 1024-cell tile's rows divided by 1, 2 or 4 (1024, 512 or 256 cells per
- * CTA).  Results do not depend on it; small grids get more CTAs from
+ * tile's 32 rows divided by 1, 2 or 4 (512, 256 or 128 cells per CTA).  Results do not depend on it; small grids get more CTAs from
  * smaller tiles.  gpk_batch_autotune_tiles picks it per instance size.     */
 int gpk_grid_set_tile_rows(gpk_grid* grid, int divisor);
 int gpk_grid_graph_supported(gpk_grid* grid, int* supported);
