@@ -203,56 +203,167 @@ __device__ __forceinline__ bool bounded_branches_connected(const Dims& D, const 
     return true;
 }
 
-// The same two tests from a 5^d occupancy mask already gathered (bit
-// b = lz*25 + ly*5 + lx, lz = 0 in 2-D): the topological number of the inner
-// 3^d box (centre removed) and the bounded branch connectivity.
-__device__ __forceinline__ int topological_number_mask(u128 occ5, bool is3d) {
-    uint32_t occ = 0;
-    const int lzn = is3d ? 3 : 1;
-    for (int lz = 0; lz < lzn; ++lz)
-        for (int ly = 0; ly < 3; ++ly)
-            for (int lx = 0; lx < 3; ++lx) {
-                const int b5 = (is3d ? (lz + 1) * 25 : 0) + (ly + 1) * 5 + lx + 1;
-                occ |= (uint32_t)((occ5 >> b5) & 1) << (lz * 9 + ly * 3 + lx);
-            }
-    occ &= ~(1u << (is3d ? 13 : 4));
-    return count_face_components(occ, is3d);
-}
-
-__device__ __forceinline__ bool bounded_branches_connected_mask(u128 occ, bool is3d, bool exclude_centre) {
-    const int centre = (is3d ? 2 * 25 : 0) + 12;
-    u128 lx0 = 0, lx4 = 0, ly0 = 0, ly4 = 0;
-    const int zcount = is3d ? 5 : 1;
-    for (int lz = 0; lz < zcount; ++lz)
-        for (int l = 0; l < 5; ++l) {
-            lx0 |= bit128(lz * 25 + l * 5);
-            lx4 |= bit128(lz * 25 + l * 5 + 4);
-            ly0 |= bit128(lz * 25 + l);
-            ly4 |= bit128(lz * 25 + 20 + l);
+// The same two tests from a 5^d occupancy mask already gathered as ballots
+// (bit b = lz*25 + ly*5 + lx, lz = 0 in 2-D): the topological number of the
+// inner 3^d box (centre removed) and the bounded branch connectivity.  The
+// mask is held as planes of 25 bits, all shifts and masks compile-time
+// constants (with the dimension a run-time value, 128-bit shifts in loops took
+// a lane thousands of cycles).
+template <bool IS3D>
+struct Box5 {
+    static constexpr int NP = IS3D ? 5 : 1, PC = IS3D ? 2 : 0;
+    static constexpr uint32_t ALL = 0x1FFFFFFu, X0 = 0x108421u, X4 = X0 << 4, CENTRE = 1u << 12;
+    uint32_t p[NP];
+    __device__ __forceinline__ explicit Box5(const uint32_t (&w)[4]) {
+        p[0] = w[0] & ALL;
+        if (IS3D) {
+            p[1] = __funnelshift_r(w[0], w[1], 25) & ALL;
+            p[2] = __funnelshift_r(w[1], w[2], 18) & ALL;
+            p[3] = __funnelshift_r(w[2], w[3], 11) & ALL;
+            p[4] = (w[3] >> 4) & ALL;
         }
-    if (exclude_centre) occ &= ~bit128(centre);
-    const int branch_bit[6] = {centre - 1, centre + 1, centre - 5, centre + 5, centre - 25, centre + 25};
-    const int nf = is3d ? 6 : 4;
-    int branches[6], nb = 0;
-    for (int k = 0; k < nf; ++k)
-        if (occ & bit128(branch_bit[k])) branches[nb++] = branch_bit[k];
-    if (nb <= 1) return true;
-    const u128 all = is3d ? ((((u128)1) << 125) - 1) : ((((u128)1) << 25) - 1);
-    u128 comp = bit128(branches[0]);
-    for (;;) {
-        u128 r = comp;
-        r |= (comp << 1) & ~lx0;
-        r |= (comp >> 1) & ~lx4;
-        r |= (comp << 5) & ~ly0;
-        r |= (comp >> 5) & ~ly4;
-        if (is3d) { r |= (comp << 25); r |= (comp >> 25); }
-        r &= all & occ;
-        if (r == comp) break;
-        comp = r;
     }
-    for (int k = 1; k < nb; ++k)
-        if (!(comp & bit128(branches[k]))) return false;
-    return true;
+    __device__ __forceinline__ int topological_number() const {
+        auto inner = [](uint32_t q) { return ((q >> 6) & 7u) | (((q >> 11) & 7u) << 3) | (((q >> 16) & 7u) << 6); };
+        uint32_t occ = IS3D ? inner(p[1]) | (inner(p[PC]) << 9) | (inner(p[NP - 2]) << 18) : inner(p[0]);
+        occ &= ~(1u << (IS3D ? 13 : 4));
+        return count_face_components(occ, IS3D);
+    }
+    __device__ __forceinline__ bool branches_connected(bool exclude_centre) const {
+        uint32_t o[NP], c[NP], b[NP];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            o[q] = q == PC && exclude_centre ? p[q] & ~CENTRE : p[q];
+            b[q] = q == PC ? o[q] & ((CENTRE << 1) | (CENTRE >> 1) | (CENTRE << 5) | (CENTRE >> 5))
+                           : (q == PC - 1 || q == PC + 1 ? o[q] & CENTRE : 0u);
+            c[q] = 0u;
+        }
+        // from the first branch; connected when it reaches the others
+        bool seeded = false;
+#pragma unroll
+        for (int q = 0; q < NP; ++q)
+            if (!seeded && b[q]) {
+                c[q] = b[q] & (0u - b[q]);
+                seeded = true;
+            }
+        if (!seeded) return true;
+        uint32_t changed;
+        do {
+            changed = 0u;
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+                uint32_t r = c[q] | ((c[q] << 1) & ~X0) | ((c[q] >> 1) & ~X4) | (c[q] << 5) | (c[q] >> 5);
+                if (q > 0) r |= c[q - 1];
+                if (q + 1 < NP) r |= c[q + 1];
+                r &= o[q];
+                changed |= r ^ c[q];
+                c[q] = r;
+            }
+        } while (changed);
+        uint32_t missed = 0u;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) missed |= b[q] & ~c[q];
+        return missed == 0u;
+    }
+};
+
+// Are the cell's branches of `label` connected (a warp's work; labels in the
+// serial-time view)?  1 yes, 0 no, -1 when the window around the cell does
+// not tell: 9^3 cells (27 lanes hold three rows of nine bits each) or 15^2
+// (15 lanes, a row each).  Branches united inside the window are connected; a
+// branch whose part of the window reaches no window border is a component of
+// its own.  The flood fill visits 7 (2-D) to 12 cells on average, so the
+// window nearly always tells (512^2: 675 -> 29 cells filled a step); the
+// fill's rounds are four dependent loads and an exchange each, 34 k cycles for
+// a wave's slowest where the window's two rounds of loads leave 18 k.
+template <bool IS3D>
+__device__ int window_connected(const Dims& D, const SerialView& v, int cell, int32_t label, bool exclude_centre) {
+    constexpr int E = IS3D ? 9 : 15, H = E / 2;
+    if (D.Nx < E || D.Ny < E || (IS3D && D.Nz < E)) return -1;
+    const int lane = threadIdx.x & 31;
+    int z0, y0, x0;
+    D.decode(cell, z0, y0, x0);
+    uint32_t occ = 0, branch = 0, border = 0;
+    if (IS3D) {
+        const int wz = lane / 3, wy = 3 * (lane % 3);
+        if (lane < 27) {
+            const int z = wrap1(z0 + wz - H, D.Nz);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const int row = (z * D.Ny + wrap1(y0 + wy + r - H, D.Ny)) * D.Nx;
+                int c[9], q[9];
+#pragma unroll
+                for (int e = 0; e < 9; ++e) {
+                    const int j = row + wrap1(x0 + e - H, D.Nx);
+                    c[e] = v.cmap[j];
+                    q[e] = v.phi[j];
+                }
+#pragma unroll
+                for (int e = 0; e < 9; ++e) {
+                    if (c[e] > v.k && v.cres[c[e]] == 2) q[e] = v.cinfo[c[e]].y;
+                    occ |= (uint32_t)(q[e] == label) << (9 * r + e);
+                }
+            }
+            constexpr uint32_t X0 = 0x40201u, X8 = X0 << 8;
+            border = wz == 0 || wz == 8 ? 0x7FFFFFFu : (X0 | X8 | (wy == 0 ? 0x1FFu : 0u) | (wy == 6 ? 0x1FFu << 18 : 0u));
+            if (exclude_centre && lane == 13) occ &= ~(1u << 13);
+            if (lane == 13) branch = occ & ((1u << 12) | (1u << 14) | (1u << 4) | (1u << 22));
+            if (lane == 10 || lane == 16) branch = occ & (1u << 13);
+        }
+    } else {
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            // two rows at a time, a half warp each
+            const int r = 2 * it + (lane >> 4), e = lane & 15;
+            bool hit = false;
+            if (r < E && e < E) {
+                const int j = wrap1(y0 + r - H, D.Ny) * D.Nx + wrap1(x0 + e - H, D.Nx);
+                const int c = v.cmap[j];
+                int32_t q = v.phi[j];
+                if (c > v.k && v.cres[c] == 2) q = v.cinfo[c].y;
+                hit = q == label;
+            }
+            const uint32_t b = __ballot_sync(0xffffffffu, hit);
+            if (lane == 2 * it) occ = b & 0x7FFFu;
+            if (lane == 2 * it + 1) occ = b >> 16;
+        }
+        border = lane == 0 || lane == E - 1 ? 0x7FFFu : 0x4001u;
+        if (exclude_centre && lane == H) occ &= ~(1u << H);
+        if (lane == H) branch = occ & ((1u << (H - 1)) | (1u << (H + 1)));
+        if (lane == H - 1 || lane == H + 1) branch = occ & (1u << H);
+    }
+    bool first = true, open = false;
+    for (;;) {
+        const unsigned have = __ballot_sync(0xffffffffu, branch != 0u);
+        if (have == 0u) break;
+        uint32_t m = lane == __ffs(have) - 1 ? branch & (0u - branch) : 0u;
+        for (;;) {
+            uint32_t n;
+            if (IS3D) {
+                constexpr uint32_t X0 = 0x40201u, X8 = X0 << 8;
+                const uint32_t ym = __shfl_up_sync(0xffffffffu, m, 1), yp = __shfl_down_sync(0xffffffffu, m, 1);
+                const uint32_t zm = __shfl_up_sync(0xffffffffu, m, 3), zp = __shfl_down_sync(0xffffffffu, m, 3);
+                n = m | ((m << 1) & ~X0) | ((m >> 1) & ~X8) | (m << 9) | (m >> 9);
+                if (lane % 3 != 0) n |= ym >> 18;
+                if (lane % 3 != 2) n |= yp << 18;
+                if (lane >= 3) n |= zm;
+                if (lane < 24) n |= zp;
+            } else {
+                const uint32_t ym = __shfl_up_sync(0xffffffffu, m, 1), yp = __shfl_down_sync(0xffffffffu, m, 1);
+                n = m | (m << 1) | (m >> 1) | (lane > 0 ? ym : 0u) | (lane < 31 ? yp : 0u);
+            }
+            n &= occ;
+            if (!__any_sync(0xffffffffu, n != m)) break;
+            m = n;
+        }
+        branch &= ~m;
+        const bool all = !__any_sync(0xffffffffu, branch != 0u);
+        if (first && all) return 1;
+        if (!__any_sync(0xffffffffu, (m & border) != 0u)) return 0;
+        open = true;
+        first = false;
+    }
+    return open ? -1 : 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -601,126 +712,258 @@ __device__ bool warp_branches_connected_ms(const Dims& D, const Lab& lab, int ce
     return single;
 }
 
-template <typename real>
-__global__ void __launch_bounds__(256) k_crossing_sweep(CrossArgs a, int m, int max_waves) {
+// Threads of a sweep's block, and the pending candidates from which on one
+// block goes on alone: its barriers cost tens of nanoseconds instead of the
+// microseconds of a grid barrier, and its reads hit its own L1.  Most waves of
+// a sweep hold few candidates (2-D 512^2: 290 in 9 waves; 128^3 at sigma 5:
+// 250 in 18).  Crossing stage with this and the window test: 512^2 254 -> 112
+// us a step, 128^3 sigma 5 193 -> 137, 96^3 539 -> 357, 256^3 1262 -> 1012.
+// 512 threads: with 1024 the window's loads spill (256^3 1243).
+static constexpr int CROSS_TPB = 512, CROSS_SOLO = 128;
+
+template <typename real, bool is3d>
+__global__ void __launch_bounds__(CROSS_TPB, 1) k_crossing_sweep(CrossArgs a, int m, int max_waves, int solo_max) {
     const int nblocks = gridDim.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = nblocks * blockDim.x;
     const Dims D = a.D;
-    const bool is3d = D.is3d();
+    constexpr int nbox = is3d ? 125 : 25, centre = is3d ? 62 : 12;
     unsigned* rem = a.s->wave_rem;  // three rotating counters
     unsigned prev_left = (unsigned)m + 1u;  // pending counts at wave starts: m, then strictly fewer
+    // the one block's own lists
+    __shared__ int s_list[2][CROSS_SOLO], s_tasks[CROSS_SOLO];
+    __shared__ unsigned s_pending, s_n, s_ntask;
+    bool solo = false;
+    int cur = 0;
+    auto barrier = [&]() -> bool {
+        if (solo) {
+            __syncthreads();
+            return true;
+        }
+        return grid_barrier(a.s, nblocks);
+    };
+    // Phase A of candidate k (one warp): locality, local certificate parts,
+    // label-wide needs; earliest pending candidate touching each label.  The
+    // lanes read the 5^d box around its cell at once (labels in the
+    // serial-time view, and the earlier pending candidates there), and ballots
+    // give the occupancy masks of its old and new label.
+    auto phase_a = [&](int k, int32_t* minA, int32_t* minN) {
+        const int4 ci = a.cinfo[k];
+        if (lane == 0) {
+            atomicMin(&minA[ci.y], k);
+            atomicMin(&minA[ci.z], k);
+            minN[ci.y] = INT_BIG;
+            minN[ci.z] = INT_BIG;
+        }
+        int z0, y0, x0;
+        D.decode(ci.x, z0, y0, x0);
+        // the box in three rounds of loads: cell indices, then labels
+        // and candidate slots, then the candidates' states
+        int jq[4], cq4[4];
+        int32_t lq[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int e = q * 32 + lane;
+            jq[q] = -1;
+            if (e < nbox && (q == 0 || nbox > 32)) {
+                const int lz = e / 25, ly = (e / 5) % 5, lx = e % 5;
+                // offsets of at most 2: one period at extents of 3 or more
+                const int zz = !is3d ? z0 : (D.Nz >= 3 ? wrap1(z0 + lz - 2, D.Nz) : wrap_any(z0 + lz - 2, D.Nz));
+                const int yy = D.Ny >= 3 ? wrap1(y0 + ly - 2, D.Ny) : wrap_any(y0 + ly - 2, D.Ny);
+                const int xx = D.Nx >= 3 ? wrap1(x0 + lx - 2, D.Nx) : wrap_any(x0 + lx - 2, D.Nx);
+                jq[q] = D.idx(zz, yy, xx);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            cq4[q] = jq[q] >= 0 ? a.cmap[jq[q]] : -1;
+            lq[q] = jq[q] >= 0 ? a.phi[jq[q]] : -1;
+        }
+        bool conflict = false;
+        uint32_t wo[4] = {0u, 0u, 0u, 0u}, wn[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int e = q * 32 + lane;
+            const int c = cq4[q];
+            int32_t lbl = lq[q];
+            if (c > k) {
+                if (a.cres[c] == 2) lbl = a.cinfo[c].y;  // accepted later: the old label
+            } else if (c >= 0 && c < k && e != centre && a.cres[c] == 0) {
+                const int4 cq = a.cinfo[c];
+                conflict |= cq.y == ci.y || cq.y == ci.z || cq.z == ci.y || cq.z == ci.z;
+            }
+            wo[q] = __ballot_sync(0xffffffffu, lbl == ci.y);
+            wn[q] = __ballot_sync(0xffffffffu, lbl == ci.z);
+            if (nbox <= 32) break;
+        }
+        const bool local = !__any_sync(0xffffffffu, conflict);
+        // lane 0 takes the old label's topology, lane 1 the new one's
+        // (the same code on two masks runs side by side)
+        int part = 0;
+        if (local && lane < 2) {
+            uint32_t wv[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) wv[q] = lane == 0 ? wo[q] : wn[q];
+            const Box5<is3d> box(wv);
+            const int tv = box.topological_number();
+            part = min(tv, 2);
+            if (tv > 1) part |= box.branches_connected(lane == 0) ? 4 : 8;
+        }
+        const int part_n = __shfl_sync(0xffffffffu, part, 1);
+        if (lane == 0) {
+            int st = 0;
+            if (local) {
+                const int to = part & 3, tn = part_n & 3;
+                st = CS_LOCAL | (to << CS_TO_SHIFT) | (tn << CS_TN_SHIFT);
+                if (to == 0) {
+                    // at k's serial time the label holds at least count0 - (its other candidates) cells
+                    if (a.count0[ci.y] - (a.n_old[ci.y] - 1) >= 2) st |= CS_CNT_REJECT;
+                    else st |= CS_GC;
+                } else if (to > 1) {
+                    st |= (part & 4) ? CS_OLD_LOCAL : CS_GO;
+                }
+                if (tn > 1) st |= (part_n & 4) ? CS_NEW_LOCAL : CS_GN;
+            }
+            a.cinfo[k].w = st;
+        }
+    };
+    // Phase B of candidate k (one thread): readiness; decisions that need only
+    // local reads are committed at once (they depend on nothing another
+    // decision of this wave writes: their local reads hold no earlier pending
+    // candidate, and later ones read back through the serial view).  True
+    // when it needs label-wide work.
+    auto phase_b = [&](int k, const int32_t* minA) -> bool {
+        const int4 ci = a.cinfo[k];
+        const int st = ci.w;
+        if (!(st & CS_LOCAL)) return false;
+        if ((st & (CS_GO | CS_GC)) && minA[ci.y] < k) return false;
+        if ((st & CS_GN) && minA[ci.z] < k) return false;
+        if (st & (CS_GO | CS_GN | CS_GC)) return true;
+        const int to = (st >> CS_TO_SHIFT) & 3, tn = (st >> CS_TN_SHIFT) & 3;
+        // to == 0 without GC is CS_CNT_REJECT; to > 1 without GO passed the 5^d proof
+        bool acc = to != 0;
+        if (acc && tn == 0) acc = false;
+        cross_commit<real>(a, k, ci, acc);
+        return false;
+    };
+    // Phase B2 of candidate k (one warp): global flood fills and exact counts
+    auto phase_b2 = [&](int k) {
+        const int4 ci = a.cinfo[k];
+        const int st = ci.w;
+        const SerialView view{a.phi, a.cmap, a.cres, a.cinfo, k};
+        const int to = (st >> CS_TO_SHIFT) & 3, tn = (st >> CS_TN_SHIFT) & 3;
+        int base = 0, cap = 0;
+        uint32_t my_stamp = 0;
+        int visited = 0;
+        // are the label's branches connected: the window around the cell, else
+        // the flood fill, whose queue is requested once
+        auto connected = [&](int32_t label, bool old_label) -> bool {
+            const int win = window_connected<is3d>(D, view, ci.x, label, old_label);
+            if (win >= 0) return win != 0;
+            if (cap == 0) {
+                // the view of a label holds at most its count plus its later candidates' cells
+                cap = max((st & CS_GO) ? a.count[ci.y] + a.n_old[ci.y] : 0,
+                          (st & CS_GN) ? a.count[ci.z] + a.n_old[ci.z] : 0) + 1;
+                if (lane == 0) {
+                    // queue of cap cells plus cap search ids; 8 stamps per flood fill
+                    base = (int)atomicAdd(&a.s->ff_pool, (unsigned)(2 * cap));
+                    my_stamp = atomicAdd(&a.s->stamp, 16u) + 1u;
+                }
+                base = __shfl_sync(0xffffffffu, base, 0);
+                my_stamp = __shfl_sync(0xffffffffu, my_stamp, 0);
+                if ((long long)base + 2 * cap > a.pool_size) {
+                    if (lane == 0) atomicCAS(&a.s->error, 0u, (unsigned)GPK_ERR_INTERNAL);
+                    cap = 0;
+                    base = 0;
+                }
+            }
+            int vis = 0;
+            const bool r = warp_branches_connected_ms(D, view, ci.x, label, old_label, a.stamp, a.stamp_rev,
+                                                      a.ff_stack + base, cap, my_stamp + (old_label ? 0u : 8u),
+                                                      &a.s->error, vis);
+            visited += vis;
+            return r;
+        };
+        bool acc = true;
+        if (to == 0) {
+            if (st & CS_CNT_REJECT) acc = false;
+            else {
+                acc = warp_serial_count(a, k, ci.y) <= 1;
+                if (lane == 0) {
+                    atomicAdd(&a.s->count_tasks, 1ull);
+                    atomicAdd(&a.s->count_scanned, (unsigned long long)k);
+                }
+            }
+        } else if (to > 1 && !(st & CS_OLD_LOCAL)) {
+            acc = connected(ci.y, true);
+        }
+        if (acc) {
+            if (tn == 0) acc = false;
+            else if (tn > 1 && !(st & CS_NEW_LOCAL)) acc = connected(ci.z, false);
+        }
+        if (lane == 0) {
+            a.cinfo[k].w = st | CS_READY | (acc ? CS_ACCEPT : 0);
+            if (st & (CS_GO | CS_GN)) {
+                atomicAdd(&a.s->flood_tasks, 1ull);
+                if (visited) atomicAdd(&a.s->flood_cells, (unsigned long long)visited);
+            }
+        }
+    };
+    if (m <= solo_max) {
+        // (a grid of one block)
+        solo = true;
+        if (threadIdx.x < m) s_list[0][threadIdx.x] = threadIdx.x;
+        if (threadIdx.x == 0) s_n = m;
+        __syncthreads();
+    }
     for (int w = 0; w < max_waves; ++w) {
-        // ---- phase A: locality, local certificate parts, label-wide needs;
-        //      earliest pending candidate touching each label.  One warp per
-        //      pending candidate: the lanes read the 5^d box around its cell
-        //      at once (labels in the serial-time view, and the earlier
-        //      pending candidates there), and ballots give the occupancy
-        //      masks of its old and new label.
         int32_t* minA = a.minL[w & 1];        // this wave's per-label minima
         int32_t* minN = a.minL[(w + 1) & 1];  // the next wave's, cleared here
-        if (tid == 0) a.s->ff_pool = 0;
-        __shared__ unsigned s_pending;
-        if (threadIdx.x == 0) s_pending = 0;
-        __syncthreads();
-        {
-            const int lane = threadIdx.x & 31;
+        unsigned left;
+        if (solo) {
+            // the candidates still pending
+            const int n = (int)s_n;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                s_n = 0;
+                s_ntask = 0;
+                a.s->ff_pool = 0;
+            }
+            __syncthreads();
+            if ((int)threadIdx.x < n) {
+                const int k = s_list[cur][threadIdx.x];
+                if (a.cres[k] == 0) s_list[cur ^ 1][atomicAdd(&s_n, 1u)] = k;
+            }
+            cur ^= 1;
+            __syncthreads();
+            left = s_n;
+            for (unsigned t = warp; t < left; t += CROSS_TPB / 32) phase_a(s_list[cur][t], minA, minN);
+            __syncthreads();
+        } else {
+            if (tid == 0) a.s->ff_pool = 0;
+            if (threadIdx.x == 0) s_pending = 0;
+            __syncthreads();
             const int gwarp = tid >> 5, nwarps = nthr >> 5;
-            const int nbox = is3d ? 125 : 25, centre = is3d ? 62 : 12;
             unsigned pending = 0;
             // warp w takes candidates w, w + nwarps, ...; its lanes read the
             // states of 32 of them at once, then it walks the pending ones
             for (int k0 = gwarp; k0 < m; k0 += 32 * nwarps) {
                 const int kl = k0 + lane * nwarps;
                 unsigned todo = __ballot_sync(0xffffffffu, kl < m && a.cres[kl] == 0);
-            while (todo) {
-                const int k = k0 + (__ffs(todo) - 1) * nwarps;
-                todo &= todo - 1;
-                const int4 ci = a.cinfo[k];
-                ++pending;
-                if (lane == 0) {
-                    atomicMin(&minA[ci.y], k);
-                    atomicMin(&minA[ci.z], k);
-                    minN[ci.y] = INT_BIG;
-                    minN[ci.z] = INT_BIG;
+                while (todo) {
+                    const int k = k0 + (__ffs(todo) - 1) * nwarps;
+                    todo &= todo - 1;
+                    ++pending;
+                    phase_a(k, minA, minN);
                 }
-                int z0, y0, x0;
-                D.decode(ci.x, z0, y0, x0);
-                // the box in three rounds of loads: cell indices, then labels
-                // and candidate slots, then the candidates' states
-                int jq[4], cq4[4];
-                int32_t lq[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int e = q * 32 + lane;
-                    jq[q] = -1;
-                    if (e < nbox && (q == 0 || nbox > 32)) {
-                        const int lz = e / 25, ly = (e / 5) % 5, lx = e % 5;
-                        // offsets of at most 2: one period at extents of 3 or more
-                        const int zz = !is3d ? z0 : (D.Nz >= 3 ? wrap1(z0 + lz - 2, D.Nz) : wrap_any(z0 + lz - 2, D.Nz));
-                        const int yy = D.Ny >= 3 ? wrap1(y0 + ly - 2, D.Ny) : wrap_any(y0 + ly - 2, D.Ny);
-                        const int xx = D.Nx >= 3 ? wrap1(x0 + lx - 2, D.Nx) : wrap_any(x0 + lx - 2, D.Nx);
-                        jq[q] = D.idx(zz, yy, xx);
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    cq4[q] = jq[q] >= 0 ? a.cmap[jq[q]] : -1;
-                    lq[q] = jq[q] >= 0 ? a.phi[jq[q]] : -1;
-                }
-                bool conflict = false;
-                uint32_t wo[4] = {0u, 0u, 0u, 0u}, wn[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int e = q * 32 + lane;
-                    const int c = cq4[q];
-                    int32_t lbl = lq[q];
-                    if (c > k) {
-                        if (a.cres[c] == 2) lbl = a.cinfo[c].y;  // accepted later: the old label
-                    } else if (c >= 0 && c < k && e != centre && a.cres[c] == 0) {
-                        const int4 cq = a.cinfo[c];
-                        conflict |= cq.y == ci.y || cq.y == ci.z || cq.z == ci.y || cq.z == ci.z;
-                    }
-                    wo[q] = __ballot_sync(0xffffffffu, lbl == ci.y);
-                    wn[q] = __ballot_sync(0xffffffffu, lbl == ci.z);
-                    if (nbox <= 32) break;
-                }
-                const bool local = !__any_sync(0xffffffffu, conflict);
-                // lane 0 takes the old label's topology, lane 1 the new one's
-                // (the same code on two masks runs side by side)
-                int part = 0;
-                if (local && lane < 2) {
-                    const uint32_t* wv = lane == 0 ? wo : wn;
-                    const u128 occ = (u128)wv[0] | ((u128)wv[1] << 32) | ((u128)wv[2] << 64) | ((u128)wv[3] << 96);
-                    const int tv = topological_number_mask(occ, is3d);
-                    part = min(tv, 2);
-                    if (tv > 1) part |= bounded_branches_connected_mask(occ, is3d, lane == 0) ? 4 : 8;
-                }
-                const int part_n = __shfl_sync(0xffffffffu, part, 1);
-                if (lane == 0) {
-                    int st = 0;
-                    if (local) {
-                        const int to = part & 3, tn = part_n & 3;
-                        st = CS_LOCAL | (to << CS_TO_SHIFT) | (tn << CS_TN_SHIFT);
-                        if (to == 0) {
-                            // at k's serial time the label holds at least count0 - (its other candidates) cells
-                            if (a.count0[ci.y] - (a.n_old[ci.y] - 1) >= 2) st |= CS_CNT_REJECT;
-                            else st |= CS_GC;
-                        } else if (to > 1) {
-                            st |= (part & 4) ? CS_OLD_LOCAL : CS_GO;
-                        }
-                        if (tn > 1) st |= (part_n & 4) ? CS_NEW_LOCAL : CS_GN;
-                    }
-                    a.cinfo[k].w = st;
-                }
-            }
             }
             if (lane == 0 && pending) atomicAdd(&s_pending, pending);
+            __syncthreads();
+            if (threadIdx.x == 0 && s_pending) atomicAdd(&rem[w % 3], s_pending);
+            if (!grid_barrier(a.s, nblocks)) return;
+            left = *((volatile unsigned*)&rem[w % 3]);
         }
-        __syncthreads();
-        if (threadIdx.x == 0 && s_pending) atomicAdd(&rem[w % 3], s_pending);
-        if (!grid_barrier(a.s, nblocks)) return;
-        const unsigned left = *((volatile unsigned*)&rem[w % 3]);
         if (left == 0) {
             if (tid == 0) a.s->waves = w;
             return;
@@ -733,113 +976,68 @@ __global__ void __launch_bounds__(256) k_crossing_sweep(CrossArgs a, int m, int 
             return;
         }
         prev_left = left;
-        if (tid == 0) rem[(w + 1) % 3] = 0;
-        // ---- phase B: readiness; decisions that need only local reads are
-        //      committed at once (they depend on nothing another decision of
-        //      this wave writes: their local reads hold no earlier pending
-        //      candidate, and later ones read back through the serial view)
-        for (int k = tid; k < m; k += nthr) {
-            if (a.cres[k] != 0) continue;
-            const int4 ci = a.cinfo[k];
-            const int st = ci.w;
-            if (!(st & CS_LOCAL)) continue;
-            if ((st & (CS_GO | CS_GC)) && minA[ci.y] < k) continue;
-            if ((st & CS_GN) && minA[ci.z] < k) continue;
-            if (st & (CS_GO | CS_GN | CS_GC)) {
-                // label-wide work: one warp per candidate in phase B2
-                a.tasks[atomicAdd(&a.s->n_tasks, 1u)] = k;
-                continue;
+        if (!solo && left <= (unsigned)solo_max) {
+            // few are left: block 0 lists them and goes on alone
+            if (blockIdx.x != 0) return;
+            solo = true;
+            if (threadIdx.x == 0) {
+                s_n = 0;
+                s_ntask = 0;
             }
-            const int to = (st >> CS_TO_SHIFT) & 3, tn = (st >> CS_TN_SHIFT) & 3;
-            // to == 0 without GC is CS_CNT_REJECT; to > 1 without GO passed the 5^d proof
-            bool acc = to != 0;
-            if (acc && tn == 0) acc = false;
-            cross_commit<real>(a, k, ci, acc);
+            __syncthreads();
+            for (int k16 = threadIdx.x * 16; k16 < m; k16 += CROSS_TPB * 16) {
+                // sixteen states at a time (the buffer extends past the last)
+                const int4 v = *reinterpret_cast<const int4*>(a.cres + k16);
+                const int word[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int b = 0; b < 16; ++b)
+                    if (k16 + b < m && ((word[b / 4] >> (8 * (b % 4))) & 0xff) == 0) s_list[cur][atomicAdd(&s_n, 1u)] = k16 + b;
+            }
+            __syncthreads();
         }
-        if (!grid_barrier(a.s, nblocks)) return;
-        const unsigned ntask = *((volatile unsigned*)&a.s->n_tasks);
+        if (!solo && tid == 0) rem[(w + 1) % 3] = 0;
+        if (solo) {
+            if (threadIdx.x < left) {
+                const int k = s_list[cur][threadIdx.x];
+                if (phase_b(k, minA)) s_tasks[atomicAdd(&s_ntask, 1u)] = k;
+            }
+        } else {
+            for (int k = tid; k < m; k += nthr)
+                if (a.cres[k] == 0 && phase_b(k, minA)) a.tasks[atomicAdd(&a.s->n_tasks, 1u)] = k;
+        }
+        if (!barrier()) return;
+        const unsigned ntask = solo ? s_ntask : *((volatile unsigned*)&a.s->n_tasks);
         if (ntask == 0) continue;  // no label-wide work: the next wave reads these commits
-        // ---- phase B2: global flood fills and exact counts, a warp per candidate
-        {
-            const int lane = threadIdx.x & 31;
-            const int gwarp = tid >> 5, nwarps = nthr >> 5;
-            for (unsigned t = gwarp; t < ntask; t += nwarps) {
-                const int k = a.tasks[t];
-                const int4 ci = a.cinfo[k];
-                const int st = ci.w;
-                const SerialView view{a.phi, a.cmap, a.cres, a.cinfo, k};
-                const int to = (st >> CS_TO_SHIFT) & 3, tn = (st >> CS_TN_SHIFT) & 3;
-                int base = 0, cap = 0;
-                uint32_t my_stamp = 0;
-                if (st & (CS_GO | CS_GN)) {
-                    // the view of a label holds at most its count plus its later candidates' cells
-                    cap = max((st & CS_GO) ? a.count[ci.y] + a.n_old[ci.y] : 0,
-                              (st & CS_GN) ? a.count[ci.z] + a.n_old[ci.z] : 0) + 1;
-                    if (lane == 0) {
-                        // queue of cap cells plus cap search ids; 8 stamps per flood fill
-                        base = (int)atomicAdd(&a.s->ff_pool, (unsigned)(2 * cap));
-                        my_stamp = atomicAdd(&a.s->stamp, 16u) + 1u;
-                    }
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    my_stamp = __shfl_sync(0xffffffffu, my_stamp, 0);
-                    if ((long long)base + 2 * cap > a.pool_size) {
-                        if (lane == 0) atomicCAS(&a.s->error, 0u, (unsigned)GPK_ERR_INTERNAL);
-                        cap = 0;
-                        base = 0;
-                    }
-                }
-                bool acc = true;
-                int visited = 0, vis = 0;
-                if (to == 0) {
-                    if (st & CS_CNT_REJECT) acc = false;
-                    else {
-                        acc = warp_serial_count(a, k, ci.y) <= 1;
-                        if (lane == 0) {
-                            atomicAdd(&a.s->count_tasks, 1ull);
-                            atomicAdd(&a.s->count_scanned, (unsigned long long)k);
-                        }
-                    }
-                } else if (to > 1 && !(st & CS_OLD_LOCAL)) {
-                    acc = warp_branches_connected_ms(D, view, ci.x, ci.y, true, a.stamp, a.stamp_rev,
-                                                     a.ff_stack + base, cap, my_stamp, &a.s->error, vis);
-                    visited += vis;
-                }
-                if (acc) {
-                    if (tn == 0) acc = false;
-                    else if (tn > 1 && !(st & CS_NEW_LOCAL))
-                        acc = warp_branches_connected_ms(D, view, ci.x, ci.z, false, a.stamp, a.stamp_rev,
-                                                         a.ff_stack + base, cap, my_stamp + 8u, &a.s->error, vis);
-                    visited += vis;
-                }
-                if (lane == 0) {
-                    a.cinfo[k].w = st | CS_READY | (acc ? CS_ACCEPT : 0);
-                    if (st & (CS_GO | CS_GN)) {
-                        atomicAdd(&a.s->flood_tasks, 1ull);
-                        atomicAdd(&a.s->flood_cells, (unsigned long long)visited);
-                    }
-                }
-            }
-        }
-        if (!grid_barrier(a.s, nblocks)) return;
+        const int32_t* tasks = solo ? s_tasks : a.tasks;
+        for (unsigned t = solo ? warp : tid >> 5; t < ntask; t += (solo ? CROSS_TPB : nthr) >> 5) phase_b2(tasks[t]);
+        if (!barrier()) return;
         // ---- phase C: commit the label-wide decisions (after all of them
         //      were taken, on the labels as they stood)
-        for (unsigned t = tid; t < ntask; t += nthr) {
-            const int k = a.tasks[t];
+        for (unsigned t = solo ? threadIdx.x : tid; t < ntask; t += solo ? CROSS_TPB : nthr) {
+            const int k = tasks[t];
             const int4 ci = a.cinfo[k];
             cross_commit<real>(a, k, ci, (ci.w & CS_ACCEPT) != 0);
         }
-        if (!grid_barrier(a.s, nblocks)) return;
-        if (tid == 0) a.s->n_tasks = 0;
+        if (!barrier()) return;
+        if (!solo && tid == 0) a.s->n_tasks = 0;
     }
     if (tid == 0) atomicCAS(&a.s->error, 0u, (unsigned)GPK_ERR_INTERNAL);
 }
 
-// Gathers the candidates (in active order), maps their cells and counts
-// the candidates per old label.
+// Gathers the candidates (in active order), maps their cells, counts the
+// candidates per old label, keeps the label counts as the sweep starts (exact
+// counts near extinction) and clears the sweep's counters.
 __global__ void k_cross_setup(const int32_t* __restrict__ active, const int32_t* __restrict__ cpos, int m,
                               const int32_t* __restrict__ phi, const int32_t* __restrict__ phi_comp, int4* cinfo,
-                              int32_t* cmap, int8_t* cres, int32_t* n_old) {
+                              int32_t* cmap, int8_t* cres, int32_t* n_old, const int32_t* __restrict__ count,
+                              int32_t* __restrict__ count0, int label_cap, StepScalars* s) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == 0) {
+        s->n_tasks = 0;
+        s->bar_count = 0;
+        s->wave_rem[0] = s->wave_rem[1] = s->wave_rem[2] = 0;
+    }
+    for (int L = k; L < label_cap; L += gridDim.x * blockDim.x) count0[L] = count[L];
     if (k >= m) return;
     const int cell = active[cpos[k]];
     const int32_t o = phi[cell];
@@ -974,7 +1172,12 @@ __device__ __forceinline__ int lower_bound_u64(const unsigned long long* a, int 
 // becomes exchange t; unmatched slots get a = -1.
 __global__ void k_bgr_match(int n, const unsigned long long* __restrict__ key1, const int32_t* __restrict__ val,
                             int4* __restrict__ exch, int32_t* __restrict__ estate, int32_t* __restrict__ pmap,
-                            const unsigned* n_dev = nullptr) {
+                            StepScalars* s, const unsigned* n_dev = nullptr) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        // the exchange loop's counters
+        s->bar_count = 0;
+        s->wave_rem[0] = s->wave_rem[1] = s->wave_rem[2] = 0;
+    }
     if (n_dev) n = (int)*n_dev;  // count read on the device (captured step); grid-stride below
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const unsigned long long k = key1[t];
@@ -1026,36 +1229,6 @@ __device__ __forceinline__ int mismatch_count(const Dims& D, const int32_t* phi,
     return m;
 }
 
-// Bounded certificate (local_only = true) with one overridden cell.
-__device__ __forceinline__ bool certificate_local(const Dims& D, const int32_t* phi, int cell, int32_t old_label,
-                                                  int32_t new_label, int old_count, int ov_cell, int32_t ov_label) {
-    if (old_label == new_label) return false;
-    const PhiReader lab{phi, ov_cell, ov_label};
-    const int old_object = topological_number(D, lab, cell, old_label);
-    const bool old_ext = old_count <= 1;
-    if (old_object == 0 && !old_ext) return false;
-    if (old_object > 1 && !bounded_branches_connected(D, lab, cell, old_label, true)) return false;
-    const int new_object = topological_number(D, lab, cell, new_label);
-    if (new_object == 0) return false;
-    if (new_object > 1 && !bounded_branches_connected(D, lab, cell, new_label, false)) return false;
-    return true;
-}
-
-// certificate_local from the 5^d occupancy masks of the old and new label
-__device__ __forceinline__ bool certificate_mask(u128 occ_old, u128 occ_new, int old_count, bool is3d) {
-    const int old_object = topological_number_mask(occ_old, is3d);
-    if (old_object == 0 && !(old_count <= 1)) return false;
-    if (old_object > 1 && !bounded_branches_connected_mask(occ_old, is3d, true)) return false;
-    const int new_object = topological_number_mask(occ_new, is3d);
-    if (new_object == 0) return false;
-    if (new_object > 1 && !bounded_branches_connected_mask(occ_new, is3d, false)) return false;
-    return true;
-}
-
-__device__ __forceinline__ u128 mask128(const uint32_t w[4]) {
-    return (u128)w[0] | ((u128)w[1] << 32) | ((u128)w[2] << 64) | ((u128)w[3] << 96);
-}
-
 struct ExchArgs {
     const unsigned* n_dev;  // exchange slots read on the device (captured step), else null
     Dims D;
@@ -1068,144 +1241,204 @@ struct ExchArgs {
 
 enum : int32_t { ES_PENDING = 1, ES_READY = 2, ES_ACCEPT = 4 };
 
-template <typename real>
-__global__ void __launch_bounds__(256) k_bgr_exchange_waves(ExchArgs a, int n, int max_waves) {
+// One block goes on alone with at most solo_max pending exchanges, as in the
+// crossing sweep.
+static constexpr int EXCH_TPB = 512, EXCH_SOLO = 128;
+
+template <typename real, bool is3d>
+__global__ void __launch_bounds__(EXCH_TPB, 1) k_bgr_exchange_waves(ExchArgs a, int n, int max_waves, int solo_max) {
     if (a.n_dev) {
         n = (int)*a.n_dev;
         max_waves = n + 1;
         if (n == 0) return;
     }
+    __shared__ int s_list[2][EXCH_SOLO];
+    __shared__ unsigned s_n;
     const int nblocks = gridDim.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = nblocks * blockDim.x;
     const Dims D = a.D;
-    const bool is3d = D.is3d();
+    constexpr int nbox = is3d ? 125 : 25;
     real* g = (real*)a.g;
     unsigned* rem = a.s->wave_rem;
     unsigned prev_left = 0xffffffffu;  // slots without an exchange are never pending
-    for (int w = 0; w < max_waves; ++w) {
-        if (tid == 0) rem[(w + 1) % 3] = 0;
-        // ---- phase 1: readiness (no earlier pending exchange of an
-        //      intersecting label pair within Chebyshev distance 2) + decision.
-        //      One warp per pending exchange: the lanes read the 5^d boxes
-        //      around both cells at once; ballots give the occupancy masks
-        //      of the two labels that the certificates test.
-        {
-            const int lane = threadIdx.x & 31;
+    // Phase 1 of exchange t (one warp): readiness (no earlier pending exchange
+    // of an intersecting label pair within Chebyshev distance 2) and decision.
+    // The lanes read the 5^d boxes around both cells at once; ballots give the
+    // occupancy masks of the two labels that the certificates test.
+    auto phase_1 = [&](int t, int32_t st) {
+        const int4 e = a.exch[t];
+        const int A = e.x, B = e.y;
+        const int32_t low = e.z, high = e.w;
+        bool blocked = false;
+        uint32_t aLow[4] = {0u, 0u, 0u, 0u}, aHigh[4] = {0u, 0u, 0u, 0u};
+        uint32_t bLow[4] = {0u, 0u, 0u, 0u}, bHigh[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            int z0, y0, x0;
+            D.decode(side ? B : A, z0, y0, x0);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int b = q * 32 + lane;
+                int32_t lbl = -1;
+                if (b < nbox) {
+                    const int lz = b / 25, ly = (b / 5) % 5, lx = b % 5;
+                    // offsets of at most 2: one period at extents of 3 or more
+                    const int zz = !is3d ? z0
+                                         : (D.Nz >= 3 ? wrap1(z0 + lz - 2, D.Nz) : wrap_any(z0 + lz - 2, D.Nz));
+                    const int yy = D.Ny >= 3 ? wrap1(y0 + ly - 2, D.Ny) : wrap_any(y0 + ly - 2, D.Ny);
+                    const int xx = D.Nx >= 3 ? wrap1(x0 + lx - 2, D.Nx) : wrap_any(x0 + lx - 2, D.Nx);
+                    const int j = D.idx(zz, yy, xx);
+                    const int pq = a.pmap[j];
+                    if (pq >= 0 && pq < t) {
+                        const int4 o = a.exch[pq];
+                        blocked |= o.z == e.z || o.z == e.w || o.w == e.z || o.w == e.w;
+                    }
+                    lbl = a.phi[j];
+                    if (side == 1 && j == A) lbl = high;  // B's certificate sees A already exchanged
+                }
+                const uint32_t ml = __ballot_sync(0xffffffffu, lbl == low);
+                const uint32_t mh = __ballot_sync(0xffffffffu, lbl == high);
+                if (side) { bLow[q] = ml; bHigh[q] = mh; } else { aLow[q] = ml; aHigh[q] = mh; }
+                if (nbox <= 32) break;
+            }
+        }
+        if (__any_sync(0xffffffffu, blocked)) return;
+        // lanes 0 to 3 take A's and B's old and new label: the local
+        // certificate of src/gpk_connectivity.cpp:10-173 and the mismatches
+        // before and after the exchange, side by side
+        bool ok = true;
+        int mm = 0;
+        if (lane < 4) {
+            uint32_t wv[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                wv[q] = lane == 0 ? aLow[q] : (lane == 1 ? aHigh[q] : (lane == 2 ? bHigh[q] : bLow[q]));
+            const bool old_label = (lane & 1) == 0;
+            const Box5<is3d> box(wv);
+            const int tn = box.topological_number();
+            if (tn == 0) ok = old_label && (lane == 0 ? a.count[low] : a.count[high] + 1) <= 1;
+            else if (tn > 1) ok = box.branches_connected(old_label);
+            const int cell = lane == 0 || lane == 2 ? A : B, other = lane == 0 || lane == 2 ? B : A;
+            const int32_t own = lane == 0 || lane == 3 ? low : high, oth = lane == 0 || lane == 3 ? high : low;
+            mm = mismatch_count(D, a.phi, cell, own, other, oth);
+        }
+        const bool certified = __all_sync(0xffffffffu, ok);
+        const int before = __shfl_sync(0xffffffffu, mm, 0) + __shfl_sync(0xffffffffu, mm, 1);
+        const int after = __shfl_sync(0xffffffffu, mm, 2) + __shfl_sync(0xffffffffu, mm, 3);
+        if (lane == 0) {
+            const bool acc = certified && after < before && a.phi[A] == low && a.phi[B] == high;
+            a.estate[t] = st | ES_READY | (acc ? ES_ACCEPT : 0);
+        }
+    };
+    // Phase 2 of a pending exchange t (one thread): commits a decided one;
+    // true when it stays pending
+    auto phase_2 = [&](int t, int32_t st) -> bool {
+        if (!(st & ES_READY)) return true;
+        const int4 e = a.exch[t];
+        if (st & ES_ACCEPT) {
+            const real ga = target_orientation<real>(D, a.phi, g, e.x, e.w);
+            const real gb = target_orientation<real>(D, a.phi, g, e.y, e.z);
+            // ga/gb are read before any write of this exchange; other
+            // exchanges committing now never touch these labels' cells
+            a.phi[e.x] = e.w;
+            a.phi[e.y] = e.z;
+            g[e.x] = ga;
+            g[e.y] = gb;
+            ((real*)a.alpha)[e.x] = (real)1;
+            ((real*)a.alpha)[e.y] = (real)1;
+            if (a.sweep_rho) {
+                const real r = sizeof(real) == 4 ? (real)a.rho_rex_f : (real)a.rho_rex_d;
+                ((real*)a.rho)[e.x] = r;
+                ((real*)a.rho)[e.y] = r;
+            }
+            atomicAdd(&a.s->exch_pass, 2ull);
+        }
+        a.pmap[e.x] = -1;
+        a.pmap[e.y] = -1;
+        a.estate[t] = 0;
+        return false;
+    };
+    // the exchanges whose state is pending, by block 0
+    auto list_pending = [&]() {
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        for (int t = threadIdx.x; t < n; t += EXCH_TPB)
+            if (a.estate[t] & ES_PENDING) s_list[0][atomicAdd(&s_n, 1u)] = t;
+        __syncthreads();
+    };
+    int w = 0;
+    if (n > solo_max) {
+        unsigned left = 0;
+        for (; w < max_waves; ++w) {
+            if (tid == 0) rem[(w + 1) % 3] = 0;
             const int gwarp = tid >> 5, nwarps = nthr >> 5;
-            const int nbox = is3d ? 125 : 25;
             // warp w takes exchanges w, w + nwarps, ...; its lanes read the
             // states of 32 of them at once, then it walks the pending ones
             for (int t0 = gwarp; t0 < n; t0 += 32 * nwarps) {
                 const int tl = t0 + lane * nwarps;
                 const int32_t stl = tl < n ? a.estate[tl] : 0;
                 unsigned todo = __ballot_sync(0xffffffffu, (stl & ES_PENDING) != 0);
-            while (todo) {
-                const int j0 = __ffs(todo) - 1;
-                todo &= todo - 1;
-                const int t = t0 + j0 * nwarps;
-                const int32_t st = __shfl_sync(0xffffffffu, stl, j0);
-                const int4 e = a.exch[t];
-                const int A = e.x, B = e.y;
-                const int32_t low = e.z, high = e.w;
-                bool blocked = false;
-                uint32_t aLow[4] = {0u, 0u, 0u, 0u}, aHigh[4] = {0u, 0u, 0u, 0u};
-                uint32_t bLow[4] = {0u, 0u, 0u, 0u}, bHigh[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-                for (int side = 0; side < 2; ++side) {
-                    int z0, y0, x0;
-                    D.decode(side ? B : A, z0, y0, x0);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int b = q * 32 + lane;
-                        int32_t lbl = -1;
-                        if (b < nbox) {
-                            const int lz = b / 25, ly = (b / 5) % 5, lx = b % 5;
-                            // offsets of at most 2: one period at extents of 3 or more
-                            const int zz = !is3d ? z0
-                                                 : (D.Nz >= 3 ? wrap1(z0 + lz - 2, D.Nz) : wrap_any(z0 + lz - 2, D.Nz));
-                            const int yy = D.Ny >= 3 ? wrap1(y0 + ly - 2, D.Ny) : wrap_any(y0 + ly - 2, D.Ny);
-                            const int xx = D.Nx >= 3 ? wrap1(x0 + lx - 2, D.Nx) : wrap_any(x0 + lx - 2, D.Nx);
-                            const int j = D.idx(zz, yy, xx);
-                            const int pq = a.pmap[j];
-                            if (pq >= 0 && pq < t) {
-                                const int4 o = a.exch[pq];
-                                blocked |= o.z == e.z || o.z == e.w || o.w == e.z || o.w == e.w;
-                            }
-                            lbl = a.phi[j];
-                            if (side == 1 && j == A) lbl = high;  // B's certificate sees A already exchanged
-                        }
-                        const uint32_t ml = __ballot_sync(0xffffffffu, lbl == low);
-                        const uint32_t mh = __ballot_sync(0xffffffffu, lbl == high);
-                        if (side) { bLow[q] = ml; bHigh[q] = mh; } else { aLow[q] = ml; aHigh[q] = mh; }
-                        if (nbox <= 32) break;
-                    }
-                }
-                if (__any_sync(0xffffffffu, blocked)) continue;
-                if (lane == 0) {
-                    bool acc = false;
-                    if (a.phi[A] == low && a.phi[B] == high) {
-                        const int before =
-                            mismatch_count(D, a.phi, A, low, B, high) + mismatch_count(D, a.phi, B, high, A, low);
-                        const int after =
-                            mismatch_count(D, a.phi, A, high, B, low) + mismatch_count(D, a.phi, B, low, A, high);
-                        if (after < before) {
-                            const int cl = a.count[low], ch = a.count[high];
-                            if (certificate_mask(mask128(aLow), mask128(aHigh), cl, is3d) &&
-                                certificate_mask(mask128(bHigh), mask128(bLow), ch + 1, is3d))
-                                acc = true;
-                        }
-                    }
-                    a.estate[t] = st | ES_READY | (acc ? ES_ACCEPT : 0);
+                while (todo) {
+                    const int j0 = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    phase_1(t0 + j0 * nwarps, __shfl_sync(0xffffffffu, stl, j0));
                 }
             }
+            if (!grid_barrier(a.s, nblocks)) return;
+            for (int t = tid; t < n; t += nthr) {
+                const int32_t st = a.estate[t];
+                if ((st & ES_PENDING) && phase_2(t, st)) atomicAdd(&rem[w % 3], 1u);
             }
+            if (!grid_barrier(a.s, nblocks)) return;
+            left = *((volatile unsigned*)&rem[w % 3]);
+            if (left <= (unsigned)solo_max) break;
+            if (left >= prev_left) {
+                if (threadIdx.x == 0) atomicCAS(&a.s->error, 0u, (unsigned)GPK_ERR_INTERNAL);
+                return;
+            }
+            prev_left = left;
         }
-        if (!grid_barrier(a.s, nblocks)) return;
-        // ---- phase 2: commit
-        for (int t = tid; t < n; t += nthr) {
-            const int32_t st = a.estate[t];
-            if (!(st & ES_PENDING)) continue;
-            if (st & ES_READY) {
-                const int4 e = a.exch[t];
-                if (st & ES_ACCEPT) {
-                    const real ga = target_orientation<real>(D, a.phi, g, e.x, e.w);
-                    const real gb = target_orientation<real>(D, a.phi, g, e.y, e.z);
-                    // ga/gb are read before any write of this exchange; other
-                    // exchanges committing now never touch these labels' cells
-                    a.phi[e.x] = e.w;
-                    a.phi[e.y] = e.z;
-                    g[e.x] = ga;
-                    g[e.y] = gb;
-                    ((real*)a.alpha)[e.x] = (real)1;
-                    ((real*)a.alpha)[e.y] = (real)1;
-                    if (a.sweep_rho) {
-                        const real r = sizeof(real) == 4 ? (real)a.rho_rex_f : (real)a.rho_rex_d;
-                        ((real*)a.rho)[e.x] = r;
-                        ((real*)a.rho)[e.y] = r;
-                    }
-                    atomicAdd(&a.s->exch_pass, 2ull);
-                }
-                a.pmap[e.x] = -1;
-                a.pmap[e.y] = -1;
-                a.estate[t] = 0;
-            } else {
-                atomicAdd(&rem[w % 3], 1u);
-            }
-        }
-        if (!grid_barrier(a.s, nblocks)) return;
-        const unsigned left = *((volatile unsigned*)&rem[w % 3]);
-        if (left == 0) {
-            if (tid == 0) a.s->waves = w + 1;
+        if (w == max_waves) {
+            if (tid == 0) atomicCAS(&a.s->error, 0u, (unsigned)GPK_ERR_INTERNAL);
             return;
         }
-        if (left >= prev_left) {
+        ++w;
+        if (blockIdx.x != 0) return;
+        if (left == 0) {
+            if (threadIdx.x == 0) a.s->waves = w;
+            return;
+        }
+        prev_left = left + 1u;
+    }
+    if (blockIdx.x != 0) return;
+    list_pending();
+    for (int cur = 0;; cur ^= 1, ++w) {
+        const unsigned left = s_n;
+        // (a pass without exchanges counts one wave, as it does on the grid)
+        if (left == 0) {
+            if (threadIdx.x == 0) a.s->waves = w < 1 ? 1 : w;
+            return;
+        }
+        if (left >= prev_left || w >= max_waves) {
             if (threadIdx.x == 0) atomicCAS(&a.s->error, 0u, (unsigned)GPK_ERR_INTERNAL);
             return;
         }
         prev_left = left;
+        for (unsigned i = warp; i < left; i += EXCH_TPB / 32) {
+            const int t = s_list[cur][i];
+            phase_1(t, a.estate[t]);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        if (threadIdx.x < left) {
+            const int t = s_list[cur][threadIdx.x];
+            if (phase_2(t, a.estate[t])) s_list[cur ^ 1][atomicAdd(&s_n, 1u)] = t;
+        }
+        __syncthreads();
     }
-    if (tid == 0) atomicCAS(&a.s->error, 0u, (unsigned)GPK_ERR_INTERNAL);
 }
 
 // ---------------------------------------------------------------------------
@@ -1432,8 +1665,7 @@ static int coop_grid(gpk_grid* G, const void* kernel, int block, int want_items)
 }
 
 static int launch_coop(gpk_grid* G, const void* kernel, int grid, int block, void** args) {
-    GPK_CUDA_TRY(cudaMemsetAsync(&G->scal->bar_count, 0, sizeof(unsigned), G->stream));
-    GPK_CUDA_TRY(cudaMemsetAsync(G->scal->wave_rem, 0, sizeof(G->scal->wave_rem), G->stream));
+    // (the barrier's and the wave counters were cleared by the kernel before)
     const bool inject = G->inject_spin_limit > 0;
     if (inject) {
         // failure injection (gpk_grid_inject_wait_timeout): the first grid
@@ -1460,12 +1692,10 @@ template <typename real>
 int gpk_crossings(gpk_grid* G, int m) {
     if (m == 0) return GPK_OK;
     const int B = 256;
-    // label counts at the start of the sweep (exact counts near extinction)
-    GPK_CUDA_TRY(cudaMemcpyAsync(G->count0, G->count, sizeof(int32_t) * G->label_cap, cudaMemcpyDeviceToDevice,
-                                 G->stream));
     int8_t* cres = (int8_t*)G->val_a;  // candidate results, scratch until the remap
     k_cross_setup<<<(m + B - 1) / B, B, 0, G->stream>>>(G->active, G->cand, m, G->phi, G->phi_comp,
-                                                        (int4*)G->cand_info, G->pmap, cres, G->n_old);
+                                                        (int4*)G->cand_info, G->pmap, cres, G->n_old, G->count, G->count0,
+                                                        G->label_cap, G->scal);
     G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     CrossArgs a;
@@ -1479,14 +1709,15 @@ int gpk_crossings(gpk_grid* G, int m) {
     a.stamp = G->stamp; a.stamp_rev = G->stamp_rev; a.ff_stack = G->ff_stack; a.pool_size = 5LL * G->d.N + 64;
     a.s = G->scal;
     a.tasks = (int32_t*)G->key_a;  // free until the remap
-    GPK_CUDA_TRY(cudaMemsetAsync(&G->scal->n_tasks, 0, sizeof(unsigned), G->stream));
     a.sweep_rho = G->th.dislocation_enabled; a.rho_rex_f = G->th.rho_rex; a.rho_rex_d = (double)G->th.rho_rex;
     int max_waves = m + 1;
-    void* args[] = {&a, &m, &max_waves};
-    const void* kern = (const void*)k_crossing_sweep<real>;
+    // (an injected wait needs the grid's barriers)
+    int solo_max = G->inject_spin_limit > 0 ? 0 : CROSS_SOLO;
+    void* args[] = {&a, &m, &max_waves, &solo_max};
+    const void* kern = G->d.is3d() ? (const void*)k_crossing_sweep<real, true> : (const void*)k_crossing_sweep<real, false>;
     // phase A runs one warp per pending candidate
-    const int grid = coop_grid(G, kern, 256, (int)std::min<long long>(32LL * m, 1LL << 30));
-    GPK_TRY(launch_coop(G, kern, grid, 256, args));
+    const int grid = m <= solo_max ? 1 : coop_grid(G, kern, CROSS_TPB, (int)std::min<long long>(32LL * m, 1LL << 30));
+    GPK_TRY(launch_coop(G, kern, grid, CROSS_TPB, args));
     k_cross_cleanup<<<(m + B - 1) / B, B, 0, G->stream>>>(m, (const int4*)G->cand_info, G->pmap, G->n_old, G->minL,
                                                         G->minF);
     G->launches++;
@@ -1557,7 +1788,8 @@ int gpk_remap_pass(gpk_grid* G, const unsigned long long* gate) {
     while (lbits < 27 && (1LL << lbits) < (long long)G->label_cap) ++lbits;
     GPK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(G->cub_tmp, bytes, (const unsigned long long*)G->key_b, G->key_a,
                                                  (const int32_t*)G->val_b, G->val_a, n, 10, 37 + lbits, G->stream));
-    k_bgr_match<<<(n + B - 1) / B, B, 0, G->stream>>>(n, G->key_a, G->val_a, (int4*)G->exch, G->val_b, G->pmap);
+    k_bgr_match<<<(n + B - 1) / B, B, 0, G->stream>>>(n, G->key_a, G->val_a, (int4*)G->exch, G->val_b, G->pmap,
+                                                  G->scal);
     G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     ExchArgs a;
@@ -1570,10 +1802,13 @@ int gpk_remap_pass(gpk_grid* G, const unsigned long long* gate) {
     a.sweep_rho = G->th.dislocation_enabled; a.rho_rex_f = G->th.rho_rex; a.rho_rex_d = (double)G->th.rho_rex;
     int max_waves = n + 1;
     int nn = n;
-    void* args[] = {&a, &nn, &max_waves};
-    const void* kern = (const void*)k_bgr_exchange_waves<real>;
+    int solo_max = G->inject_spin_limit > 0 ? 0 : EXCH_SOLO;
+    void* args[] = {&a, &nn, &max_waves, &solo_max};
+    const void* kern =
+        D.is3d() ? (const void*)k_bgr_exchange_waves<real, true> : (const void*)k_bgr_exchange_waves<real, false>;
     // phase 1 runs one warp per pending exchange
-    return launch_coop(G, kern, coop_grid(G, kern, 256, (int)std::min<long long>(32LL * n, 1LL << 30)), 256, args);
+    const int grid_x = n <= solo_max ? 1 : coop_grid(G, kern, EXCH_TPB, (int)std::min<long long>(32LL * n, 1LL << 30));
+    return launch_coop(G, kern, grid_x, EXCH_TPB, args);
 }
 
 template <typename real>
@@ -1664,7 +1899,7 @@ int gpk_remap_pass_graph(gpk_grid* G, const unsigned long long* gate) {
                                                 G->val_b, k1b, k2b, G->val_a);
     // sorted: primary keys in key_a, cells in val_b
     k_bgr_match<<<grid, B, 0, G->stream>>>(0, G->key_a, G->val_b, (int4*)G->exch, G->val_a, G->pmap,
-                                           &G->scal->n_prop);
+                                           G->scal, &G->scal->n_prop);
     G->launches += 4;
     GPK_CUDA_TRY(cudaGetLastError());
     ExchArgs a;
@@ -1675,14 +1910,15 @@ int gpk_remap_pass_graph(gpk_grid* G, const unsigned long long* gate) {
     a.g = G->f[GPK_FIELD_G]; a.alpha = G->f[GPK_FIELD_ALPHA]; a.rho = G->f[GPK_FIELD_RHO];
     a.s = G->scal;
     a.sweep_rho = G->th.dislocation_enabled; a.rho_rex_f = G->th.rho_rex; a.rho_rex_d = (double)G->th.rho_rex;
-    int max_waves = 1, nn = 0;
-    void* args[] = {&a, &nn, &max_waves};
-    const void* kern = (const void*)k_bgr_exchange_waves<real>;
+    int max_waves = 1, nn = 0, solo_max = EXCH_SOLO;
+    void* args[] = {&a, &nn, &max_waves, &solo_max};
+    const void* kern =
+        D.is3d() ? (const void*)k_bgr_exchange_waves<real, true> : (const void*)k_bgr_exchange_waves<real, false>;
     // the slot count is known only on the device: one block per 8192 cells
     // (at most the usual cap), so that the exchange loops of many small grids
     // captured side by side fit on the GPU together
-    const long long want = std::max(1LL, ((long long)D.N + 8191) / 8192) * 256;
-    return launch_coop(G, kern, coop_grid(G, kern, 256, (int)std::min<long long>(want, 1LL << 30)), 256, args);
+    const long long want = std::max(1LL, ((long long)D.N + 8191) / 8192) * EXCH_TPB;
+    return launch_coop(G, kern, coop_grid(G, kern, EXCH_TPB, (int)std::min<long long>(want, 1LL << 30)), EXCH_TPB, args);
 }
 
 template int gpk_remap_pass<float>(gpk_grid*, const unsigned long long*);

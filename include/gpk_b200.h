@@ -241,7 +241,8 @@ int gpk_grid_profile(gpk_grid* grid, int enable);
  * calls[k] = profiled steps; both reset after reading.                     */
 int gpk_grid_stage_times(gpk_grid* grid, double ms[GPK_NUM_STAGES], uint64_t calls[GPK_NUM_STAGES]);
 /* out = {waves of the crossing sweeps, waves of the remap exchange loops,
- * crossing candidates, remap proposals, global flood fills, cells they
+ * crossing candidates, remap proposals, label-wide tests (global flood
+ * fills, most of them settled in a window around the cell), cells the fills
  * visited, exact label counts, candidates those counts scanned, interface
  * cells given remap scores, those of them summed tap by tap}, summed since
  * the last read.                                                           */
