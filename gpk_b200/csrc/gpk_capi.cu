@@ -393,13 +393,6 @@ extern "C" int gpk_grid_create(int Nz, int Ny, int Nx, double dx, const gpk_ther
     if (cudaMemsetAsync(G->scal, 0, sizeof(StepScalars), G->stream) != cudaSuccess) return fail(GPK_ERR_CUDA);
     rc = precision == GPK_PREC_F32 ? gpk_build_tables<float>(G) : gpk_build_tables<double>(G);
     if (rc != GPK_OK) return fail(rc);
-    bool sep = precision == GPK_PREC_F32 ? ((HostKernels<float>*)G->host_kernels)->global_separable
-                                         : ((HostKernels<double>*)G->host_kernels)->global_separable;
-    if (sep) {
-        if ((rc = gpk_alloc(G, &G->sep_I, rb)) || (rc = gpk_alloc(G, &G->sep_t1, rb)) ||
-            (rc = gpk_alloc(G, &G->sep_t2, rb)) || (rc = gpk_alloc(G, &G->sep_S, rb)))
-            return fail(rc);
-    }
     rc = precision == GPK_PREC_F32 ? init_fields<float>(G) : init_fields<double>(G);
     if (rc != GPK_OK) return fail(rc);
     if ((rc = gpk_ensure_label_capacity(G, 64)) != GPK_OK) return fail(rc);

@@ -86,8 +86,10 @@ struct gpk_grid {
     void* cub_tmp = nullptr; size_t cub_tmp_bytes = 0;
     // extinction
     uint8_t* unres = nullptr; int32_t* ero_target = nullptr; void* ero_g = nullptr;
-    // separable geometry
+    // separable geometry: label by label over the whole grid, or per label box
+    // (gpk_separable.cu: values of the passes; label index and regions)
     void* sep_I = nullptr; void* sep_t1 = nullptr; void* sep_t2 = nullptr; void* sep_S = nullptr;
+    void* sep_box = nullptr; void* sep_table = nullptr; size_t sep_table_bytes = 0;
     // labels
     int32_t* count = nullptr;              // cells per label
     int32_t* count0 = nullptr;             // cells per label when the crossing sweep started
@@ -161,6 +163,7 @@ template <typename real> int gpk_phase_volume_impl(gpk_grid* G, int32_t label, d
 template <typename real>
 int gpk_geometry_items(gpk_grid* G, int R, real inv_dx, real inv_dx2, real dx, real kappa_limit);
 template <typename real> int gpk_geometry_items_init(gpk_grid* G);
+template <typename real> int gpk_geometry_separable(gpk_grid* G, real dx, real kappa_limit);
 // FP64 separable tiles (throughput geometry); -1 when they do not apply
 int gpk_geometry_sep_tiles(gpk_grid* G, int R, const double* gauss, int gauss_radius, double dx,
                            double kappa_limit);

@@ -1,0 +1,387 @@
+// gpk_separable.cu — the separable geometry of broad 3-D kernels, sm_100a.
+//
+// The reference smooths the indicator of every interface label over the whole
+// grid (src/gpk_gaussian.cpp:9-72: per axis acc = 0; acc += w[k] * in[q+k-R]
+// for k = 0..2R), then takes fourth-order differences at that label's
+// interface cells (src/gpk_geometry.cpp:185-390).  The smoothed values are
+// read only within two cells of those interface cells, so each label's passes
+// here cover the periodic box of its interface cells plus two cells (and the
+// kernel's radius more along the axes still to be smoothed), and all labels'
+// boxes run in one launch per pass.  Every value that is formed has the
+// reference's operations in its order.
+//
+//   x  the window of a row is 2R+1 bits of the label's row; a run of ones has
+//      one of (2R+1)(2R+2)/2 sums, tabulated on the host in tap order, and
+//      other patterns add their set taps (adding w * 0 = +0 changes nothing);
+//   y, z  a thread forms eight outputs of a line from a register ring: one
+//      value load and one tap load per tap and eight outputs; bound by the
+//      unfused multiplies and adds (74 per output at radius 18).
+// The whole-grid passes, one label after another (four launches each), took
+// 7.0 ms plus 2.9 ms of evaluation and gaps for eight steps of 128^3 with 24
+// grains at sigma 5.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <vector>
+
+#include "gpk_grid.h"
+
+namespace gpk_dev {
+
+struct SepRegion {
+    int32_t label;
+    int ox, oy, oz;           // first smoothed cell (in the grid)
+    int nx, ny, nz;           // smoothed cells per axis
+    int sy, ey, sz, ez;       // rows and planes that the y and z sums read: start, count (at most a period)
+    long long t1, t2, s;      // offsets of the x-smoothed, y-smoothed and smoothed values
+};
+
+static constexpr int SEP_MAX_R = 31;  // a window of 63 bits
+
+// marks the coordinates of each label's interface cells, per axis
+__global__ void k_sep_marks(Dims D, const int32_t* __restrict__ active, const unsigned* __restrict__ n_active,
+                            const int32_t* __restrict__ phi, uint8_t* __restrict__ marks) {
+    const int na = (int)*n_active, S = D.Nx + D.Ny + D.Nz;
+    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
+        const int i = active[a];
+        int z, y, x;
+        D.decode(i, z, y, x);
+        uint8_t* m = marks + (size_t)phi[i] * S;
+        m[x] = 1;
+        m[D.Nx + y] = 1;
+        m[D.Nx + D.Ny + z] = 1;
+    }
+}
+
+// x sums: a warp per row of a region, blockIdx.y = region
+template <typename real>
+__global__ void __launch_bounds__(256) k_sep_box_x(Dims D, const int32_t* __restrict__ phi,
+                                                   const SepRegion* __restrict__ regions, int R, int words,
+                                                   const real* __restrict__ w, const real* __restrict__ runs,
+                                                   real* __restrict__ out) {
+    extern __shared__ uint32_t sep_words[];
+    const SepRegion g = regions[blockIdx.y];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, K = 2 * R + 1;
+    uint32_t* row_bits = sep_words + warp * (words + 2);
+    const int rows = g.ey * g.ez, nbit = g.nx + 2 * R;
+    const int x0 = wrap_any(g.ox - R + lane, D.Nx);
+    for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
+        int y = g.sy + r % g.ey, z = g.sz + r / g.ey;
+        if (y >= D.Ny) y -= D.Ny;
+        if (z >= D.Nz) z -= D.Nz;
+        const int32_t* row = phi + (size_t)(z * D.Ny + y) * D.Nx;
+        __syncwarp();
+        int x = x0;
+        for (int b = 0; b < nbit; b += 128) {
+            int32_t v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                v[u] = row[x];
+                x += 32;
+                while (x >= D.Nx) x -= D.Nx;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t bits = __ballot_sync(0xffffffffu, v[u] == g.label);
+                if (lane == 0 && b + 32 * u < nbit) row_bits[(b >> 5) + u] = bits;
+            }
+        }
+        if (lane < 2) row_bits[((nbit + 31) >> 5) + lane] = 0u;
+        __syncwarp();
+        real* o = out + g.t1 + (long long)r * g.nx;
+        for (int e = lane; e < g.nx; e += 32) {
+            const int q = e >> 5, sh = e & 31;
+            const uint32_t lo = __funnelshift_r(row_bits[q], row_bits[q + 1], sh);
+            const uint32_t hi = __funnelshift_r(row_bits[q + 1], row_bits[q + 2], sh);
+            uint64_t p = (((uint64_t)hi << 32) | lo) & ((1ull << K) - 1ull);
+            real v = (real)0;
+            if (p) {
+                const int first = __ffsll((long long)p) - 1;
+                const uint64_t t = p >> first;
+                if ((t & (t + 1ull)) == 0ull) {
+                    v = runs[first * (K + 1) + __popcll(t)];
+                } else {
+                    while (p) {
+                        v += w[__ffsll((long long)p) - 1];
+                        p &= p - 1ull;
+                    }
+                }
+            }
+            o[e] = v;
+        }
+    }
+}
+
+// y sums (AXIS 1: ey rows -> ny) and z sums (AXIS 2: ez planes -> nz)
+template <typename real, int AXIS>
+__global__ void __launch_bounds__(256) k_sep_box_line(Dims D, const SepRegion* __restrict__ regions, int R,
+                                                      const real* __restrict__ w, const real* __restrict__ in,
+                                                      real* __restrict__ out) {
+    constexpr int M = 8;
+    __shared__ real tap[2 * SEP_MAX_R + 1];
+    const SepRegion g = regions[blockIdx.y];
+    const int K = 2 * R + 1;
+    for (int k = threadIdx.x; k < K; k += 256) tap[k] = w[k];
+    __syncthreads();
+    const int n = AXIS == 1 ? g.ny : g.nz, e = AXIS == 1 ? g.ey : g.ez;
+    const int period = AXIS == 1 ? D.Ny : D.Nz;
+    const int nb = (n + M - 1) / M;
+    // lines: (x, z) for y, (x, y) for z; threads run along x
+    const int plane = AXIS == 1 ? g.nx : g.nx * g.ny;  // in and out: step along the line
+    const int others = AXIS == 1 ? g.ez : 1;
+    const int inner = AXIS == 1 ? g.nx : g.nx * g.ny;
+    const long long total = (long long)inner * nb * others;
+    for (long long t = blockIdx.x * 256LL + threadIdx.x; t < total; t += gridDim.x * 256LL) {
+        const int l = (int)(t % inner), b = (int)(t / inner % nb), o = (int)(t / inner / nb);
+        const real* src = in + (AXIS == 1 ? g.t1 + (long long)o * g.ey * g.nx : g.t2) + l;
+        real* dst = out + (AXIS == 1 ? g.t2 + (long long)o * g.ny * g.nx : g.s) + l;
+        // position of the window's first value; past the last one a period
+        // starts again, or (values that no stored output reads) the last stays
+        int j = b * M;
+        if (e == period) j %= period;
+        auto next = [&]() {
+            const real v = src[(long long)j * plane];
+            if (++j >= e) j = e == period ? 0 : e - 1;
+            return v;
+        };
+        real v[M], acc[M];
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            v[m] = next();
+            acc[m] = (real)0;
+        }
+        int k = 0;
+        for (; k + M <= K; k += M) {
+#pragma unroll
+            for (int q = 0; q < M; ++q) {
+                const real wk = tap[k + q];
+#pragma unroll
+                for (int m = 0; m < M; ++m) acc[m] += wk * v[(m + q) % M];
+                v[q] = next();
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < M - 1; ++q) {
+            if (k + q >= K) break;
+            const real wk = tap[k + q];
+#pragma unroll
+            for (int m = 0; m < M; ++m) acc[m] += wk * v[(m + q) % M];
+            v[q] = next();
+        }
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+            if (b * M + m < n) dst[(long long)(b * M + m) * plane] = acc[m];
+    }
+}
+
+// fourth-order differences at the interface cells of the labels in `index`
+// (label -> region, -1: another batch's)
+template <typename real>
+__global__ void k_sep_box_eval(Dims D, const int32_t* __restrict__ active, const unsigned* __restrict__ n_active,
+                               const int32_t* __restrict__ phi, const int32_t* __restrict__ index,
+                               const SepRegion* __restrict__ regions, const real* __restrict__ Sv, real dx,
+                               real kappa_limit, real* __restrict__ nxo, real* __restrict__ nyo,
+                               real* __restrict__ nzo, real* __restrict__ ko) {
+    const real idx12 = (real)1 / ((real)12 * dx);
+    const real idx_sq = (real)1 / (dx * dx);
+    const real idx12_sq = idx_sq / (real)12;
+    const real idx144_sq = idx_sq / (real)144;
+    const int na = (int)*n_active;
+    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
+        const int i = active[a];
+        const int r = index[phi[i]];
+        if (r < 0) continue;
+        const SepRegion g = regions[r];
+        int z, y, x;
+        D.decode(i, z, y, x);
+        // the cell in its region, and the two cells to each side (a region
+        // that is a whole period wraps)
+        int xo[5], yo[5], zo[5];
+#pragma unroll
+        for (int d = 0; d < 5; ++d) {
+            xo[d] = wrap_any(x - g.ox + d - 2, D.Nx);
+            yo[d] = wrap_any(y - g.oy + d - 2, D.Ny) * g.nx;
+            zo[d] = wrap_any(z - g.oz + d - 2, D.Nz) * (g.nx * g.ny);
+        }
+        const real* S = Sv + g.s;
+        auto at = [&](int c, int b, int e) { return S[zo[c] + yo[b] + xo[e]]; };
+        const real I0 = at(2, 2, 2);
+        const real Ix = (at(2, 2, 0) - (real)8 * at(2, 2, 1) + (real)8 * at(2, 2, 3) - at(2, 2, 4)) * idx12;
+        const real Iy = (at(2, 0, 2) - (real)8 * at(2, 1, 2) + (real)8 * at(2, 3, 2) - at(2, 4, 2)) * idx12;
+        const real Iz = (at(0, 2, 2) - (real)8 * at(1, 2, 2) + (real)8 * at(3, 2, 2) - at(4, 2, 2)) * idx12;
+        const real Ixx = (-at(2, 2, 4) + (real)16 * at(2, 2, 3) - (real)30 * I0 + (real)16 * at(2, 2, 1) - at(2, 2, 0)) * idx12_sq;
+        const real Iyy = (-at(2, 4, 2) + (real)16 * at(2, 3, 2) - (real)30 * I0 + (real)16 * at(2, 1, 2) - at(2, 0, 2)) * idx12_sq;
+        const real Izz = (-at(4, 2, 2) + (real)16 * at(3, 2, 2) - (real)30 * I0 + (real)16 * at(1, 2, 2) - at(0, 2, 2)) * idx12_sq;
+        constexpr int off[4] = {0, 1, 3, 4};
+        const real dc[4] = {(real)1, (real)-8, (real)8, (real)-1};
+        real Ixy_sum = 0, Ixz_sum = 0, Iyz_sum = 0;
+#pragma unroll
+        for (int aa = 0; aa < 4; ++aa)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const real wt = dc[aa] * dc[b];
+                Ixy_sum += wt * at(2, off[b], off[aa]);
+                Ixz_sum += wt * at(off[b], 2, off[aa]);
+                Iyz_sum += wt * at(off[b], off[aa], 2);
+            }
+        const real Ixy = Ixy_sum * idx144_sq, Ixz = Ixz_sum * idx144_sq, Iyz = Iyz_sum * idx144_sq;
+        const real grad_sq = Ix * Ix + Iy * Iy + Iz * Iz;
+        if (grad_sq * dx * dx > (real)1e-8) {
+            const real inv_grad = (real)1 / sqrt(grad_sq);
+            nxo[i] = -Ix * inv_grad;
+            nyo[i] = -Iy * inv_grad;
+            nzo[i] = -Iz * inv_grad;
+            const real trace_H = Ixx + Iyy + Izz;
+            const real gHg = Ix * Ix * Ixx + Iy * Iy * Iyy + Iz * Iz * Izz + (real)2 * (Ix * Iy * Ixy + Ix * Iz * Ixz + Iy * Iz * Iyz);
+            real k = (gHg - grad_sq * trace_H) / (grad_sq * sqrt(grad_sq));
+            if (fabs(k * dx) < (real)1e-6) k = (real)0;
+            ko[i] = dclamp(k, -kappa_limit, kappa_limit);
+        }
+    }
+}
+
+// the shortest periodic run of coordinates that holds every marked one
+static void arc_of(const uint8_t* m, int n, int& start, int& len) {
+    int best = -1, best_end = 0, run = 0, first = -1;
+    for (int k = 0; k < n && first < 0; ++k)
+        if (m[k]) first = k;
+    for (int q = 1; q <= n; ++q) {
+        const int k = (first + q) % n;
+        if (m[k]) {
+            if (run > best) {
+                best = run;
+                best_end = k;
+            }
+            run = 0;
+        } else {
+            ++run;
+        }
+    }
+    start = best_end;     // the marked coordinate after the longest gap
+    len = n - best;
+}
+
+}  // namespace gpk_dev
+
+using namespace gpk_dev;
+
+// Smoothing and differences of every interface label into nx, ny, nz, kappa
+// (zero on entry); -1 where this form does not apply (the caller then smooths
+// label by label over the whole grid).
+template <typename real>
+int gpk_geometry_separable(gpk_grid* G, real dx, real kappa_limit) {
+    HostKernels<real>* hk = (HostKernels<real>*)G->host_kernels;
+    const Dims D = G->d;
+    const int R = hk->gauss_radius, K = 2 * R + 1, span = D.Nx + D.Ny + D.Nz;
+    // (the marks lie in the proposal keys' buffer, free until the remap)
+    const size_t mark_bytes = (size_t)G->label_cap * span;
+    if (R > SEP_MAX_R || !D.is3d() || D.Nx < 2 || D.Ny < 2 || mark_bytes > 8 * (size_t)D.N) return -1;
+    uint8_t* marks = (uint8_t*)G->key_a;
+    GPK_CUDA_TRY(cudaMemsetAsync(marks, 0, mark_bytes, G->stream));
+    k_sep_marks<<<G->num_sms * 8, 256, 0, G->stream>>>(D, G->active, &G->scal->n_active, G->phi, marks);
+    G->launches++;
+    std::vector<uint8_t> hm(mark_bytes);
+    GPK_CUDA_TRY(cudaMemcpyAsync(hm.data(), marks, mark_bytes, cudaMemcpyDeviceToHost, G->stream));
+    GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
+    std::vector<SepRegion> regions;
+    for (int p = 0; p < G->label_cap; ++p) {
+        const uint8_t* m = hm.data() + (size_t)p * span;
+        bool any = false;
+        for (int k = 0; k < D.Nx && !any; ++k) any = m[k] != 0;
+        if (!any) continue;
+        SepRegion g{};
+        g.label = p;
+        auto box = [&](const uint8_t* mk, int n, int& o, int& c) {
+            int a, len;
+            arc_of(mk, n, a, len);
+            c = len + 4;
+            o = a - 2 < 0 ? a - 2 + n : a - 2;
+            if (c >= n) { o = 0; c = n; }
+        };
+        auto ext = [&](int o, int c, int n, int& s, int& e) {
+            e = c + 2 * R < n ? c + 2 * R : n;
+            s = wrap_any(o - R, n);
+        };
+        box(m, D.Nx, g.ox, g.nx);
+        box(m + D.Nx, D.Ny, g.oy, g.ny);
+        box(m + D.Nx + D.Ny, D.Nz, g.oz, g.nz);
+        ext(g.oy, g.ny, D.Ny, g.sy, g.ey);
+        ext(g.oz, g.nz, D.Nz, g.sz, g.ez);
+        regions.push_back(g);
+    }
+    if (regions.empty()) return GPK_OK;
+    // workspace (kept): values of the three passes, taps' run sums, label index and regions
+    const size_t cap1 = 8 * (size_t)D.N, cap2 = 5 * (size_t)D.N, cap3 = 4 * (size_t)D.N;
+    if (!G->sep_box) {
+        void* p = nullptr;
+        GPK_TRY(gpk_alloc(G, &p, sizeof(real) * (cap1 + cap2 + cap3 + (size_t)K * (K + 1))));
+        G->sep_box = p;
+        std::vector<real> runs((size_t)K * (K + 1), (real)0);
+        for (int s = 0; s < K; ++s) {
+            real acc = (real)0;
+            for (int l = 1; s + l <= K; ++l) {
+                acc += hk->gauss_w[s + l - 1];
+                runs[(size_t)s * (K + 1) + l] = acc;
+            }
+        }
+        GPK_CUDA_TRY(cudaMemcpyAsync((real*)p + cap1 + cap2 + cap3, runs.data(), sizeof(real) * runs.size(),
+                                     cudaMemcpyHostToDevice, G->stream));
+        GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
+    }
+    real* t1 = (real*)G->sep_box;
+    real* t2 = t1 + cap1;
+    real* s = t2 + cap2;
+    const real* runs = s + cap3;
+    const size_t table = ((sizeof(int32_t) * (size_t)G->label_cap + 15) & ~(size_t)15) + sizeof(SepRegion) * regions.size();
+    if (table > G->sep_table_bytes) {
+        // (an outgrown table stays allocated until the grid goes: it may still be read)
+        const size_t room = table + table / 2;
+        GPK_TRY(gpk_alloc(G, &G->sep_table, room));
+        G->sep_table_bytes = room;
+    }
+    std::vector<unsigned char> host(table);
+    for (size_t r0 = 0; r0 < regions.size();) {
+        size_t n = 0, u1 = 0, u2 = 0, u3 = 0;
+        int max_rows = 0, max_y = 0, max_z = 0, max_x = 0;
+        for (; r0 + n < regions.size(); ++n) {
+            SepRegion& g = regions[r0 + n];
+            const size_t a = (size_t)g.nx * g.ey * g.ez, b = (size_t)g.nx * g.ny * g.ez, c = (size_t)g.nx * g.ny * g.nz;
+            if (n > 0 && (u1 + a > cap1 || u2 + b > cap2 || u3 + c > cap3 || n == 65535)) break;
+            g.t1 = (long long)u1; g.t2 = (long long)u2; g.s = (long long)u3;
+            u1 += a; u2 += b; u3 += c;
+            max_rows = std::max(max_rows, g.ey * g.ez);
+            max_y = std::max(max_y, (int)std::min<long long>((long long)g.nx * ((g.ny + 7) / 8) * g.ez, 1 << 30));
+            max_z = std::max(max_z, (int)std::min<long long>((long long)g.nx * ((g.nz + 7) / 8) * g.ny, 1 << 30));
+            max_x = std::max(max_x, g.nx);
+        }
+        int32_t* index = (int32_t*)host.data();
+        std::fill(index, index + G->label_cap, -1);
+        for (size_t k = 0; k < n; ++k) index[regions[r0 + k].label] = (int32_t)k;
+        const size_t head = (sizeof(int32_t) * (size_t)G->label_cap + 15) & ~(size_t)15;
+        std::copy((const unsigned char*)&regions[r0], (const unsigned char*)(&regions[r0] + n), host.data() + head);
+        // (pageable memory: staged when the call returns, so `host` may be filled again)
+        GPK_CUDA_TRY(cudaMemcpyAsync(G->sep_table, host.data(), head + sizeof(SepRegion) * n, cudaMemcpyHostToDevice,
+                                     G->stream));
+        const SepRegion* dr = (const SepRegion*)((unsigned char*)G->sep_table + head);
+        const int words = (max_x + 2 * R + 31) / 32 + 1;
+        auto blocks = [&](long long work) { return (unsigned)std::max(1LL, std::min(work, 4096LL)); };
+        const size_t smem = sizeof(uint32_t) * 8 * (size_t)(words + 2);
+        if (smem > 48 * 1024) return -1;  // (rows of 48 000 cells)
+        k_sep_box_x<real><<<dim3(blocks((max_rows + 7) / 8), (unsigned)n), 256, smem, G->stream>>>(
+            D, G->phi, dr, R, words, (const real*)G->d_gauss, runs, t1);
+        k_sep_box_line<real, 1><<<dim3(blocks((max_y + 255) / 256), (unsigned)n), 256, 0, G->stream>>>(
+            D, dr, R, (const real*)G->d_gauss, t1, t2);
+        k_sep_box_line<real, 2><<<dim3(blocks((max_z + 255) / 256), (unsigned)n), 256, 0, G->stream>>>(
+            D, dr, R, (const real*)G->d_gauss, t2, s);
+        k_sep_box_eval<real><<<G->num_sms * 8, 256, 0, G->stream>>>(
+            D, G->active, &G->scal->n_active, G->phi, (const int32_t*)G->sep_table, dr, s, dx, kappa_limit,
+            (real*)G->f[GPK_FIELD_NX], (real*)G->f[GPK_FIELD_NY], (real*)G->f[GPK_FIELD_NZ],
+            (real*)G->f[GPK_FIELD_KAPPA]);
+        G->launches += 4;
+        GPK_CUDA_TRY(cudaGetLastError());
+        r0 += n;
+    }
+    return GPK_OK;
+}
+template int gpk_geometry_separable<float>(gpk_grid*, float, float);
+template int gpk_geometry_separable<double>(gpk_grid*, double, double);
