@@ -258,9 +258,9 @@ template <bool IS3D> struct BitTile;
 template <> struct BitTile<true> { static constexpr int TY = 8, TZ = 8; };
 template <> struct BitTile<false> { static constexpr int TY = 32, TZ = 1; };
 
-template <bool IS3D>
+template <bool IS3D, int R_ = 3>
 struct BitShape {
-    static constexpr int R = 3;
+    static constexpr int R = R_;
     static constexpr int TX = 32 - 2 * R, HX = 32;
     static constexpr int TY = BitTile<IS3D>::TY, TZ = BitTile<IS3D>::TZ;
     static constexpr int HY = TY + 2 * R, HZ = IS3D ? TZ + 2 * R : 1;
@@ -269,7 +269,7 @@ struct BitShape {
     static constexpr int NCELL = TX * TY * TZ;
     static constexpr int NH = NROW * HX;
     static constexpr int R2MAX = (IS3D ? 3 : 2) * R * R;
-    static constexpr int NL = 16;       // bitmaps per tile
+    static constexpr int NL = R == 3 ? 16 : 8;  // bitmaps per tile (wider kernels meet fewer pairs)
     static constexpr int HSLOT = 64;    // label hash slots
     static constexpr int NRS = 10;      // distinct dy^2 + dz^2 of a 7 x 7 row block
 };
@@ -587,16 +587,20 @@ __global__ void __launch_bounds__(256) k_bgr_scores_screen(Dims D, const int32_t
 }
 
 // ---------------------------------------------------------------------------
-// pair projection on pair bitmaps (radius 3)
+// pair projection on pair bitmaps (radii 3 to 9)
 // ---------------------------------------------------------------------------
 // A tap of the projection counts when its cell is an interface cell with the
 // centre's unordered label pair (src/gpk_physics.cpp:152-193).  A tile of
-// 26 x TY x TZ cells lists the distinct pairs of its interface cells; per
-// pair, one 32-bit word per halo row marks the halo cells holding that pair
-// (a halo row is 32 cells), so a row of 7 taps is a 7-bit pattern and only
-// its set bits add: num += w * (orientation_j * vn_j), den += w, in double,
-// z -> y -> x, as the reference adds them.  The 28 weights by squared
-// distance are kernel parameters (constant-bank operands of the products).
+// (32 - 2R) x TY x TZ cells lists the distinct pairs of its interface cells;
+// per pair, one 32-bit word per halo row marks the halo cells holding that
+// pair (a halo row is 32 cells), so a row of 2R+1 taps is a pattern of bits
+// and only its set bits add: num += w * (orientation_j * vn_j), den += w, in
+// double, z -> y -> x, as the reference adds them.
+//   R = 3: the taps are unrolled, the 28 weights by squared distance kernel
+//     parameters (constant-bank operands of the products).
+//   R > 3: a few per cent of the taps are set, so each cell walks its rows'
+//     set bits.  At R = 6 (sigma 5, 128^3) 0.88 -> 0.37 ms a step against
+//     comparing the pair of every tap.
 // Tiles with more than 64 distinct pairs sum their cells straight from global
 // memory in the same order.
 struct ProjW {
@@ -629,11 +633,12 @@ __device__ __forceinline__ int pair_slot_find(const unsigned long long* keys, un
 
 // One cell's sums read from global memory (tiles whose pairs overflow the
 // slot table): the same taps, order and operations as the bitmap path.
-template <typename real, bool IS3D>
+template <typename real, bool IS3D, int R>
 __device__ void proj_cell_global(const Dims& D, const int32_t* __restrict__ phi, const int32_t* __restrict__ phi_comp,
-                                 const uint8_t* __restrict__ mask, const real* __restrict__ vn, const ProjW& pw,
-                                 int x, int y, int z, unsigned long long key, double& num, double& den) {
-    constexpr int R = 3, RZ = IS3D ? 3 : 0;
+                                 const uint8_t* __restrict__ mask, const real* __restrict__ vn,
+                                 const double* __restrict__ w, int x, int y, int z, unsigned long long key,
+                                 double& num, double& den) {
+    constexpr int RZ = IS3D ? R : 0;
 #pragma unroll 1
     for (int dz = -RZ; dz <= RZ; ++dz)
 #pragma unroll 1
@@ -643,7 +648,7 @@ __device__ void proj_cell_global(const Dims& D, const int32_t* __restrict__ phi,
                 const int j = D.idx(IS3D ? wrap_any(z + dz, D.Nz) : 0, wrap_any(y + dy, D.Ny), wrap_any(x + dx, D.Nx));
                 const int32_t pj = phi[j], qj = phi_comp[j];
                 if (mask[j] && pj != qj && pair_key(pj, qj) == key) {
-                    const double wt = pw.w[dz * dz + dy * dy + dx * dx];
+                    const double wt = w[dz * dz + dy * dy + dx * dx];
                     const double sv = pj < qj ? (double)vn[j] : -(double)vn[j];
                     num = num + wt * sv;
                     den = den + wt;
@@ -651,17 +656,25 @@ __device__ void proj_cell_global(const Dims& D, const int32_t* __restrict__ phi,
             }
 }
 
-template <typename real, bool IS3D>
-__global__ void __launch_bounds__(256) k_projection_bits(Dims D, const int32_t* __restrict__ phi,
+// staged halo velocities: doubles at R = 3 (no conversion per tap), the grid's
+// type at larger radii (shared memory)
+template <typename real, int R> struct ProjStage { typedef real T; };
+template <typename real> struct ProjStage<real, 3> { typedef double T; };
+
+template <typename real, bool IS3D, int R>
+__global__ void __launch_bounds__(256, R > 3 && sizeof(real) == 4 ? 3 : 1) k_projection_bits(Dims D, const int32_t* __restrict__ phi,
                                                          const int32_t* __restrict__ phi_comp,
                                                          const uint8_t* __restrict__ mask, const real* __restrict__ vn,
                                                          real* __restrict__ vn_out, int ntx, int nty, int nl_cap,
-                                                         ProjW pw) {
-    typedef BitShape<IS3D> S;
-    constexpr int R = S::R, RZ = IS3D ? R : 0;
+                                                         const double* __restrict__ wtab, ProjW pw) {
+    typedef BitShape<IS3D, R> S;
+    typedef typename ProjStage<real, R>::T stage_t;
+    constexpr int RZ = IS3D ? R : 0;
     constexpr unsigned long long NONE = ~0ull;
-    extern __shared__ __align__(16) double svn[];  // S::NH signed velocities of the halo
-    __shared__ uint32_t bm[S::NL * S::NROWP];
+    extern __shared__ __align__(16) unsigned char proj_dyn[];
+    stage_t* svn = reinterpret_cast<stage_t*>(proj_dyn);  // S::NH signed velocities of the halo
+    uint32_t* bm = reinterpret_cast<uint32_t*>(svn + S::NH);
+    double* w = reinterpret_cast<double*>(bm + S::NL * S::NROWP + (S::NL * S::NROWP & 1));  // R > 3: weights by r2
     __shared__ int16_t cells[S::NCELL];
     __shared__ int8_t cslot[S::NCELL];  // pair slot of a listed cell; -1: no competitor, -2: slots full
     __shared__ unsigned long long keys[64];
@@ -704,6 +717,8 @@ __global__ void __launch_bounds__(256) k_projection_bits(Dims D, const int32_t* 
         if (tid == 0) { s_ncell = total; s_full = 0; }
     }
     if (tid < 64) keys[tid] = NONE;
+    if (R > 3)
+        for (int e = tid; e <= S::R2MAX; e += 256) w[e] = wtab[e];
     __syncthreads();
     const int ncell = s_ncell;
     if (ncell == 0) return;
@@ -739,7 +754,7 @@ __global__ void __launch_bounds__(256) k_projection_bits(Dims D, const int32_t* 
             const int i = D.idx(z0 + lz, y0 + ly, x0 + lx);
             const int32_t p = phi[i], q = phi_comp[i];
             double num = 0.0, den = 0.0;
-            proj_cell_global<real, IS3D>(D, phi, phi_comp, mask, vn, pw, x0 + lx, y0 + ly, z0 + lz, pair_key(p, q),
+            proj_cell_global<real, IS3D, R>(D, phi, phi_comp, mask, vn, wtab, x0 + lx, y0 + ly, z0 + lz, pair_key(p, q),
                                          num, den);
             real out = vn[i];
             if (den > 0.0) out = (p < q ? (real)1 : (real)-1) * (real)(num / den);
@@ -767,13 +782,14 @@ __global__ void __launch_bounds__(256) k_projection_bits(Dims D, const int32_t* 
         const int nb = np - b0 < nlb ? np - b0 : nlb;
         for (int e = tid; e < nb * S::NROWP; e += 256) bm[e] = 0u;
         __syncthreads();
-        // a warp takes four rows at a time, their loads issued together
-        for (int r0 = warp; r0 < S::NROW; r0 += 32) {
-            int32_t pj[4], qj[4];
-            uint8_t mj[4];
-            real vj[4];
+        // a warp takes U rows at a time, their loads issued together
+        constexpr int U = R == 3 ? 4 : 8;
+        for (int r0 = warp; r0 < S::NROW; r0 += 8 * U) {
+            int32_t pj[U], qj[U];
+            uint8_t mj[U];
+            real vj[U];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < U; ++u) {
                 const int r = r0 + 8 * u;
                 if (r < S::NROW) {
                     const int j = rowbase[r] + xw;
@@ -784,12 +800,12 @@ __global__ void __launch_bounds__(256) k_projection_bits(Dims D, const int32_t* 
                 }
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < U; ++u) {
                 const int r = r0 + 8 * u;
                 if (r >= S::NROW) break;
                 const bool valid = mj[u] && pj[u] != qj[u];
                 const unsigned long long key = valid ? pair_key(pj[u], qj[u]) : NONE;
-                if (b0 == 0) svn[r * S::HX + lane] = valid ? (pj[u] < qj[u] ? (double)vj[u] : -(double)vj[u]) : 0.0;
+                if (b0 == 0) svn[r * S::HX + lane] = (stage_t)(valid ? (pj[u] < qj[u] ? vj[u] : -vj[u]) : (real)0);
                 const unsigned grp = __match_any_sync(0xffffffffu, key);
                 if (key != NONE && lane == __ffs(grp) - 1) {
                     const int sl = pair_slot_find(keys, key);
@@ -810,24 +826,52 @@ __global__ void __launch_bounds__(256) k_projection_bits(Dims D, const int32_t* 
             const int lx = lc % S::TX, ly = (lc / S::TX) % S::TY, lz = lc / (S::TX * S::TY);
             const int rc = (IS3D ? lz * S::HY : 0) + ly;  // halo row of tap (-RZ, -R)
             const uint32_t* bmb = bm + d * S::NROWP + rc;
-            const double* sv = svn + rc * S::HX + lx;
+            const stage_t* sv = svn + rc * S::HX + lx;
             double num = 0.0, den = 0.0;
-#pragma unroll
-            for (int dz = -RZ; dz <= RZ; ++dz)
-#pragma unroll
-                for (int dy = -R; dy <= R; ++dy) {
-                    const int ro = (dz + RZ) * S::HY + dy + R;
-                    const uint32_t bits = (bmb[ro] >> lx) & 0x7Fu;
-                    if (!bits) continue;
-                    const double* s = sv + ro * S::HX;
-#pragma unroll
-                    for (int k = 0; k < 2 * R + 1; ++k)
-                        if (bits & (1u << k)) {
-                            const double wt = pw.w[dz * dz + dy * dy + (k - R) * (k - R)];
-                            num = num + wt * s[k];
-                            den = den + wt;
+            if constexpr (R > 3) {
+#pragma unroll 1
+                for (int dz = -RZ; dz <= RZ; ++dz)
+#pragma unroll 1
+                    for (int dy = -R; dy <= R; ++dy) {
+                        const int ro = (dz + RZ) * S::HY + dy + R;
+                        uint32_t bits = (bmb[ro] >> lx) & ((1u << (2 * R + 1)) - 1u);
+                        const double* wr = w + dz * dz + dy * dy;
+                        const stage_t* s = sv + ro * S::HX;
+                        // two taps' loads at a time, their additions in order
+                        while (bits) {
+                            const int k0 = __ffs(bits) - 1;
+                            bits &= bits - 1u;
+                            const bool two = bits != 0u;
+                            const int k1 = two ? __ffs(bits) - 1 : k0;
+                            bits &= bits - 1u;
+                            const double w0 = wr[(k0 - R) * (k0 - R)], w1 = wr[(k1 - R) * (k1 - R)];
+                            const double p0 = w0 * (double)s[k0], p1 = w1 * (double)s[k1];
+                            num = num + p0;
+                            den = den + w0;
+                            if (two) {
+                                num = num + p1;
+                                den = den + w1;
+                            }
                         }
-                }
+                    }
+            } else {
+#pragma unroll
+                for (int dz = -RZ; dz <= RZ; ++dz)
+#pragma unroll
+                    for (int dy = -R; dy <= R; ++dy) {
+                        const int ro = (dz + RZ) * S::HY + dy + R;
+                        const uint32_t bits = (bmb[ro] >> lx) & 0x7Fu;
+                        if (!bits) continue;
+                        const stage_t* s = sv + ro * S::HX;
+#pragma unroll
+                        for (int k = 0; k < 2 * R + 1; ++k)
+                            if (bits & (1u << k)) {
+                                const double wt = pw.w[dz * dz + dy * dy + (k - R) * (k - R)];
+                                num = num + wt * s[k];
+                                den = den + wt;
+                            }
+                    }
+            }
             const int i = D.idx(z0 + lz, y0 + ly, x0 + lx);
             const int32_t p = phi[i], q = phi_comp[i];
             real out = vn[i];
@@ -838,23 +882,26 @@ __global__ void __launch_bounds__(256) k_projection_bits(Dims D, const int32_t* 
     }
 }
 
-template <typename real, bool IS3D>
+template <typename real, bool IS3D, int R>
 static int launch_projection_bits(gpk_grid* G) {
-    typedef BitShape<IS3D> S;
+    typedef BitShape<IS3D, R> S;
     const HostKernels<real>* hk = (const HostKernels<real>*)G->host_kernels;
-    if (hk->proj_w.size() > 28) return -1;
     ProjW pw{};
-    for (size_t k = 0; k < hk->proj_w.size(); ++k) pw.w[k] = hk->proj_w[k];
+    for (size_t k = 0; k < hk->proj_w.size() && k < 28; ++k) pw.w[k] = hk->proj_w[k];
     const Dims D = G->d;
     const int ntx = (D.Nx + S::TX - 1) / S::TX, nty = (D.Ny + S::TY - 1) / S::TY, ntz = (D.Nz + S::TZ - 1) / S::TZ;
-    const size_t smem = sizeof(double) * S::NH;
+    constexpr size_t smem = sizeof(typename ProjStage<real, R>::T) * S::NH +
+                            4 * (size_t)(S::NL * S::NROWP + (S::NL * S::NROWP & 1)) +
+                            (R > 3 ? sizeof(double) * (S::R2MAX + 1) : 0);
+    // (8 KB: the static lists)
+    if (smem + 8 * 1024 > 227 * 1024) return -1;
     // set once per process (thread-safe initialisation of a function-local static)
     static const cudaError_t attr_rc = cudaFuncSetAttribute(
-        k_projection_bits<real, IS3D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_projection_bits<real, IS3D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     GPK_CUDA_TRY(attr_rc);
-    k_projection_bits<real, IS3D><<<ntx * nty * ntz, 256, smem, G->stream>>>(
+    k_projection_bits<real, IS3D, R><<<ntx * nty * ntz, 256, smem, G->stream>>>(
         D, G->phi, G->phi_comp, G->mask, (const real*)G->f[GPK_FIELD_VN], (real*)G->vn2, ntx, nty,
-        G->geometry_kernel == 2 ? 1 : S::NL, pw);
+        G->geometry_kernel == 2 ? 1 : S::NL, G->d_proj_w, pw);
     G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     return GPK_OK;
@@ -925,30 +972,24 @@ int gpk_bgr_scores_tiled(gpk_grid* G, int radius, real* res, real* best, const u
                        : launch_scores_screen<real, false>(G, res, best, gate);
 }
 
-// Tiled projection for the radii ceil(3 s) of the velocity kernel (s =
-// clamp(0.375 sigma, 0.85, 3) in 3-D: radii 3 to 9) whose 3-D halo tile fits
-// in the 227 KB of shared memory: 3 to 8 in FP32, 3 to 6 in FP64 (2-D: 3 to
-// 9).  -1 otherwise (the per-cell kernel runs).
-template <typename real, int R>
-static constexpr bool proj_fits() {
-    // dynamic halo arrays plus 8 KB for the static cell list, weights and scan
-    return (size_t)LocShape<R, true>::NH * (sizeof(int2) + sizeof(real)) + 8 * 1024 <= 227 * 1024;
-}
-
+// Projection on pair bitmaps for the radii ceil(3 s) of the velocity kernel (s =
+// clamp(0.375 sigma, 0.85, 3) in 3-D, 0.85 in 2-D: radii 3 to 9, and 3); -1
+// where the halo does not fit in shared memory (FP64 at R = 9: the per-cell
+// kernel runs).  Kind 3 keeps the pair-compare tiles at R = 3 (comparison runs).
 template <typename real, int R>
 static int projection_r(gpk_grid* G) {
-    if (!G->d.is3d()) return launch_projection<real, R, false>(G);
-    if constexpr (proj_fits<real, R>()) return launch_projection<real, R, true>(G);
-    return -1;
+    if constexpr (R == 3) {
+        if (!G->d.is3d()) return launch_projection_bits<real, false, R>(G);
+    }
+    return G->d.is3d() ? launch_projection_bits<real, true, R>(G) : -1;
 }
 
 template <typename real>
 int gpk_projection_tiled(gpk_grid* G, int radius) {
     switch (radius) {
         case 3:
-            // pair bitmaps; kind 3 keeps the pair-compare tiles (comparison runs)
-            if (G->geometry_kernel != 3)
-                return G->d.is3d() ? launch_projection_bits<real, true>(G) : launch_projection_bits<real, false>(G);
+            if (G->geometry_kernel == 3)
+                return G->d.is3d() ? launch_projection<real, 3, true>(G) : launch_projection<real, 3, false>(G);
             return projection_r<real, 3>(G);
         case 4: return projection_r<real, 4>(G);
         case 5: return projection_r<real, 5>(G);
