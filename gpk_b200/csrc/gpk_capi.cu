@@ -354,8 +354,8 @@ extern "C" int gpk_grid_create(int Nz, int Ny, int Nx, double dx, const gpk_ther
     ALLOC(G->vn2, rb);
     ALLOC(G->c_new, rb);
     ALLOC(G->active, 4 * N);
-    G->ntiles = (int)((N + 2047) / 2048);
-    ALLOC(G->tile_off, 4 * (size_t)(2 * G->ntiles + 8));
+    const size_t list_bytes = 16 + 8 * ((N + 2047) / 2048);
+    ALLOC(G->list_state, list_bytes);
     ALLOC(G->alpha_new_a, rb + 16);
     ALLOC(G->cand, 4 * N);
     ALLOC(G->cand_info, 16 * N);
@@ -390,7 +390,9 @@ extern "C" int gpk_grid_create(int Nz, int Ny, int Nx, double dx, const gpk_ther
         return fail(GPK_ERR_OUT_OF_MEMORY);
     }
     std::memset(G->h_scal, 0, sizeof(StepScalars));
-    if (cudaMemsetAsync(G->scal, 0, sizeof(StepScalars), G->stream) != cudaSuccess) return fail(GPK_ERR_CUDA);
+    if (cudaMemsetAsync(G->scal, 0, sizeof(StepScalars), G->stream) != cudaSuccess ||
+        cudaMemsetAsync(G->list_state, 0, list_bytes, G->stream) != cudaSuccess)
+        return fail(GPK_ERR_CUDA);
     rc = precision == GPK_PREC_F32 ? gpk_build_tables<float>(G) : gpk_build_tables<double>(G);
     if (rc != GPK_OK) return fail(rc);
     rc = precision == GPK_PREC_F32 ? init_fields<float>(G) : init_fields<double>(G);

@@ -69,8 +69,7 @@ struct gpk_grid {
     void* solid_old = nullptr; void* s_new = nullptr; uint8_t* grew = nullptr;
     int have_solid_old = 0;
     int32_t* active = nullptr;             // sorted interface cells
-    int32_t* tile_off = nullptr;           // compaction tile offsets
-    int ntiles = 0;
+    void* list_state = nullptr;            // ordered compactions: tickets and tile counts
     void* alpha_new_a = nullptr;           // per active position
     int32_t* cand = nullptr;               // candidate active positions
     int32_t* cand_info = nullptr;          // packed per-candidate wave state
@@ -182,4 +181,4 @@ int gpk_step_graph_supported(gpk_grid* G, std::string* why);
 // when G->step_graph holds a graph that replays two of its steps
 int gpk_grid_graph_prepare(gpk_grid* G, double dt, double dt_cap);
 void gpk_grid_graph_release(gpk_grid* G);
-int gpk_remap_gates(gpk_grid* G, int stage);
+int gpk_remap_second_gate(gpk_grid* G);

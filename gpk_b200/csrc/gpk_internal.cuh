@@ -86,7 +86,7 @@ struct StepScalars {
     // (0 in normal use; gpk_grid_inject_wait_timeout sets them for one launch)
     long long spin_limit;
     unsigned bar_extra;
-    unsigned pad2;
+    unsigned vmax_blocks;   // blocks that have added their largest velocity
     // remap passes inside a captured step: the first pass's exchanges and
     // the gate of the second (3-D) pass
     unsigned long long exch_first, gate2;

@@ -30,167 +30,228 @@ static constexpr int MASK_TPB = 256;
 static constexpr int MASK_IPT = 8;
 static constexpr int MASK_TILE = MASK_TPB * MASK_IPT;
 
-// `item_counters` (may be null): the three counters of the geometry's items,
-// cleared here for the geometry that follows.
-// `gate` (may be null): when it points to zero the launch does nothing
-// (device-side skip of a stage inside a captured step)
-__global__ void __launch_bounds__(MASK_TPB) k_mask_tiles(Dims D, const int32_t* __restrict__ phi,
-                                                         uint8_t* __restrict__ mask, int32_t* __restrict__ tile_cnt,
-                                                         unsigned* __restrict__ item_counters,
-                                                         const unsigned long long* gate = nullptr) {
-    if (gate && *gate == 0ull) return;
-    if (blockIdx.x == 0 && threadIdx.x < 3 && item_counters) item_counters[threadIdx.x] = 0u;
-    typedef cub::BlockReduce<int, MASK_TPB> BR;
-    __shared__ typename BR::TempStorage tmp;
-    const int base = blockIdx.x * MASK_TILE;
-    int cnt = 0;
-#pragma unroll
-    for (int k = 0; k < MASK_IPT; ++k) {
-        const int i = base + k * MASK_TPB + threadIdx.x;
-        if (i < D.N) {
-            int nb[6];
-            D.faces(i, nb);
-            const int32_t v = phi[i];
-            const uint8_t act = (uint8_t)((v != phi[nb[0]]) | (v != phi[nb[1]]) | (v != phi[nb[2]]) |
-                                          (v != phi[nb[3]]) | (v != phi[nb[4]]) | (v != phi[nb[5]]));
-            mask[i] = act;
-            cnt += act;
-        }
-    }
-    const int total = BR(tmp).Sum(cnt);
-    if (threadIdx.x == 0) tile_cnt[blockIdx.x] = total;
-}
+static constexpr int MASK_WARPS = MASK_TPB / 32;
 
-// The same mask when Nx is a multiple of 4: each thread takes groups of four
-// cells of a row (one int4 load per face-neighbour row or plane, two scalar
-// loads for the x neighbours of the group's ends) and stores four flags at once.
-__global__ void __launch_bounds__(MASK_TPB) k_mask_tiles4(Dims D, const int32_t* __restrict__ phi,
-                                                          uint8_t* __restrict__ mask, int32_t* __restrict__ tile_cnt,
-                                                          unsigned* __restrict__ item_counters,
-                                                         const unsigned long long* gate = nullptr) {
-    if (gate && *gate == 0ull) return;
-    if (blockIdx.x == 0 && threadIdx.x < 3 && item_counters) item_counters[threadIdx.x] = 0u;
-    typedef cub::BlockReduce<int, MASK_TPB> BR;
-    __shared__ typename BR::TempStorage tmp;
-    const int nx4 = D.Nx >> 2, plane = D.Nx * D.Ny;
-    int cnt = 0;
-#pragma unroll
-    for (int k = 0; k < MASK_IPT / 4; ++k) {
-        const int g = blockIdx.x * (MASK_TILE / 4) + k * MASK_TPB + threadIdx.x;
-        const int i = g * 4;
-        if (i < D.N) {
-            const int row = g / nx4, x = (g - row * nx4) * 4;
-            const int y = row % D.Ny, z = row / D.Ny;
-            const int oym = (y == 0 ? D.Ny - 1 : -1) * D.Nx, oyp = (y == D.Ny - 1 ? 1 - D.Ny : 1) * D.Nx;
-            const int ozm = (z == 0 ? D.Nz - 1 : -1) * plane, ozp = (z == D.Nz - 1 ? 1 - D.Nz : 1) * plane;
-            const int4 c = *reinterpret_cast<const int4*>(phi + i);
-            const int4 a = *reinterpret_cast<const int4*>(phi + i + oym);
-            const int4 b = *reinterpret_cast<const int4*>(phi + i + oyp);
-            const int4 d = *reinterpret_cast<const int4*>(phi + i + ozm);
-            const int4 e = *reinterpret_cast<const int4*>(phi + i + ozp);
-            const int32_t l = phi[i - x + (x == 0 ? D.Nx - 1 : x - 1)];
-            const int32_t r = phi[i - x + (x + 4 == D.Nx ? 0 : x + 4)];
-            uchar4 m;
-            m.x = (uint8_t)((c.x != l) | (c.x != c.y) | (c.x != a.x) | (c.x != b.x) | (c.x != d.x) | (c.x != e.x));
-            m.y = (uint8_t)((c.y != c.x) | (c.y != c.z) | (c.y != a.y) | (c.y != b.y) | (c.y != d.y) | (c.y != e.y));
-            m.z = (uint8_t)((c.z != c.y) | (c.z != c.w) | (c.z != a.z) | (c.z != b.z) | (c.z != d.z) | (c.z != e.z));
-            m.w = (uint8_t)((c.w != c.z) | (c.w != r) | (c.w != a.w) | (c.w != b.w) | (c.w != d.w) | (c.w != e.w));
-            *reinterpret_cast<uchar4*>(mask + i) = m;
-            cnt += m.x + m.y + m.z + m.w;
-        }
-    }
-    const int total = BR(tmp).Sum(cnt);
-    if (threadIdx.x == 0) tile_cnt[blockIdx.x] = total;
-}
+// Ordered compaction in one launch.  Blocks take their tiles in ticket order
+// and publish the tile's count, then the count up to and including it; a tile
+// adds up its predecessors' counts, looking back at 32 of them at a time
+// (those tiles' blocks are running or done, since tickets go up).  A word is
+// (launch tag << 32) | (2: inclusive, 1: own count) << 30 | count; the tag, kept
+// on the device so that captured launches need no argument, makes the words of
+// earlier launches read as not yet written.  The last block to finish starts
+// the next launch's tickets and tag.  Waits are bounded.
+struct ListState {
+    unsigned ticket, done, tag, pad;
+    unsigned long long word[1];  // one per tile
+};
 
-// Exclusive scan of tile counts in one block; writes the total.
-__global__ void __launch_bounds__(1024) k_scan_tiles(int32_t* __restrict__ tile, int ntiles, unsigned* __restrict__ total,
-                                                     const unsigned long long* gate = nullptr) {
-    if (gate && *gate == 0ull) return;
-    typedef cub::BlockScan<int, 1024> BS;
-    __shared__ typename BS::TempStorage tmp;
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
+__device__ __forceinline__ unsigned list_ticket(ListState* L, unsigned& tag) {
+    __shared__ unsigned s_ticket, s_tag;
+    if (threadIdx.x == 0) {
+        s_tag = *((volatile unsigned*)&L->tag) + 1u;
+        s_ticket = atomicAdd(&L->ticket, 1u);
+    }
     __syncthreads();
-    for (int base = 0; base < ntiles; base += 1024) {
-        const int i = base + threadIdx.x;
-        const int v = i < ntiles ? tile[i] : 0;
-        int ex, agg;
-        BS(tmp).ExclusiveSum(v, ex, agg);
-        if (i < ntiles) tile[i] = ex + carry;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += agg;
-        __syncthreads();
+    tag = s_tag;
+    return s_ticket;
+}
+// sum of the tiles before `tile` (one warp calls it); -1 when a wait gave up
+__device__ __forceinline__ long long list_prefix(ListState* L, unsigned tile, unsigned tag, unsigned own,
+                                                 unsigned* error) {
+    const int lane = threadIdx.x & 31;
+    const unsigned long long head = (unsigned long long)tag << 32;
+    volatile unsigned long long* w = L->word;
+    if (tile == 0) {
+        if (lane == 0) w[0] = head | (2ull << 30) | own;
+        return 0;
     }
-    if (threadIdx.x == 0) *total = (unsigned)carry;
+    if (lane == 0) w[tile] = head | (1ull << 30) | own;
+    long long sum = 0;
+    bool bad = false;
+    for (int base = (int)tile - 1; base >= 0; base -= 32) {
+        const int k = base - lane;
+        unsigned long long v = head | (2ull << 30);  // before the first tile: an inclusive count of 0
+        if (k >= 0) {
+            v = w[k];
+            for (int it = 0; (v >> 32) != tag; ++it) {
+                if (it > (1 << 24)) {
+                    bad = true;
+                    break;
+                }
+                __nanosleep(20);
+                v = w[k];
+            }
+        }
+        if (__any_sync(0xffffffffu, bad)) {
+            if (lane == 0) atomicCAS(error, 0u, (unsigned)GPK_ERR_TIMEOUT);
+            return -1;
+        }
+        const unsigned incl = __ballot_sync(0xffffffffu, ((v >> 30) & 3ull) == 2ull);
+        // counts up to the nearest inclusive one
+        const int stop = incl ? __ffs(incl) - 1 : 31;
+        sum += (long long)__reduce_add_sync(0xffffffffu, lane <= stop ? (unsigned)(v & 0x3fffffffull) : 0u);
+        if (incl) break;
+    }
+    if (lane == 0) w[tile] = head | (2ull << 30) | (unsigned long long)(sum + own);
+    return sum;
+}
+__device__ __forceinline__ void list_done(ListState* L, unsigned tag) {
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&L->done, 1u) == gridDim.x - 1) {
+        L->ticket = 0;
+        L->done = 0;
+        __threadfence();
+        *((volatile unsigned*)&L->tag) = tag;
+    }
 }
 
-// Writes the flat indices of flagged cells in increasing order.
-__global__ void __launch_bounds__(MASK_TPB) k_compact_u8(int n, const uint8_t* __restrict__ flag,
-                                                         const int32_t* __restrict__ tile_off, int32_t* __restrict__ out,
-                                                         const unsigned long long* gate = nullptr) {
-    if (gate && *gate == 0ull) return;
-    typedef cub::BlockScan<int, MASK_TPB> BS;
-    __shared__ typename BS::TempStorage tmp;
-    const int base = blockIdx.x * MASK_TILE;
-    int f[MASK_IPT];
-    int cnt = 0;
-#pragma unroll
-    for (int k = 0; k < MASK_IPT; ++k) {
-        const int i = base + threadIdx.x * MASK_IPT + k;
-        f[k] = (i < n) ? flag[i] : 0;
-        cnt += f[k];
-    }
-    int ex;
-    BS(tmp).ExclusiveSum(cnt, ex);
-    int pos = tile_off[blockIdx.x] + ex;
-#pragma unroll
-    for (int k = 0; k < MASK_IPT; ++k) {
-        const int i = base + threadIdx.x * MASK_IPT + k;
-        if (f[k]) out[pos++] = i;
-    }
+// What else a mask launch does on its way.
+struct MaskJob {
+    // `gate` (may be null): when it points to zero the launch does nothing
+    // (device-side skip of a stage inside a captured step)
+    const unsigned long long* gate = nullptr;
+    unsigned* item_counters = nullptr;  // the geometry's item counters, cleared
+    void* zero[7] = {};                 // fields set to zero everywhere
+    int nzero = 0, rsz = 4;
+    int32_t* copy = nullptr;            // phi copied here (phi_comp before a remap pass) ...
+    const unsigned long long* copy_cond = nullptr;  // ... where this is not zero (null: always)
+    int reset = 0;                      // clears the step's counters
+    int clear_waves = 0;
+    int total = 0;                      // 1: forms the step's remap totals (2-D), 2: 3-D (before the gate is read)
+};
+
+// The step's counters as a remap pass left them become its totals.
+__device__ __forceinline__ void remap_total(StepScalars* s, bool is3d) {
+    s->remap_waves_sum += s->waves;  // the last pass (a skipped pass left 0 in both)
+    s->remap_props_sum += s->n_prop;
+    s->exchanges = is3d ? s->exch_first + (s->gate2 ? s->exch_pass : 0ull) : s->exch_pass;
 }
 
-// Tile counts of a u8 flag array whose valid length is read on the device.
-__global__ void __launch_bounds__(MASK_TPB) k_count_u8(const uint8_t* __restrict__ flag, const unsigned* __restrict__ n_ptr,
-                                                       int32_t* __restrict__ tile_cnt) {
-    typedef cub::BlockReduce<int, MASK_TPB> BR;
-    __shared__ typename BR::TempStorage tmp;
-    const int n = (int)*n_ptr;
-    const int base = blockIdx.x * MASK_TILE;
-    int cnt = 0;
-    for (int k = 0; k < MASK_IPT; ++k) {
-        const int i = base + k * MASK_TPB + threadIdx.x;
-        if (i < n) cnt += flag[i];
+// Interface mask (src/gpk_geometry.cpp:42-82) and the interface cells in
+// increasing order.  With W4 (Nx a multiple of 4) a thread takes four cells of
+// a row with one int4 load per face-neighbour row or plane and two scalar loads
+// for the x neighbours of the group's ends, and stores four flags at once.
+// One launch where the mask, a one-block scan of its tile counts and the
+// compaction took three, and the fields' memsets, the copy of phi and the
+// counters' resets up to nine more: a step of 64^2 takes 20 launches instead of 47.
+template <bool W4, int IPT>
+__global__ void __launch_bounds__(MASK_TPB) k_mask_list(Dims D, const int32_t* __restrict__ phi,
+                                                        uint8_t* __restrict__ mask, int32_t* __restrict__ active,
+                                                        StepScalars* s, ListState* L,
+                                                        const __grid_constant__ MaskJob job) {
+    if (job.total && blockIdx.x == 0 && threadIdx.x == 0) remap_total(s, job.total == 2);
+    if (job.gate && *job.gate == 0ull) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (job.reset) {
+            s->accepted = 0; s->deferred = 0; s->exchanges = 0; s->exch_pass = 0;
+            s->n_cand = 0; s->n_prop = 0; s->waves = 0; s->n_near = 0; s->vmax = 0.0;
+        }
+        if (job.clear_waves) s->waves = 0;
+        if (job.item_counters) job.item_counters[0] = job.item_counters[1] = job.item_counters[2] = 0u;
     }
-    const int total = BR(tmp).Sum(cnt);
-    if (threadIdx.x == 0) tile_cnt[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(MASK_TPB) k_compact_u8_dyn(const unsigned* __restrict__ n_ptr,
-                                                             const uint8_t* __restrict__ flag,
-                                                             const int32_t* __restrict__ tile_off,
-                                                             int32_t* __restrict__ out) {
-    typedef cub::BlockScan<int, MASK_TPB> BS;
-    __shared__ typename BS::TempStorage tmp;
-    const int n = (int)*n_ptr;
-    const int base = blockIdx.x * MASK_TILE;
-    int f[MASK_IPT];
-    int cnt = 0;
+    constexpr int TILE = MASK_TPB * IPT;
+    constexpr int G = W4 ? 4 : 1, ROUNDS = IPT / G, CHUNKS = ROUNDS * MASK_WARPS;
+    __shared__ int s_off[CHUNKS];
+    __shared__ long long s_base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned tag;
+    const unsigned tile = list_ticket(L, tag);
+    const bool copy = job.copy && (!job.copy_cond || *job.copy_cond != 0ull);
+    const int plane = D.Nx * D.Ny;
+    uint32_t f[ROUNDS];  // G flags each
+    unsigned bal[ROUNDS][G];
 #pragma unroll
-    for (int k = 0; k < MASK_IPT; ++k) {
-        const int i = base + threadIdx.x * MASK_IPT + k;
-        f[k] = (i < n) ? flag[i] : 0;
-        cnt += f[k];
-    }
-    int ex;
-    BS(tmp).ExclusiveSum(cnt, ex);
-    int pos = tile_off[blockIdx.x] + ex;
+    for (int k = 0; k < ROUNDS; ++k) {
+        const int i = (int)tile * TILE + (k * MASK_TPB + (int)threadIdx.x) * G;
+        f[k] = 0;
+        if (i < D.N) {
+            if (W4) {
+                const int nx4 = D.Nx >> 2, g = i >> 2;
+                const int row = g / nx4, x = (g - row * nx4) * 4;
+                const int y = row % D.Ny, z = row / D.Ny;
+                const int oym = (y == 0 ? D.Ny - 1 : -1) * D.Nx, oyp = (y == D.Ny - 1 ? 1 - D.Ny : 1) * D.Nx;
+                const int ozm = (z == 0 ? D.Nz - 1 : -1) * plane, ozp = (z == D.Nz - 1 ? 1 - D.Nz : 1) * plane;
+                const int4 c = *reinterpret_cast<const int4*>(phi + i);
+                const int4 a = *reinterpret_cast<const int4*>(phi + i + oym);
+                const int4 b = *reinterpret_cast<const int4*>(phi + i + oyp);
+                const int4 d = *reinterpret_cast<const int4*>(phi + i + ozm);
+                const int4 e = *reinterpret_cast<const int4*>(phi + i + ozp);
+                const int32_t l = phi[i - x + (x == 0 ? D.Nx - 1 : x - 1)];
+                const int32_t r = phi[i - x + (x + 4 == D.Nx ? 0 : x + 4)];
+                uchar4 m;
+                m.x = (uint8_t)((c.x != l) | (c.x != c.y) | (c.x != a.x) | (c.x != b.x) | (c.x != d.x) | (c.x != e.x));
+                m.y = (uint8_t)((c.y != c.x) | (c.y != c.z) | (c.y != a.y) | (c.y != b.y) | (c.y != d.y) | (c.y != e.y));
+                m.z = (uint8_t)((c.z != c.y) | (c.z != c.w) | (c.z != a.z) | (c.z != b.z) | (c.z != d.z) | (c.z != e.z));
+                m.w = (uint8_t)((c.w != c.z) | (c.w != r) | (c.w != a.w) | (c.w != b.w) | (c.w != d.w) | (c.w != e.w));
+                *reinterpret_cast<uchar4*>(mask + i) = m;
+                f[k] = (uint32_t)m.x | (uint32_t)m.y << 1 | (uint32_t)m.z << 2 | (uint32_t)m.w << 3;
+                if (copy) *reinterpret_cast<int4*>(job.copy + i) = c;
+                for (int q = 0; q < job.nzero; ++q) {
+                    uint4* o = reinterpret_cast<uint4*>((unsigned char*)job.zero[q] + (size_t)i * job.rsz);
+                    o[0] = make_uint4(0, 0, 0, 0);
+                    if (job.rsz == 8) o[1] = make_uint4(0, 0, 0, 0);
+                }
+            } else {
+                int nb[6];
+                D.faces(i, nb);
+                const int32_t v = phi[i];
+                const uint8_t act = (uint8_t)((v != phi[nb[0]]) | (v != phi[nb[1]]) | (v != phi[nb[2]]) |
+                                              (v != phi[nb[3]]) | (v != phi[nb[4]]) | (v != phi[nb[5]]));
+                mask[i] = act;
+                f[k] = act;
+                if (copy) job.copy[i] = v;
+                for (int q = 0; q < job.nzero; ++q) {
+                    if (job.rsz == 4) ((uint32_t*)job.zero[q])[i] = 0u;
+                    else ((unsigned long long*)job.zero[q])[i] = 0ull;
+                }
+            }
+        }
+        int n = 0;
 #pragma unroll
-    for (int k = 0; k < MASK_IPT; ++k) {
-        const int i = base + threadIdx.x * MASK_IPT + k;
-        if (f[k]) out[pos++] = i;
+        for (int q = 0; q < G; ++q) {
+            bal[k][q] = __ballot_sync(0xffffffffu, (f[k] >> q) & 1u);
+            n += __popc(bal[k][q]);
+        }
+        if (lane == 0) s_off[k * MASK_WARPS + warp] = n;
     }
+    __syncthreads();
+    if (warp == 0) {
+        // exclusive prefix of the chunks, in cell order
+        int carry = 0;
+#pragma unroll
+        for (int c0 = 0; c0 < CHUNKS; c0 += 32) {
+            const int v = c0 + lane < CHUNKS ? s_off[c0 + lane] : 0;
+            int x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += u;
+            }
+            if (c0 + lane < CHUNKS) s_off[c0 + lane] = carry + x - v;
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+        const long long before = list_prefix(L, tile, tag, (unsigned)carry, &s->error);
+        if (lane == 0) {
+            s_base = before;
+            if (tile == gridDim.x - 1) s->n_active = before < 0 ? 0u : (unsigned)(before + carry);
+        }
+    }
+    __syncthreads();
+    if (s_base >= 0) {
+#pragma unroll
+        for (int k = 0; k < ROUNDS; ++k) {
+            const int i = (int)tile * TILE + (k * MASK_TPB + (int)threadIdx.x) * G;
+            const unsigned lt = (1u << lane) - 1u;
+            int pos = (int)s_base + s_off[k * MASK_WARPS + warp];
+#pragma unroll
+            for (int q = 0; q < G; ++q) pos += __popc(bal[k][q] & lt);
+#pragma unroll
+            for (int q = 0; q < G; ++q)
+                if ((f[k] >> q) & 1u) active[pos++] = i + q;
+        }
+    }
+    list_done(L, tag);
 }
 
 // ---------------------------------------------------------------------------
@@ -977,26 +1038,11 @@ template <> struct RealBits<double> {
 };
 
 template <typename real>
-__global__ void k_vmax(const int32_t* __restrict__ active, const unsigned* __restrict__ n_active,
-                       const real* __restrict__ vn, typename RealBits<real>::U* out) {
-    typedef typename RealBits<real>::U U;
-    const int na = (int)*n_active;
-    real m = (real)0;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x)
-        m = dmax(m, (real)fabs(vn[active[a]]));
-    typedef cub::BlockReduce<U, 256> BR;
-    __shared__ typename BR::TempStorage tmp;
-    // non-negative reals order like their bit patterns
-    const U agg = BR(tmp).Reduce(RealBits<real>::bits(m), cub::Max());
-    if (threadIdx.x == 0) atomicMax(out, agg);
-}
-
-// dt selection of GPKGrid::step (src/gpk_simulation.cpp:31-37)
-template <typename real>
-__global__ void k_select_dt(StepScalars* s, const typename RealBits<real>::U* vbits, real dx, real D, int is3d,
-                            double dt_req_d, double dt_cap_d) {
+__device__ __forceinline__ void select_dt(StepScalars* s, real vfound, real dx, real D, int is3d, double dt_req_d,
+                                          double dt_cap_d) {
+    // dt selection of GPKGrid::step (src/gpk_simulation.cpp:31-37)
     real vmax = (real)1e-30;
-    vmax = dmax(vmax, RealBits<real>::val(*vbits));
+    vmax = dmax(vmax, vfound);
     const real neighbors = is3d ? (real)6 : (real)4;
     const real dt_iface = (real)0.125 * dx / vmax;
     const real dt_diff = (D > (real)0) ? (real)0.4 * dx * dx / (neighbors * D) : (real)1e30;
@@ -1007,6 +1053,34 @@ __global__ void k_select_dt(StepScalars* s, const typename RealBits<real>::U* vb
     dt = dmin(dt, (real)dt_cap_d);
     s->dt = (double)dt;
     s->vmax = (double)vmax;
+    s->time += s->dt;
+}
+
+// Largest |vn| of the interface cells into *out (bits); with `s`, the last
+// block selects the step's dt from it and advances the time.
+template <typename real>
+__global__ void k_vmax(const int32_t* __restrict__ active, const unsigned* __restrict__ n_active,
+                       const real* __restrict__ vn, typename RealBits<real>::U* out, StepScalars* s, real dx, real D,
+                       int is3d, double dt_req_d, double dt_cap_d) {
+    typedef typename RealBits<real>::U U;
+    const int na = (int)*n_active;
+    real m = (real)0;
+    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x)
+        m = dmax(m, (real)fabs(vn[active[a]]));
+    typedef cub::BlockReduce<U, 256> BR;
+    __shared__ typename BR::TempStorage tmp;
+    // non-negative reals order like their bit patterns
+    const U agg = BR(tmp).Reduce(RealBits<real>::bits(m), cub::Max());
+    if (threadIdx.x == 0) {
+        atomicMax(out, agg);
+        if (s) {
+            __threadfence();
+            if (atomicAdd(&s->vmax_blocks, 1u) == gridDim.x - 1) {
+                s->vmax_blocks = 0;
+                select_dt<real>(s, RealBits<real>::val(atomicMax(out, (U)0)), dx, D, is3d, dt_req_d, dt_cap_d);
+            }
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1032,37 +1106,85 @@ __device__ __forceinline__ real normal_from_cell_step(int i, uint64_t step_id, u
     return sqrt((real)-2 * log(u1)) * cos((real)2 * dev_pi<real>() * u2);
 }
 
+// One tile of MASK_TILE interface cells per block; the candidates' positions
+// are listed in order (see ListState) in the same launch.
 template <typename real>
-__global__ void k_alpha(Dims D, const int32_t* __restrict__ active, const unsigned* __restrict__ n_active,
-                        const int32_t* __restrict__ phi, const int32_t* __restrict__ phi_comp,
-                        const real* __restrict__ vn, const real* __restrict__ T, real* __restrict__ alpha,
-                        real* __restrict__ alpha_new_a, uint8_t* __restrict__ cand_flag, StepScalars* s, real dx,
-                        int do_noise_flag, real M0, real kB, real noise_scale, uint64_t step_id,
-                        real near_tol, int32_t* __restrict__ near_list, int near_cap) {
+__global__ void __launch_bounds__(MASK_TPB)
+k_alpha(Dims D, const int32_t* __restrict__ active, const unsigned* __restrict__ n_active,
+        const int32_t* __restrict__ phi, const int32_t* __restrict__ phi_comp, const real* __restrict__ vn,
+        const real* __restrict__ T, real* __restrict__ alpha, real* __restrict__ alpha_new_a,
+        int32_t* __restrict__ cand, StepScalars* s, ListState* L, real dx, int do_noise_flag, real M0, real kB,
+        real noise_scale, uint64_t step_id, real near_tol, int32_t* __restrict__ near_list, int near_cap) {
+    __shared__ int s_off[MASK_IPT * MASK_WARPS];
+    __shared__ long long s_base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned tag;
+    const unsigned tile = list_ticket(L, tag);
+    const int na = (int)*n_active;
+    if ((long long)tile * MASK_TILE >= na) {
+        list_done(L, tag);
+        return;
+    }
     const real dt = (real)s->dt;
     const real idt = dt / dx;
     const real cell_vol = dx * dx * dx;
     const real inv_dt = (dt > (real)0) ? ((real)1 / dt) : (real)0;
     const bool do_noise = do_noise_flag && dt > (real)0;
     const real noise_amp = do_noise ? noise_scale * sqrt((real)2 * M0 * kB * inv_dt / dmax(cell_vol, (real)1e-30)) : (real)0;
-    const int na = (int)*n_active;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
-        const int i = active[a];
-        real vn_eff = vn[i];
-        if (do_noise) vn_eff += noise_amp * sqrt(dmax(T[i], (real)1)) * normal_from_cell_step<real>(i, step_id, 0xabcddcbaULL);
-        const real an = dmin(alpha[i] + vn_eff * idt, (real)1);
-        alpha_new_a[a] = an;
-        const bool other = phi_comp[i] != phi[i];
-        const bool cand = an <= (real)1e-6 && other;
-        cand_flag[a] = cand ? 1 : 0;
-        if (!cand) alpha[i] = an;
-        // near-threshold listing: the switching margin an - 1e-6 within
-        // near_tol of zero (order restored when the list is read)
-        if (other && fabs(an - (real)1e-6) <= near_tol) {
-            const unsigned q = atomicAdd(&s->n_near, 1u);
-            if (q < (unsigned)near_cap) near_list[q] = i;
+    unsigned bal[MASK_IPT];
+#pragma unroll
+    for (int k = 0; k < MASK_IPT; ++k) {
+        const int a = (int)tile * MASK_TILE + k * MASK_TPB + (int)threadIdx.x;
+        bool c = false;
+        if (a < na) {
+            const int i = active[a];
+            real vn_eff = vn[i];
+            if (do_noise) vn_eff += noise_amp * sqrt(dmax(T[i], (real)1)) * normal_from_cell_step<real>(i, step_id, 0xabcddcbaULL);
+            const real an = dmin(alpha[i] + vn_eff * idt, (real)1);
+            alpha_new_a[a] = an;
+            const bool other = phi_comp[i] != phi[i];
+            c = an <= (real)1e-6 && other;
+            if (!c) alpha[i] = an;
+            // near-threshold listing: the switching margin an - 1e-6 within
+            // near_tol of zero (order restored when the list is read)
+            if (other && fabs(an - (real)1e-6) <= near_tol) {
+                const unsigned q = atomicAdd(&s->n_near, 1u);
+                if (q < (unsigned)near_cap) near_list[q] = i;
+            }
+        }
+        bal[k] = __ballot_sync(0xffffffffu, c);
+        if (lane == 0) s_off[k * MASK_WARPS + warp] = __popc(bal[k]);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int carry = 0;
+#pragma unroll
+        for (int c0 = 0; c0 < MASK_IPT * MASK_WARPS; c0 += 32) {
+            const int v = s_off[c0 + lane];
+            int x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += u;
+            }
+            s_off[c0 + lane] = carry + x - v;
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+        const long long before = list_prefix(L, tile, tag, (unsigned)carry, &s->error);
+        if (lane == 0) {
+            s_base = before;
+            if ((int)tile == (na - 1) / MASK_TILE) s->n_cand = before < 0 ? 0u : (unsigned)(before + carry);
         }
     }
+    __syncthreads();
+    if (s_base >= 0) {
+#pragma unroll
+        for (int k = 0; k < MASK_IPT; ++k)
+            if ((bal[k] >> lane) & 1u)
+                cand[(int)s_base + s_off[k * MASK_WARPS + warp] + __popc(bal[k] & ((1u << lane) - 1u))] =
+                    (int)tile * MASK_TILE + k * MASK_TPB + (int)threadIdx.x;
+    }
+    list_done(L, tag);
 }
 
 // crossings without region identity: every candidate is accepted
@@ -1370,13 +1492,6 @@ __global__ void k_scale(int N, real* __restrict__ v, real f) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) v[i] *= f;
 }
 
-__global__ void k_advance_time(StepScalars* s) { s->time += s->dt; }
-
-__global__ void k_reset_step(StepScalars* s) {
-    s->accepted = 0; s->deferred = 0; s->exchanges = 0; s->exch_pass = 0;
-    s->n_cand = 0; s->n_prop = 0; s->waves = 0; s->n_near = 0;
-}
-
 }  // namespace gpk_dev
 
 using namespace gpk_dev;
@@ -1482,18 +1597,55 @@ static int sep_gauss3(const Dims& D, const real* in, const int32_t* phi, int32_t
 }
 
 // mask + sorted interface list (src/gpk_geometry.cpp:42-82)
-template <typename real>
-int gpk_interface_mask(gpk_grid* G, const unsigned long long* gate) {
-    const int nt = (G->d.N + MASK_TILE - 1) / MASK_TILE;
-    if (G->d.Nx % 4 == 0)
-        k_mask_tiles4<<<nt, MASK_TPB, 0, G->stream>>>(G->d, G->phi, G->mask, G->tile_off, G->item_counters, gate);
-    else
-        k_mask_tiles<<<nt, MASK_TPB, 0, G->stream>>>(G->d, G->phi, G->mask, G->tile_off, G->item_counters, gate);
-    k_scan_tiles<<<1, 1024, 0, G->stream>>>(G->tile_off, nt, &G->scal->n_active, gate);
-    k_compact_u8<<<nt, MASK_TPB, 0, G->stream>>>(G->d.N, G->mask, G->tile_off, G->active, gate);
-    G->launches += 3;
+static int launch_mask(gpk_grid* G, MaskJob job) {
+    // larger tiles for larger grids: with tiles of 2048 cells the tickets of
+    // 8192 blocks and their look-back chain cost more than the cells of 256^3
+    // (129 -> 88 us a launch with tiles of 8192); small grids want the blocks
+    const bool large = G->d.N >= 1 << 22;
+    const int tile = MASK_TPB * (large ? 32 : 8);
+    const int nt = (G->d.N + tile - 1) / tile;
+    job.item_counters = G->item_counters;
+    job.rsz = (int)G->rsz;
+    ListState* L = (ListState*)G->list_state;
+    const Dims D = G->d;
+    if (D.Nx % 4 == 0) {
+        if (large) k_mask_list<true, 32><<<nt, MASK_TPB, 0, G->stream>>>(D, G->phi, G->mask, G->active, G->scal, L, job);
+        else k_mask_list<true, 8><<<nt, MASK_TPB, 0, G->stream>>>(D, G->phi, G->mask, G->active, G->scal, L, job);
+    } else {
+        if (large) k_mask_list<false, 32><<<nt, MASK_TPB, 0, G->stream>>>(D, G->phi, G->mask, G->active, G->scal, L, job);
+        else k_mask_list<false, 8><<<nt, MASK_TPB, 0, G->stream>>>(D, G->phi, G->mask, G->active, G->scal, L, job);
+    }
+    G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     return GPK_OK;
+}
+template <typename real>
+int gpk_interface_mask(gpk_grid* G, const unsigned long long* gate) {
+    MaskJob job;
+    job.gate = gate;
+    return launch_mask(G, job);
+}
+// the first mask of a step (or of a geometry alone): the geometry's fields start at zero
+static MaskJob geometry_job(gpk_grid* G) {
+    MaskJob job;
+    for (int f : {GPK_FIELD_NX, GPK_FIELD_NY, GPK_FIELD_NZ, GPK_FIELD_KAPPA}) job.zero[job.nzero++] = G->f[f];
+    return job;
+}
+// whether the model computes its own elastic proxy
+template <typename real>
+static bool elastic_proxy(const gpk_grid* G) {
+    const gpk_thermo_desc& th = G->th;
+    return !G->external_elastic && th.elastic_enabled && !((real)th.elastic_modulus <= (real)0) &&
+           !((real)th.eigenstrain_coeff == (real)0 && (real)th.lambda_s == (real)0);
+}
+template <typename real>
+static MaskJob step_job(gpk_grid* G) {
+    MaskJob job = geometry_job(G);
+    job.zero[job.nzero++] = G->f[GPK_FIELD_VN];
+    job.zero[job.nzero++] = G->vn2;
+    if (!G->external_elastic && !elastic_proxy<real>(G)) job.zero[job.nzero++] = G->f[GPK_FIELD_E_EL];
+    job.reset = 1;
+    return job;
 }
 
 template <typename real>
@@ -1501,8 +1653,6 @@ static int geometry(gpk_grid* G) {
     HostKernels<real>* hk = (HostKernels<real>*)G->host_kernels;
     const Dims D = G->d;
     const size_t nb = G->rsz * D.N;
-    for (int f : {GPK_FIELD_NX, GPK_FIELD_NY, GPK_FIELD_NZ, GPK_FIELD_KAPPA})
-        GPK_CUDA_TRY(cudaMemsetAsync(G->f[f], 0, nb, G->stream));
     const real dx = (real)G->dx;
     const real kappa_limit = (real)1 / (hk->gauss_sigma * dx);
     real* nx = (real*)G->f[GPK_FIELD_NX];
@@ -1589,12 +1739,8 @@ static int elastic(gpk_grid* G) {
     const gpk_thermo_desc& th = G->th;
     const Dims D = G->d;
     real* E = (real*)G->f[GPK_FIELD_E_EL];
-    if (G->external_elastic) return GPK_OK;  // E_el as the caller supplied it
-    if (!th.elastic_enabled || (real)th.elastic_modulus <= (real)0 ||
-        ((real)th.eigenstrain_coeff == (real)0 && (real)th.lambda_s == (real)0)) {
-        GPK_CUDA_TRY(cudaMemsetAsync(E, 0, G->rsz * D.N, G->stream));
-        return GPK_OK;
-    }
+    // E_el as the caller supplied it, or zero (the step's first mask launch)
+    if (!elastic_proxy<real>(G)) return GPK_OK;
     if (!G->eps_star) {
         GPK_TRY(gpk_alloc(G, &G->eps_star, G->rsz * D.N));
         GPK_TRY(gpk_alloc(G, &G->eps_smooth, G->rsz * D.N));
@@ -1713,9 +1859,8 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
     HostKernels<real>* hk = (HostKernels<real>*)G->host_kernels;
     const Dims D = G->d;
     const gpk_thermo_desc& th = G->th;
-    const int ga = G->num_sms * 8;
-    k_reset_step<<<1, 1, 0, G->stream>>>(G->scal);
-    G->launches++;
+    // grid-stride launches over at most N items
+    const int ga = grid_for(G, D.N);
     // flood-fill stamps: restart before the 32-bit cursor can wrap
     if (G->h_scal->stamp > 0x70000000u) {
         GPK_CUDA_TRY(cudaMemsetAsync(G->stamp, 0, sizeof(uint32_t) * D.N, G->stream));
@@ -1724,7 +1869,7 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
         G->h_scal->stamp = 0;
     }
     GPK_TRY(gpk_stage_begin(G, GPK_STAGE_MASK));
-    GPK_TRY(gpk_interface_mask<real>(G));
+    GPK_TRY(launch_mask(G, step_job<real>(G)));
     GPK_TRY(gpk_stage_end(G, GPK_STAGE_MASK));
     GPK_TRY(gpk_stage_begin(G, GPK_STAGE_GEOMETRY));
     GPK_TRY(geometry<real>(G));
@@ -1733,7 +1878,6 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
     GPK_TRY(elastic<real>(G));
     ThermoDev TD = make_thermo_dev(th);
     if (G->external_elastic) TD.t.elastic_enabled = 1;
-    GPK_CUDA_TRY(cudaMemsetAsync(G->f[GPK_FIELD_VN], 0, G->rsz * D.N, G->stream));
     k_velocities<real><<<ga, 256, 0, G->stream>>>(
         D, TD, G->active, &G->scal->n_active, G->phi, G->phi_comp, (const real*)G->f[GPK_FIELD_C],
         (const real*)G->f[GPK_FIELD_T], (const real*)G->f[GPK_FIELD_G], (const real*)G->f[GPK_FIELD_RHO],
@@ -1743,7 +1887,6 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
     GPK_TRY(gpk_stage_end(G, GPK_STAGE_VELOCITY));
     // projection into vn2 (zero at bulk cells), then swap
     GPK_TRY(gpk_stage_begin(G, GPK_STAGE_PROJECTION));
-    GPK_CUDA_TRY(cudaMemsetAsync(G->vn2, 0, G->rsz * D.N, G->stream));
     const int prc = G->geometry_kernel != 1 ? gpk_projection_tiled<real>(G, hk->proj_radius) : -1;
     if (prc == -1)
         k_projection<real><<<ga, 256, 0, G->stream>>>(D, G->active, &G->scal->n_active, G->phi, G->phi_comp, G->mask,
@@ -1755,9 +1898,8 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
     // stable dt
     typedef typename RealBits<real>::U U;
     U* vbits = (U*)&G->scal->vmax;
-    GPK_CUDA_TRY(cudaMemsetAsync(vbits, 0, sizeof(double), G->stream));
-    k_vmax<real><<<ga, 256, 0, G->stream>>>(G->active, &G->scal->n_active, (const real*)G->f[GPK_FIELD_VN], vbits);
-    k_select_dt<real><<<1, 1, 0, G->stream>>>(G->scal, vbits, (real)G->dx, (real)G->D, D.is3d() ? 1 : 0, dt_req, dt_cap);
+    k_vmax<real><<<ga, 256, 0, G->stream>>>(G->active, &G->scal->n_active, (const real*)G->f[GPK_FIELD_VN], vbits,
+                                            G->scal, (real)G->dx, (real)G->D, D.is3d() ? 1 : 0, dt_req, dt_cap);
     G->launches += 4;
     GPK_TRY(gpk_stage_end(G, GPK_STAGE_PROJECTION));
     GPK_TRY(gpk_stage_begin(G, GPK_STAGE_ALPHA));
@@ -1773,17 +1915,11 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
         G->launches++;
     }
     // alpha integration and candidates
-    uint8_t* cflag = (uint8_t*)G->ero_target;  // active-indexed scratch flags
-    k_alpha<real><<<ga, 256, 0, G->stream>>>(D, G->active, &G->scal->n_active, G->phi, G->phi_comp,
-                                             (const real*)G->f[GPK_FIELD_VN], (const real*)G->f[GPK_FIELD_T],
-                                             (real*)G->f[GPK_FIELD_ALPHA], (real*)G->alpha_new_a, cflag, G->scal,
-                                             (real)G->dx, th.stochastic, (real)th.M0, (real)th.kB, (real)th.noise_scale,
-                                             G->step_id, (real)G->near_tol, G->near_list, D.N);
-    const int nt = (D.N + MASK_TILE - 1) / MASK_TILE;
-    int32_t* ctile = G->tile_off + nt + 1;
-    k_count_u8<<<nt, MASK_TPB, 0, G->stream>>>(cflag, &G->scal->n_active, ctile);
-    k_scan_tiles<<<1, 1024, 0, G->stream>>>(ctile, nt, &G->scal->n_cand);
-    k_compact_u8_dyn<<<nt, MASK_TPB, 0, G->stream>>>(&G->scal->n_active, cflag, ctile, G->cand);
+    k_alpha<real><<<(D.N + MASK_TILE - 1) / MASK_TILE, MASK_TPB, 0, G->stream>>>(
+        D, G->active, &G->scal->n_active, G->phi, G->phi_comp, (const real*)G->f[GPK_FIELD_VN],
+        (const real*)G->f[GPK_FIELD_T], (real*)G->f[GPK_FIELD_ALPHA], (real*)G->alpha_new_a, G->cand, G->scal,
+        (ListState*)G->list_state, (real)G->dx, th.stochastic, (real)th.M0, (real)th.kB, (real)th.noise_scale,
+        G->step_id, (real)G->near_tol, G->near_list, D.N);
     G->launches += 4;
     GPK_CUDA_TRY(cudaGetLastError());
     GPK_TRY(gpk_stage_end(G, GPK_STAGE_ALPHA));
@@ -1809,21 +1945,33 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
     // balanced Gaussian remap, twice in 3-D when the first pass exchanged
     if (G->h_scal->accepted > 0) {
         GPK_TRY(gpk_stage_begin(G, GPK_STAGE_REMAP));
-        GPK_TRY(gpk_interface_mask<real>(G));
-        GPK_CUDA_TRY(cudaMemsetAsync(&G->scal->waves, 0, sizeof(unsigned), G->stream));
+        // phi_comp <- phi before each pass
+        MaskJob job;
+        job.copy = G->phi_comp;
+        job.clear_waves = 1;
+        GPK_TRY(launch_mask(G, job));
         GPK_TRY(gpk_remap_pass<real>(G));
-        GPK_TRY(gpk_interface_mask<real>(G));
         const bool tiled_scores = G->geometry_kernel != 1 && hk->remap_radius == 3;
-        if (D.is3d() && tiled_scores) {
+        const bool second = D.is3d() && tiled_scores;
+        job = MaskJob();
+        if (second) {
+            job.copy = G->phi_comp;
+            job.copy_cond = &G->scal->exch_pass;
+        } else if (!D.is3d()) {
+            job.total = 1;
+        }
+        GPK_TRY(launch_mask(G, job));
+        if (second) {
             // the second pass under the device-side gate of the first pass's
             // exchanges (no host round trip between the passes); the pass
             // statistics and the exchange total are formed on the device
-            GPK_TRY(gpk_remap_gates(G, 0));
+            GPK_TRY(gpk_remap_second_gate(G));
             GPK_TRY(gpk_remap_pass<real>(G, &G->scal->gate2));
-            GPK_TRY(gpk_interface_mask<real>(G, &G->scal->gate2));
-            GPK_TRY(gpk_remap_gates(G, 1));
+            job = MaskJob();
+            job.gate = &G->scal->gate2;
+            job.total = 2;
+            GPK_TRY(launch_mask(G, job));
         } else if (!D.is3d()) {
-            GPK_TRY(gpk_remap_gates(G, 1));
         } else {
             GPK_TRY(gpk_sync_scalars(G));
             G->wave_stats[1] += G->h_scal->waves;
@@ -1833,6 +1981,9 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
             if (first > 0) {
                 GPK_CUDA_TRY(cudaMemsetAsync(&G->scal->exch_pass, 0, sizeof(unsigned long long), G->stream));
                 GPK_CUDA_TRY(cudaMemsetAsync(&G->scal->waves, 0, sizeof(unsigned), G->stream));
+                GPK_CUDA_TRY(cudaMemsetAsync(&G->scal->n_prop, 0, sizeof(unsigned), G->stream));
+                GPK_CUDA_TRY(cudaMemcpyAsync(G->phi_comp, G->phi, sizeof(int32_t) * D.N, cudaMemcpyDeviceToDevice,
+                                             G->stream));
                 GPK_TRY(gpk_remap_pass<real>(G));
                 GPK_TRY(gpk_interface_mask<real>(G));
                 GPK_TRY(gpk_sync_scalars(G));
@@ -1864,8 +2015,6 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
         }
     }
     GPK_TRY(gpk_stage_end(G, GPK_STAGE_TRANSPORT));
-    k_advance_time<<<1, 1, 0, G->stream>>>(G->scal);
-    G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     GPK_TRY(gpk_stage_collect(G));
     ++G->step_id;
@@ -1878,7 +2027,8 @@ int gpk_max_dt_impl(gpk_grid* G, double* out) {
     typedef typename RealBits<real>::U U;
     U* vbits = (U*)G->alpha_new_a;  // scratch word
     GPK_CUDA_TRY(cudaMemsetAsync(vbits, 0, sizeof(U), G->stream));
-    k_vmax<real><<<G->num_sms * 8, 256, 0, G->stream>>>(G->active, &G->scal->n_active, (const real*)G->f[GPK_FIELD_VN], vbits);
+    k_vmax<real><<<G->num_sms * 8, 256, 0, G->stream>>>(G->active, &G->scal->n_active, (const real*)G->f[GPK_FIELD_VN],
+                                                        vbits, nullptr, (real)0, (real)0, 0, 0.0, 0.0);
     U h = 0;
     GPK_CUDA_TRY(cudaMemcpyAsync(&h, vbits, sizeof(U), cudaMemcpyDeviceToHost, G->stream));
     GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
@@ -1982,21 +2132,17 @@ int gpk_step_graph_body(gpk_grid* G, double dt_req, double dt_cap) {
     const gpk_thermo_desc& th = G->th;
     // grid-stride launches over at most N items, sized for the grid's cells
     const int ga = (int)std::max(1LL, std::min((long long)G->num_sms * 8, ((long long)D.N + 255) / 256));
-    k_reset_step<<<1, 1, 0, G->stream>>>(G->scal);
-    G->launches++;
-    GPK_TRY(gpk_interface_mask<real>(G));
+    GPK_TRY(launch_mask(G, step_job<real>(G)));
     GPK_TRY(geometry<real>(G));
     GPK_TRY(elastic<real>(G));
     ThermoDev TD = make_thermo_dev(th);
     if (G->external_elastic) TD.t.elastic_enabled = 1;
-    GPK_CUDA_TRY(cudaMemsetAsync(G->f[GPK_FIELD_VN], 0, G->rsz * D.N, G->stream));
     k_velocities<real><<<ga, 256, 0, G->stream>>>(
         D, TD, G->active, &G->scal->n_active, G->phi, G->phi_comp, (const real*)G->f[GPK_FIELD_C],
         (const real*)G->f[GPK_FIELD_T], (const real*)G->f[GPK_FIELD_G], (const real*)G->f[GPK_FIELD_RHO],
         (const real*)G->f[GPK_FIELD_NX], (const real*)G->f[GPK_FIELD_NY], (const real*)G->f[GPK_FIELD_NZ],
         (const real*)G->f[GPK_FIELD_KAPPA], (const real*)G->f[GPK_FIELD_E_EL], (real*)G->f[GPK_FIELD_VN],
         (real*)G->f[GPK_FIELD_G_COMP]);
-    GPK_CUDA_TRY(cudaMemsetAsync(G->vn2, 0, G->rsz * D.N, G->stream));
     const int prc = gpk_projection_tiled<real>(G, hk->proj_radius);
     if (prc == -1)
         k_projection<real><<<ga, 256, 0, G->stream>>>(D, G->active, &G->scal->n_active, G->phi, G->phi_comp, G->mask,
@@ -2007,9 +2153,8 @@ int gpk_step_graph_body(gpk_grid* G, double dt_req, double dt_cap) {
     std::swap(G->f[GPK_FIELD_VN], G->vn2);
     typedef typename RealBits<real>::U U;
     U* vbits = (U*)&G->scal->vmax;
-    GPK_CUDA_TRY(cudaMemsetAsync(vbits, 0, sizeof(double), G->stream));
-    k_vmax<real><<<ga, 256, 0, G->stream>>>(G->active, &G->scal->n_active, (const real*)G->f[GPK_FIELD_VN], vbits);
-    k_select_dt<real><<<1, 1, 0, G->stream>>>(G->scal, vbits, (real)G->dx, (real)G->D, D.is3d() ? 1 : 0, dt_req, dt_cap);
+    k_vmax<real><<<ga, 256, 0, G->stream>>>(G->active, &G->scal->n_active, (const real*)G->f[GPK_FIELD_VN], vbits,
+                                            G->scal, (real)G->dx, (real)G->D, D.is3d() ? 1 : 0, dt_req, dt_cap);
     G->launches += 4;
     if (th.solute_rejection) {
         if (!G->solid_old) {
@@ -2021,17 +2166,11 @@ int gpk_step_graph_body(gpk_grid* G, double dt_req, double dt_cap) {
         G->have_solid_old = 1;
         G->launches++;
     }
-    uint8_t* cflag = (uint8_t*)G->ero_target;
-    k_alpha<real><<<ga, 256, 0, G->stream>>>(D, G->active, &G->scal->n_active, G->phi, G->phi_comp,
-                                             (const real*)G->f[GPK_FIELD_VN], (const real*)G->f[GPK_FIELD_T],
-                                             (real*)G->f[GPK_FIELD_ALPHA], (real*)G->alpha_new_a, cflag, G->scal,
-                                             (real)G->dx, th.stochastic, (real)th.M0, (real)th.kB, (real)th.noise_scale,
-                                             G->step_id, (real)G->near_tol, G->near_list, D.N);
-    const int nt = (D.N + MASK_TILE - 1) / MASK_TILE;
-    int32_t* ctile = G->tile_off + nt + 1;
-    k_count_u8<<<nt, MASK_TPB, 0, G->stream>>>(cflag, &G->scal->n_active, ctile);
-    k_scan_tiles<<<1, 1024, 0, G->stream>>>(ctile, nt, &G->scal->n_cand);
-    k_compact_u8_dyn<<<nt, MASK_TPB, 0, G->stream>>>(&G->scal->n_active, cflag, ctile, G->cand);
+    k_alpha<real><<<(D.N + MASK_TILE - 1) / MASK_TILE, MASK_TPB, 0, G->stream>>>(
+        D, G->active, &G->scal->n_active, G->phi, G->phi_comp, (const real*)G->f[GPK_FIELD_VN],
+        (const real*)G->f[GPK_FIELD_T], (real*)G->f[GPK_FIELD_ALPHA], (real*)G->alpha_new_a, G->cand, G->scal,
+        (ListState*)G->list_state, (real)G->dx, th.stochastic, (real)th.M0, (real)th.kB, (real)th.noise_scale,
+        G->step_id, (real)G->near_tol, G->near_list, D.N);
     // every candidate switches (no region identity); the count is read on the device
     k_accept_all<real><<<ga, 256, 0, G->stream>>>(
         G->active, G->cand, -1, G->phi, G->phi_comp, (real*)G->f[GPK_FIELD_G], (const real*)G->f[GPK_FIELD_G_COMP],
@@ -2042,18 +2181,27 @@ int gpk_step_graph_body(gpk_grid* G, double dt_req, double dt_cap) {
     // balanced remap under the accepted-crossings gate; a second 3-D pass
     // under the first pass's exchanges
     const unsigned long long* gate = &G->scal->accepted;
-    GPK_TRY(gpk_interface_mask<real>(G, gate));
+    MaskJob job;
+    job.gate = gate;
+    job.copy = G->phi_comp;
+    GPK_TRY(launch_mask(G, job));
     GPK_TRY(gpk_remap_pass_graph<real>(G, gate));
-    GPK_TRY(gpk_interface_mask<real>(G, gate));
+    job = MaskJob();
+    job.gate = gate;
     if (D.is3d()) {
-        GPK_TRY(gpk_remap_gates(G, 0));
+        job.copy = G->phi_comp;
+        job.copy_cond = &G->scal->exch_pass;
+        GPK_TRY(launch_mask(G, job));
+        GPK_TRY(gpk_remap_second_gate(G));
         GPK_TRY(gpk_remap_pass_graph<real>(G, &G->scal->gate2));
-        GPK_TRY(gpk_interface_mask<real>(G, &G->scal->gate2));
+        job = MaskJob();
+        job.gate = &G->scal->gate2;
+        job.total = 2;
+    } else {
+        job.total = 1;
     }
-    GPK_TRY(gpk_remap_gates(G, 1));
+    GPK_TRY(launch_mask(G, job));
     GPK_TRY(transport<real>(G));
-    k_advance_time<<<1, 1, 0, G->stream>>>(G->scal);
-    G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     ++G->step_id;
     return GPK_OK;
@@ -2065,7 +2213,7 @@ template int gpk_step_graph_body<double>(gpk_grid*, double, double);
 // (src/gpk_geometry.cpp:42-183), without moving any interface.
 template <typename real>
 int gpk_geometry_only(gpk_grid* G) {
-    GPK_TRY(gpk_interface_mask<real>(G));
+    GPK_TRY(launch_mask(G, geometry_job(G)));
     GPK_TRY(geometry<real>(G));
     GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
     return GPK_OK;

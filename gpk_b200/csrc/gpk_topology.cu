@@ -1555,6 +1555,8 @@ __device__ __forceinline__ bool item_less(const SortItem& a, const SortItem& b) 
     return a.v < b.v;
 }
 
+static constexpr int SORT_RANKED = 1024;  // (the block's threads)
+
 __global__ void __launch_bounds__(1024) k_sort_proposals(const unsigned* __restrict__ n_dev,
                                                          const unsigned long long* __restrict__ gate,
                                                          const int32_t* __restrict__ phi,
@@ -1569,6 +1571,31 @@ __global__ void __launch_bounds__(1024) k_sort_proposals(const unsigned* __restr
             const int32_t p = phi[i], q = phi_comp[i];
             k1a[0] = ((unsigned long long)min(p, q) << 37) | ((unsigned long long)max(p, q) << 11) |
                      ((p == min(p, q) ? 0ull : 1ull) << 10);
+        }
+        return;
+    }
+    if (n <= SORT_RANKED) {
+        // few: every proposal's rank is the number of smaller ones
+        __shared__ unsigned long long r1[SORT_RANKED], r2[SORT_RANKED];
+        __shared__ int32_t rv[SORT_RANKED];
+        const int t = threadIdx.x;
+        SortItem it{0, 0, 0};
+        if (t < n) {
+            it.v = va[t];
+            const int32_t p = phi[it.v], q = phi_comp[it.v];
+            it.k1 = ((unsigned long long)min(p, q) << 37) | ((unsigned long long)max(p, q) << 11) |
+                    ((p == min(p, q) ? 0ull : 1ull) << 10);
+            it.k2 = k2a[t];
+            r1[t] = it.k1;
+            r2[t] = it.k2;
+            rv[t] = it.v;
+        }
+        __syncthreads();
+        if (t < n) {
+            int rank = 0;
+            for (int u = 0; u < n; ++u) rank += item_less(SortItem{r1[u], r2[u], rv[u]}, it);
+            k1a[rank] = it.k1;
+            va[rank] = it.v;
         }
         return;
     }
@@ -1630,17 +1657,7 @@ __global__ void k_remap_second_gate(StepScalars* s) {
     s->gate2 = (s->accepted > 0 && s->exch_pass > 0) ? 1ull : 0ull;
     s->exch_pass = 0;
     s->waves = 0;
-}
-__global__ void k_remap_total(StepScalars* s, int is3d) {
-    s->remap_waves_sum += s->waves;  // the last pass (a skipped pass left 0 in both)
-    s->remap_props_sum += s->n_prop;
-    if (is3d) s->exchanges = s->exch_first + (s->gate2 ? s->exch_pass : 0ull);
-    else s->exchanges = s->exch_pass;
-}
-__global__ void k_copy_i32_gated(int n, const int32_t* __restrict__ src, int32_t* __restrict__ dst,
-                                 const unsigned long long* __restrict__ gate) {
-    if (gate && *gate == 0ull) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
+    s->n_prop = 0;
 }
 
 }  // namespace gpk_dev
@@ -1733,15 +1750,10 @@ int gpk_remap_pass(gpk_grid* G, const unsigned long long* gate) {
     HostKernels<real>* hk = (HostKernels<real>*)G->host_kernels;
     const int B = 256;
     const int grid = 4 * G->num_sms;
-    // phi_comp <- phi everywhere, then the best candidate at interface cells;
-    // under a device-side gate (the second 3-D pass) every kernel up to the
-    // proposals checks it, and a closed gate leaves no proposal
-    if (gate) {
-        k_copy_i32_gated<<<grid, B, 0, G->stream>>>(D.N, G->phi, G->phi_comp, gate);
-        G->launches++;
-    } else {
-        GPK_CUDA_TRY(cudaMemcpyAsync(G->phi_comp, G->phi, sizeof(int32_t) * D.N, cudaMemcpyDeviceToDevice, G->stream));
-    }
+    // phi_comp holds phi everywhere (the mask launch before); the scores write
+    // the best candidate at interface cells.  Under a device-side gate (the
+    // second 3-D pass) every kernel up to the proposals checks it, and a closed
+    // gate leaves no proposal
     const int rc = G->geometry_kernel != 1
                        ? gpk_bgr_scores_tiled<real>(G, hk->remap_radius, (real*)G->bgr_res, (real*)G->bgr_best, gate)
                        : -1;
@@ -1753,50 +1765,60 @@ int gpk_remap_pass(gpk_grid* G, const unsigned long long* gate) {
     } else if (rc != GPK_OK) {
         return rc;
     }
-    GPK_CUDA_TRY(cudaMemsetAsync(&G->scal->n_prop, 0, sizeof(unsigned), G->stream));
     k_bgr_proposals<real><<<grid, B, 0, G->stream>>>(G->active, &G->scal->n_active, G->phi, G->phi_comp,
                                                      (const real*)G->bgr_res, (const real*)G->bgr_best, G->key_b,
                                                      G->val_b, G->scal, gate);
-    G->launches += 2;
+    G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     GPK_TRY(gpk_sync_scalars(G));
     const int n = (int)G->h_scal->n_prop;
     if (n == 0) return GPK_OK;
-    // secondary order: (gain desc, cell asc); in f64 the cell order comes from
-    // the proposal generation being re-sorted by cell first
-    size_t bytes = G->cub_tmp_bytes;
-    if (sizeof(real) == 8) {
-        // sort by cell first (val as key), then stable by gain
-        GPK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(G->cub_tmp, bytes, (const int32_t*)G->val_b, (int32_t*)G->val_a,
-                                                     (const unsigned long long*)G->key_b, G->key_a, n, 0, 32,
-                                                     G->stream));
-        bytes = G->cub_tmp_bytes;
-        GPK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(G->cub_tmp, bytes, (const unsigned long long*)G->key_a, G->key_b,
-                                                     (const int32_t*)G->val_a, G->val_b, n, 0, 64, G->stream));
+    int32_t *cells, *estate;  // sorted cells, exchange states
+    if (n <= SORT_RANKED) {
+        // one launch where the radix sorts and their keys take up to six
+        k_sort_proposals<<<1, 1024, 0, G->stream>>>(&G->scal->n_prop, nullptr, G->phi, G->phi_comp, G->key_a, G->key_b,
+                                                    G->val_b, nullptr, nullptr, nullptr);
+        G->launches++;
+        cells = G->val_b;
+        estate = G->val_a;
     } else {
+        // secondary order: (gain desc, cell asc); in f64 the cell order comes from
+        // the proposal generation being re-sorted by cell first
+        size_t bytes = G->cub_tmp_bytes;
+        if (sizeof(real) == 8) {
+            // sort by cell first (val as key), then stable by gain
+            GPK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(G->cub_tmp, bytes, (const int32_t*)G->val_b, (int32_t*)G->val_a,
+                                                         (const unsigned long long*)G->key_b, G->key_a, n, 0, 32,
+                                                         G->stream));
+            bytes = G->cub_tmp_bytes;
+            GPK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(G->cub_tmp, bytes, (const unsigned long long*)G->key_a, G->key_b,
+                                                         (const int32_t*)G->val_a, G->val_b, n, 0, 64, G->stream));
+        } else {
+            GPK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(G->cub_tmp, bytes, (const unsigned long long*)G->key_b, G->key_a,
+                                                         (const int32_t*)G->val_b, G->val_a, n, 0, 64, G->stream));
+            std::swap(G->val_a, G->val_b);  // val_b holds secondary-sorted values
+        }
+        // primary order: (low, high, direction), stable
+        k_bgr_primary_keys<real><<<(n + B - 1) / B, B, 0, G->stream>>>(n, G->val_b, G->phi, G->phi_comp, G->key_b);
+        G->launches++;
+        bytes = G->cub_tmp_bytes;
+        // the keys' set bits lie in [10, 37 + bits of the largest label): sorting
+        // those bits alone gives the same order with fewer digit passes
+        int lbits = 1;
+        while (lbits < 27 && (1LL << lbits) < (long long)G->label_cap) ++lbits;
         GPK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(G->cub_tmp, bytes, (const unsigned long long*)G->key_b, G->key_a,
-                                                     (const int32_t*)G->val_b, G->val_a, n, 0, 64, G->stream));
-        std::swap(G->val_a, G->val_b);  // val_b holds secondary-sorted values
+                                                     (const int32_t*)G->val_b, G->val_a, n, 10, 37 + lbits, G->stream));
+        cells = G->val_a;
+        estate = G->val_b;
     }
-    // primary order: (low, high, direction), stable
-    k_bgr_primary_keys<real><<<(n + B - 1) / B, B, 0, G->stream>>>(n, G->val_b, G->phi, G->phi_comp, G->key_b);
-    G->launches++;
-    bytes = G->cub_tmp_bytes;
-    // the keys' set bits lie in [10, 37 + bits of the largest label): sorting
-    // those bits alone gives the same order with fewer digit passes
-    int lbits = 1;
-    while (lbits < 27 && (1LL << lbits) < (long long)G->label_cap) ++lbits;
-    GPK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(G->cub_tmp, bytes, (const unsigned long long*)G->key_b, G->key_a,
-                                                 (const int32_t*)G->val_b, G->val_a, n, 10, 37 + lbits, G->stream));
-    k_bgr_match<<<(n + B - 1) / B, B, 0, G->stream>>>(n, G->key_a, G->val_a, (int4*)G->exch, G->val_b, G->pmap,
-                                                  G->scal);
+    k_bgr_match<<<(n + B - 1) / B, B, 0, G->stream>>>(n, G->key_a, cells, (int4*)G->exch, estate, G->pmap, G->scal);
     G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     ExchArgs a;
     a.n_dev = nullptr;
     a.D = D;
     a.phi = G->phi; a.pmap = G->pmap; a.count = G->count;
-    a.exch = (const int4*)G->exch; a.estate = G->val_b;
+    a.exch = (const int4*)G->exch; a.estate = estate;
     a.g = G->f[GPK_FIELD_G]; a.alpha = G->f[GPK_FIELD_ALPHA]; a.rho = G->f[GPK_FIELD_RHO];
     a.s = G->scal;
     a.sweep_rho = G->th.dislocation_enabled; a.rho_rex_f = G->th.rho_rex; a.rho_rex_d = (double)G->th.rho_rex;
@@ -1878,7 +1900,6 @@ int gpk_remap_pass_graph(gpk_grid* G, const unsigned long long* gate) {
     HostKernels<real>* hk = (HostKernels<real>*)G->host_kernels;
     const int B = 256;
     const int grid = 4 * G->num_sms;
-    k_copy_i32_gated<<<grid, B, 0, G->stream>>>(D.N, G->phi, G->phi_comp, gate);
     const int rc = G->geometry_kernel != 1
                        ? gpk_bgr_scores_tiled<real>(G, hk->remap_radius, (real*)G->bgr_res, (real*)G->bgr_best, gate)
                        : -1;
@@ -1887,7 +1908,6 @@ int gpk_remap_pass_graph(gpk_grid* G, const unsigned long long* gate) {
         return GPK_ERR_UNSUPPORTED_MODEL;
     }
     if (rc != GPK_OK) return rc;
-    GPK_CUDA_TRY(cudaMemsetAsync(&G->scal->n_prop, 0, sizeof(unsigned), G->stream));
     k_bgr_proposals<real><<<grid, B, 0, G->stream>>>(G->active, &G->scal->n_active, G->phi, G->phi_comp,
                                                      (const real*)G->bgr_res, (const real*)G->bgr_best, G->key_b,
                                                      G->val_b, G->scal, gate);
@@ -1900,7 +1920,7 @@ int gpk_remap_pass_graph(gpk_grid* G, const unsigned long long* gate) {
     // sorted: primary keys in key_a, cells in val_b
     k_bgr_match<<<grid, B, 0, G->stream>>>(0, G->key_a, G->val_b, (int4*)G->exch, G->val_a, G->pmap,
                                            G->scal, &G->scal->n_prop);
-    G->launches += 4;
+    G->launches += 3;
     GPK_CUDA_TRY(cudaGetLastError());
     ExchArgs a;
     a.n_dev = &G->scal->n_prop;
@@ -1926,9 +1946,8 @@ template int gpk_remap_pass<double>(gpk_grid*, const unsigned long long*);
 template int gpk_remap_pass_graph<float>(gpk_grid*, const unsigned long long*);
 template int gpk_remap_pass_graph<double>(gpk_grid*, const unsigned long long*);
 
-int gpk_remap_gates(gpk_grid* G, int stage) {
-    if (stage == 0) k_remap_second_gate<<<1, 1, 0, G->stream>>>(G->scal);
-    else k_remap_total<<<1, 1, 0, G->stream>>>(G->scal, G->d.is3d() ? 1 : 0);
+int gpk_remap_second_gate(gpk_grid* G) {
+    k_remap_second_gate<<<1, 1, 0, G->stream>>>(G->scal);
     G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     return GPK_OK;
