@@ -42,6 +42,7 @@
 #include <cub/cub.cuh>
 
 #include <cmath>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -454,152 +455,228 @@ __global__ void __launch_bounds__(128) k_gauss_last_trace(Ext d, Taps t, const d
 
 // ---------------------------------------------------------------- numpy's pairwise sum
 
-// a field value, or (corr * w[i]) / wsum for the correction (added to c as it is summed)
-struct LoadF {
-    const double* a;
-    __device__ __forceinline__ double operator()(long long i) const { return a[i]; }
-};
-// the same value, also added to c[i] (the leaf pass visits every i once)
-struct CorrApplyF {
-    const double* w;
-    double* c;
-    double corr, wsum;
-    __device__ __forceinline__ double operator()(long long i) const {
-        const double v = (corr * w[i]) / wsum;
-        c[i] = c[i] + v;
-        return v;
-    }
-};
-
-// 8 lanes per leaf: lane j holds numpy's running partial r[j]
-template <class F>
-__global__ void k_pw_leaves(F f, const int* __restrict__ start, const int* __restrict__ len, int L,
-                            double* __restrict__ out) {
-    const long long gid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long leaf = gid >> 3;
-    const int lane = (int)(gid & 7);
-    const bool act = leaf < L;
-    const long long s = act ? start[leaf] : 0;
-    const int n = act ? len[leaf] : 0;
-    double r = 0.0;
-    if (act && n >= 8) {
-        r = f(s + lane);
-        const int end = n - n % 8;
-        for (int i = 8; i < end; i += 8) r = r + f(s + i + lane);
-    }
-    const unsigned full = 0xffffffffu;
-    const double t = r + __shfl_down_sync(full, r, 1);  // r0+r1, r2+r3, r4+r5, r6+r7 on even lanes
-    const double u = t + __shfl_down_sync(full, t, 2);  // (r0+r1)+(r2+r3), (r4+r5)+(r6+r7)
-    const double v = u + __shfl_down_sync(full, u, 4);  // lane 0 of the group: the 8-way total
-    if (act && lane == 0) {
-        double res;
-        if (n < 8) {
-            res = 0.0;
-            for (int i = 0; i < n; ++i) res = res + f(s + i);
-        } else {
-            res = v;
-            for (int i = n - n % 8; i < n; ++i) res = res + f(s + i);
-        }
-        out[leaf] = res;
-    }
-}
-
-// the pairwise tree of a range of n values whose subtrees of size <= t have
-// been summed into lower[k], lower[k + 1], ... (left to right)
-__device__ double pw_walk(long long n, long long t, const double* __restrict__ lower, int k) {
-    long long pend[40];
-    double part[40];
-    unsigned char state[40];
-    int sp = 0;
-    double v;
-    for (;;) {
-        while (n > t && sp < 40) {
-            long long n2 = n / 2;
-            n2 -= n2 % 8;
-            pend[sp] = n - n2;
-            state[sp] = 0;
-            ++sp;
-            n = n2;
-        }
-        v = lower[k++];
-        for (;;) {
-            if (sp == 0) return v;
-            if (state[sp - 1] == 0) {
-                part[sp - 1] = v;
-                state[sp - 1] = 1;
-                n = pend[sp - 1];
-                break;
-            }
-            v = part[sp - 1] + v;
-            --sp;
-        }
-    }
-}
-
-__global__ void k_pw_nodes(const int* __restrict__ node_n, const int* __restrict__ node_first, int M, long long t,
-                           const double* __restrict__ lower, double* __restrict__ out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < M) out[k] = pw_walk(node_n[k], t, lower, node_first[k]);
-}
-// the small upper levels (at most 1024 nodes each) in one block, a barrier
-// between levels; buffers alternate as in the per-level launches
-struct PwTop {
-    const int* n[12];
-    const int* first[12];
-    int count[12];
-    long long below[12];
-    int levels;
-};
-__global__ void __launch_bounds__(1024) k_pw_top(PwTop lv, double* b0, double* b1, int cur) {
-    for (int l = 0; l < lv.levels; ++l) {
-        const double* lower = cur ? b1 : b0;
-        double* out = cur ? b0 : b1;
-        for (int k = threadIdx.x; k < lv.count[l]; k += blockDim.x)
-            out[k] = pw_walk(lv.n[l][k], lv.below[l], lower, lv.first[l][k]);
-        __syncthreads();
-        cur ^= 1;
-    }
-}
-
-// ---------------------------------------------------------------- partition transfer
-
-__global__ void k_pt_transfer(long long N, double ct, double* __restrict__ c, const double* __restrict__ oldf,
-                              const double* __restrict__ newf, const double* __restrict__ mcomp,
-                              double* __restrict__ tr, double* __restrict__ abs_tr) {
-    GRID_STRIDE(i, N) {
-        const double delta = np_clip(newf[i], 0.0, 1.0) - oldf[i];
-        const double t = delta * (ct - mcomp[i]);
-        tr[i] = t;
-        c[i] = c[i] + t;
-        abs_tr[i] = fabs(t);
-    }
-}
-
 // order-preserving key of a double (larger value, larger key)
 __device__ __forceinline__ unsigned long long okey(double v) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
     return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
 
-__global__ void k_max_key(long long N, const double* __restrict__ w, unsigned long long* __restrict__ best) {
-    typedef cub::BlockReduce<unsigned long long, 256> BR;
-    __shared__ typename BR::TempStorage tmp;
-    unsigned long long m = 0;
-    GRID_STRIDE(i, N) {
-        const unsigned long long k = okey(w[i]);
-        m = k > m ? k : m;
+// sums of one partition transfer, on the device: the later passes read them
+enum { PT_TOTAL = 0, PT_CAP, PT_WSUM, PT_APPLIED, PT_SUMS };
+
+// the correction's two refusals, on the sums so far (the host raises them)
+__host__ __device__ inline bool pt_insufficient(const double* sum, int draw) {
+    return draw && sum[PT_CAP] < sum[PT_TOTAL] * (1.0 - 1.0e-12);
+}
+__host__ __device__ inline bool pt_empty(const double* sum) { return sum[PT_WSUM] <= 0.0; }
+
+// What a sum reads.  The leaf pass visits every i exactly once, so a loader may
+// also write what the next pass needs; begin() is false where the pass has
+// nothing to do, done() runs once per thread after its values.
+struct LoadF {
+    const double* a;
+    __device__ __forceinline__ bool begin() { return true; }
+    __device__ __forceinline__ double operator()(long long i) { return a[i]; }
+    __device__ __forceinline__ void done() {}
+};
+// the transferred Cu of a cell, added to c as it is summed
+struct TransferF {
+    double* c;
+    const double *oldf, *newf, *mcomp;
+    double* abs_tr;
+    double ct;
+    unsigned long long* best;  // [0] largest weight's key, [1] its first cell: reset here
+    __device__ __forceinline__ bool begin() {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            best[0] = 0;
+            best[1] = ~0ull;
+        }
+        return true;
     }
-    const unsigned long long agg = BR(tmp).Reduce(m, cub::Max());
-    if (threadIdx.x == 0) atomicMax(best, agg);
+    __device__ __forceinline__ double operator()(long long i) {
+        const double delta = np_clip(__ldg(newf + i), 0.0, 1.0) - __ldg(oldf + i);
+        const double t = delta * (ct - __ldg(mcomp + i));
+        c[i] = c[i] + t;
+        abs_tr[i] = fabs(t);
+        return t;
+    }
+    __device__ __forceinline__ void done() {}
+};
+// the weights, with the key of the largest
+struct WeightF {
+    const double* w;
+    unsigned long long* best;
+    unsigned long long m;
+    __device__ __forceinline__ bool begin() {
+        m = 0;
+        return true;
+    }
+    __device__ __forceinline__ double operator()(long long i) {
+        const double v = w[i];
+        const unsigned long long k = okey(v);
+        m = k > m ? k : m;
+        return v;
+    }
+    __device__ __forceinline__ void done() {
+        for (int s = 16; s; s >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(0xffffffffu, m, s);
+            m = o > m ? o : m;
+        }
+        if ((threadIdx.x & 31) == 0 && m > __ldcg(best)) atomicMax(best, m);
+    }
+};
+// (corr * w[i]) / wsum for the correction, added to c as it is summed; the
+// first cell of the largest weight on the way
+struct CorrApplyF {
+    const double* w;
+    double* c;
+    unsigned long long* best;
+    const double* sum;
+    double corr;
+    int draw;
+    double wsum;
+    unsigned long long key, first;
+    __device__ __forceinline__ bool begin() {
+        if (pt_insufficient(sum, draw) || pt_empty(sum)) return false;
+        wsum = sum[PT_WSUM];
+        key = best[0];
+        first = ~0ull;
+        return true;
+    }
+    __device__ __forceinline__ double operator()(long long i) {
+        const double wi = __ldg(w + i);
+        const double v = (corr * wi) / wsum;
+        c[i] = c[i] + v;
+        if (okey(wi) == key && (unsigned long long)i < first) first = (unsigned long long)i;
+        return v;
+    }
+    __device__ __forceinline__ void done() {
+        if (first != ~0ull) atomicMin(best + 1, first);
+    }
+};
+
+// numpy's pairwise tree in one launch.  A block sums the leaves (at most 128
+// values) of one subtree of at most 4096 values, 8 lanes per leaf (lane j holds
+// numpy's running partial r[j]), and the subtree above them in shared memory;
+// the last block to finish below a node of the next level (32 times the values)
+// evaluates that node with one warp, and so on to the root.
+//
+// A node's children sit in 64 slots: the path from the node to the child, one
+// bit per split, left-aligned in six bits (halves differ by at most 8, so
+// 32 t values are cut to t within six splits).  A split is then
+// slot[p] + slot[p + s], and slot p + s is filled exactly when it exists.
+//
+// Bound: reading the field, 32.8 MB at 160^3, 5 us.  As launches of their own
+// (the leaves, then one block walking the upper levels, each thread alone
+// through its 32 children with a stack in local memory) the four sums of a
+// transfer took 62 + 193 us, the transfer and the largest weight's search 55 us
+// more; here all of it takes 125 us.
+constexpr int PW_TPB = 256, PW_LEVELS = 8;
+
+struct PwTree {
+    const int* leaf_start;
+    const int* leaf_len;
+    const int* first[PW_LEVELS];      // first child of each node, and one past the last node's
+    const int* parent[PW_LEVELS];     // node of the next level
+    const uint8_t* slot[PW_LEVELS];   // of each child
+    double* val[PW_LEVELS];           // of each node; the top level's one value goes to *out
+    unsigned* ticket[PW_LEVELS];      // children finished (levels above the lowest), zero between sums
+    int levels;
+};
+
+// the sum over 64 slots, filled where `mask` has a bit; one warp, s in shared memory
+__device__ __forceinline__ void pw_fold(double* s, unsigned long long mask, int lane) {
+    for (int d = 1; d < 64; d <<= 1) {
+        for (int p = lane * 2 * d; p < 64; p += 64 * d)
+            if ((mask >> (p + d)) & 1ull) s[p] = s[p] + s[p + d];
+        __syncwarp();
+    }
 }
-__global__ void k_first_at(long long N, const double* __restrict__ w, const unsigned long long* __restrict__ best,
-                           unsigned long long* __restrict__ idx) {
-    const unsigned long long b = *best;
-    GRID_STRIDE(i, N) if (okey(w[i]) == b) atomicMin(idx, (unsigned long long)i);
+
+template <class F>
+__global__ void __launch_bounds__(PW_TPB) k_pw_sum(const F fn, const __grid_constant__ PwTree T, double* out) {
+    __shared__ double s[64];
+    __shared__ unsigned long long s_mask;
+    F f = fn;
+    if (!f.begin()) return;
+    const int node = blockIdx.x;
+    const int k0 = T.first[0][node], nk = T.first[0][node + 1] - k0;
+    const int lane8 = threadIdx.x & 7;
+    const unsigned full = 0xffffffffu;
+    if (threadIdx.x == 0) s_mask = 0;
+    __syncthreads();
+    for (int k = threadIdx.x >> 3; k < ((nk + 31) & ~31); k += PW_TPB / 8) {
+        const bool act = k < nk;
+        const long long b = act ? T.leaf_start[k0 + k] : 0;
+        const int n = act ? T.leaf_len[k0 + k] : 0;
+        double r = 0.0;
+        if (act && n >= 8) {
+            r = f(b + lane8);
+            const int end = n - n % 8;
+#pragma unroll 8
+            for (int i = 8; i < end; i += 8) r = r + f(b + i + lane8);
+        }
+        const double t = r + __shfl_down_sync(full, r, 1);  // r0+r1, r2+r3, r4+r5, r6+r7 on even lanes
+        const double u = t + __shfl_down_sync(full, t, 2);  // (r0+r1)+(r2+r3), (r4+r5)+(r6+r7)
+        const double v = u + __shfl_down_sync(full, u, 4);  // lane 0 of the group: the 8-way total
+        if (act && lane8 == 0) {
+            double res;
+            if (n < 8) {
+                res = 0.0;
+                for (int i = 0; i < n; ++i) res = res + f(b + i);
+            } else {
+                res = v;
+                for (int i = n - n % 8; i < n; ++i) res = res + f(b + i);
+            }
+            const int p = T.slot[0][k0 + k];
+            s[p] = res;
+            atomicOr(&s_mask, 1ull << p);
+        }
+    }
+    f.done();
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    pw_fold(s, s_mask, lane);
+    int me = node;
+    for (int l = 0;; ++l) {
+        if (l + 1 == T.levels) {
+            if (lane == 0) *out = s[0];
+            return;
+        }
+        const int up = T.parent[l][me];
+        const int c0 = T.first[l + 1][up], nc = T.first[l + 1][up + 1] - c0;
+        int last = 0;
+        if (lane == 0) {
+            __stcg(&T.val[l][me], s[0]);
+            __threadfence();
+            last = atomicAdd(&T.ticket[l + 1][up], 1u) + 1u == (unsigned)nc;
+            if (last) {
+                T.ticket[l + 1][up] = 0;
+                __threadfence();
+            }
+        }
+        if (!__shfl_sync(full, last, 0)) return;
+        unsigned long long mask = 0;
+        for (int k = lane; k < nc; k += 32) {
+            const int p = T.slot[l + 1][c0 + k];
+            s[p] = __ldcg(&T.val[l][c0 + k]);
+            mask |= 1ull << p;
+        }
+        for (int d = 16; d; d >>= 1) mask |= __shfl_xor_sync(full, mask, d);
+        __syncwarp();
+        pw_fold(s, mask, lane);
+        me = up;
+    }
 }
+
+// ---------------------------------------------------------------- partition transfer
+
 __global__ void k_pt_residue(long long N, double* __restrict__ c, const unsigned long long* __restrict__ idx,
-                             double residue) {
+                             const double* __restrict__ sum, int draw) {
+    if (pt_insufficient(sum, draw) || pt_empty(sum)) return;
     const unsigned long long i = *idx;
+    const double residue = sum[PT_TOTAL] + sum[PT_APPLIED];
     if (i < (unsigned long long)N) c[i] = c[i] - residue;
 }
 
@@ -1033,73 +1110,68 @@ __global__ void k_cgr_changed(const int* __restrict__ band, const int* __restric
 // The local certificate of topology_simple_relabel(..., local_only=True)
 // (lines 464-523) on bitmasks of the periodic 3^d patch (3^2 in 2-D):
 // position p = 9 a + 3 b + c in 3-D, 3 b + c in 2-D, centre 13 or 4.
-__device__ __forceinline__ unsigned face_nbr(int b, int nd) {
-    unsigned m = 0;
-    if (nd == 3) {
-        const int a = b / 9, r = b % 9, y = r / 3, x = r % 3;
-        if (a > 0) m |= 1u << (b - 9);
-        if (a < 2) m |= 1u << (b + 9);
-        if (y > 0) m |= 1u << (b - 3);
-        if (y < 2) m |= 1u << (b + 3);
-        if (x > 0) m |= 1u << (b - 1);
-        if (x < 2) m |= 1u << (b + 1);
-    } else {
-        const int y = b / 3, x = b % 3;
-        if (y > 0) m |= 1u << (b - 3);
-        if (y < 2) m |= 1u << (b + 3);
-        if (x > 0) m |= 1u << (b - 1);
-        if (x < 2) m |= 1u << (b + 1);
-    }
-    return m;
-}
-// face-connected components of mask that touch a face neighbour of the centre
+// Positions with c = 0 or b = 0 (shifting a row or column over the patch's edge
+// would wrap); the 2-D patch is the first plane, so one code serves both.
+constexpr unsigned PATCH_C0 = 0x1249249u, PATCH_B0 = 0x1c0e07u;
+
+// face-connected components of mask that touch a face neighbour of the centre,
+// flooded a whole frontier at a time (cell by cell, with the neighbours from
+// divisions, the two counts were most of a transaction: the sweep below took
+// 216 us for 105)
 __device__ int topo_number(unsigned mask, int nd) {
     const unsigned incident = nd == 3 ? ((1u << 4) | (1u << 10) | (1u << 12) | (1u << 14) | (1u << 16) | (1u << 22))
                                       : ((1u << 1) | (1u << 3) | (1u << 5) | (1u << 7));
     int count = 0;
     unsigned unseen = mask;
-    while (unseen) {
-        unsigned comp = unseen & (~unseen + 1u);
-        unsigned frontier = comp;
-        while (frontier) {
-            unsigned grow = 0;
-            for (unsigned f = frontier; f; f &= f - 1u) grow |= face_nbr(__ffs(f) - 1, nd);
-            grow &= unseen & ~comp;
-            comp |= grow;
-            frontier = grow;
+    for (unsigned seeds = mask & incident; seeds; seeds &= unseen) {
+        unsigned comp = seeds & (~seeds + 1u);
+        for (unsigned last = 0; comp != last;) {
+            last = comp;
+            comp |= ((comp & ~(PATCH_C0 << 2)) << 1) | ((comp & ~PATCH_C0) >> 1) | ((comp & ~(PATCH_B0 << 6)) << 3) |
+                    ((comp & ~PATCH_B0) >> 3) | (comp << 9) | (comp >> 9);
+            comp &= unseen;
         }
         unseen &= ~comp;
-        if (comp & incident) ++count;
+        ++count;
     }
     return count;
 }
-// positions of the periodic patch around cell i holding label a / b (centre excluded)
-__device__ void patch_masks(const Ext& d, const int8_t* lab, long long i, int a, int b, unsigned& ma, unsigned& mb) {
-    int x0, x1, x2;
-    cell_coords(d, i, x0, x1, x2);
+// positions of the periodic patch around cell i holding label a / b (centre
+// excluded); L2: other blocks of the launch write labels
+template <bool L2>
+__device__ void patch_masks(const Ext& d, const int8_t* lab, int x0, int x1, int x2, int a, int b, unsigned& ma,
+                            unsigned& mb) {
     const int y1[3] = {x1 == 0 ? d.e[1] - 1 : x1 - 1, x1, x1 + 1 == d.e[1] ? 0 : x1 + 1};
     const int y2[3] = {x2 == 0 ? d.e[2] - 1 : x2 - 1, x2, x2 + 1 == d.e[2] ? 0 : x2 + 1};
     const int y0[3] = {x0 == 0 ? d.e[0] - 1 : x0 - 1, x0, x0 + 1 == d.e[0] ? 0 : x0 + 1};
     ma = mb = 0;
-    const int n0 = d.ndim == 3 ? 3 : 1;
-    for (int p0 = 0; p0 < n0; ++p0)
+#pragma unroll
+    for (int p0 = 0; p0 < 3; ++p0) {
+        if (p0 > 0 && d.ndim != 3) break;
+        const long long z0 = d.ndim == 3 ? y0[p0] : 0;
+#pragma unroll
         for (int p1 = 0; p1 < 3; ++p1)
+#pragma unroll
             for (int p2 = 0; p2 < 3; ++p2) {
-                const int bit = d.ndim == 3 ? 9 * p0 + 3 * p1 + p2 : 3 * p1 + p2;
-                if (bit == (d.ndim == 3 ? 13 : 4)) continue;
-                const int z0 = d.ndim == 3 ? y0[p0] : 0;
-                const int v = lab[((long long)z0 * d.e[1] + y1[p1]) * d.e[2] + y2[p2]];
-                if (v == a) ma |= 1u << bit;
-                if (v == b) mb |= 1u << bit;
+                const int bit = 9 * p0 + 3 * p1 + p2;
+                const int8_t* at = lab + (z0 * d.e[1] + y1[p1]) * d.e[2] + y2[p2];
+                const int v = L2 ? __ldcg(at) : *at;
+                ma |= (unsigned)(v == a) << bit;
+                mb |= (unsigned)(v == b) << bit;
             }
+    }
+    const unsigned centre = d.ndim == 3 ? 1u << 13 : 1u << 4;
+    ma &= ~centre;
+    mb &= ~centre;
 }
 // counts: label value + 128 -> cells holding it; null when no label can
 // fall to one cell (extinction never applies)
-__device__ bool cert_local(const Ext& d, const int8_t* lab, long long i, int old_label, int new_label,
-                           const int* counts) {
+template <bool L2>
+__device__ bool cert_at(const Ext& d, const int8_t* lab, int x0, int x1, int x2, int old_label, int new_label,
+                        const int* counts) {
     if (old_label == new_label) return false;
     unsigned mo, mn;
-    patch_masks(d, lab, i, old_label, new_label, mo, mn);
+    patch_masks<L2>(d, lab, x0, x1, x2, old_label, new_label, mo, mn);
     const int oc = topo_number(mo, d.ndim);
     const bool extinction = counts ? counts[old_label + 128] <= 1 : false;
     if (oc == 0 && !extinction) return false;
@@ -1107,6 +1179,13 @@ __device__ bool cert_local(const Ext& d, const int8_t* lab, long long i, int old
     const int nc = topo_number(mn, d.ndim);
     if (nc == 0 || nc > 1) return false;
     return true;
+}
+
+__device__ bool cert_local(const Ext& d, const int8_t* lab, long long i, int old_label, int new_label,
+                           const int* counts) {
+    int x0, x1, x2;
+    cell_coords(d, i, x0, x1, x2);
+    return cert_at<false>(d, lab, x0, x1, x2, old_label, new_label, counts);
 }
 
 __global__ void k_label_hist(long long N, const int8_t* __restrict__ lab, int* __restrict__ counts) {
@@ -1123,92 +1202,126 @@ __global__ void k_u8_flags(long long N, const uint8_t* __restrict__ m, int* __re
 }
 
 // commit_topology_transactions (lines 526-559): the crossing cells in C
-// order, each certificate against the state the earlier ones left
-__global__ void k_tx_commit(Ext d, const int* __restrict__ list, const int* __restrict__ n_list, int8_t* lab,
-                            double* alpha, const int8_t* __restrict__ comp, int* counts,
-                            unsigned long long* __restrict__ deferred) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    const int M = *n_list;
-    unsigned long long nd = 0;
-    for (int q = 0; q < M; ++q) {
-        const long long i = list[q];
-        const int old_label = lab[i], new_label = comp[i];
-        if (cert_local(d, lab, i, old_label, new_label, counts)) {
-            lab[i] = (int8_t)new_label;
-            alpha[i] = 1.0;
-            counts[old_label + 128] -= 1;
-            counts[new_label + 128] += 1;
-        } else {
-            ++nd;
-            const double a = alpha[i];
-            alpha[i] = 1.0e-6 > a ? 1.0e-6 : a;  // Python max(a, 1e-6)
-        }
-    }
-    *deferred = nd;
-}
+// order, each certificate against the state the earlier ones left.
+//
+// A transaction reads only its periodic 3^d patch, so it may run as soon as
+// every earlier (lower cell index) crossing cell in that patch has run; its
+// later neighbours wait for it, so each sees exactly the state of the serial
+// order.  That holds where the extinction test cannot fire, i.e. where no
+// label can fall to one cell in the sweep; else one thread keeps the order.
+//
+// One cooperative launch: a thread takes its cells in ascending order and polls
+// the earlier neighbours it still waits for.  The lowest pending cell of all is
+// at the head of its thread's cells and waits for none, so some thread always
+// goes on; polls are bounded all the same and set *err.  Bound: the longest
+// chain of neighbours, one L2 round trip for the poll, one for the patch and
+// one for the write per link.  As rounds of 8 launches with a count read back
+// after each 8, the 160^3 field's 24 rounds took 216 us and three waits of the
+// host; so, 105 us.
+constexpr int TX_PENDING = 0x7fffffff, TX_DONE = 0;
+constexpr int TX_POLLS = 1 << 22;
+constexpr int TX_TPB = 128;
 
-// The same commits in rounds.  A transaction reads only its periodic 3^d
-// patch, so it may run once every earlier (lower cell index) crossing cell in
-// that patch has run in an earlier round; transactions ready in one round
-// are never neighbours of one another, and their later neighbours have not
-// run yet, so each sees exactly the state of the serial order.  Used when no
-// label can fall to one cell during the sweep (then the extinction test is
-// false throughout); done[i] = round of the commit, INT_MAX while pending.
-constexpr int TX_PENDING = 0x7fffffff;
-
-__global__ void k_tx_init(const int* __restrict__ list, const int* __restrict__ n_list, int* __restrict__ done,
+__global__ void k_tx_init(const int* __restrict__ list, const int* __restrict__ n_list, int* __restrict__ state,
                           int* __restrict__ crossing_hist, const int8_t* __restrict__ lab) {
     const int M = *n_list;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < M; q += gridDim.x * blockDim.x) {
-        done[list[q]] = TX_PENDING;
+        state[list[q]] = TX_PENDING;
         atomicAdd(&crossing_hist[(int)lab[list[q]] + 128], 1);
     }
 }
-__global__ void k_tx_round(Ext d, int round, const int* __restrict__ list, const int* __restrict__ n_list,
-                           const uint8_t* __restrict__ crossing, int* done, int8_t* lab, double* alpha,
-                           const int8_t* __restrict__ comp, unsigned long long* __restrict__ counters) {
+
+// index of position p (9 a + 3 b + c; 3 b + c in 2-D) of the periodic patch around (x0, x1, x2)
+__device__ __forceinline__ int patch_cell(const Ext& d, int x0, int x1, int x2, int p) {
+    int z = d.ndim == 3 ? x0 + p / 9 - 1 : 0, y = x1 + (p % 9) / 3 - 1, x = x2 + p % 3 - 1;
+    z = z < 0 ? d.e[0] - 1 : (z == d.e[0] ? 0 : z);
+    y = y < 0 ? d.e[1] - 1 : (y == d.e[1] ? 0 : y);
+    x = x < 0 ? d.e[2] - 1 : (x == d.e[2] ? 0 : x);
+    return (int)(((long long)z * d.e[1] + y) * d.e[2] + x);
+}
+
+__global__ void __launch_bounds__(TX_TPB) k_tx_commit(Ext d, const int* __restrict__ list,
+                                                      const int* __restrict__ n_list,
+                                                      const uint8_t* __restrict__ crossing, int* state, int8_t* lab,
+                                                      double* alpha, const int8_t* __restrict__ comp,
+                                                      const int* __restrict__ counts,
+                                                      const int* __restrict__ crossing_hist,
+                                                      unsigned long long* __restrict__ deferred, unsigned* err) {
     const int M = *n_list;
-    // rounds launched after the last transaction ran return at once
-    __shared__ int finished;
-    if (threadIdx.x == 0) finished = __ldcg(&counters[0]) >= (unsigned long long)M;
-    __syncthreads();
-    if (finished) return;
-    unsigned long long ran = 0, nd = 0;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < M; q += gridDim.x * blockDim.x) {
-        const int j = list[q];
-        if (__ldcg(&done[j]) != TX_PENDING) continue;
-        int x0, x1, x2;
-        cell_coords(d, j, x0, x1, x2);
-        const int y1[3] = {x1 == 0 ? d.e[1] - 1 : x1 - 1, x1, x1 + 1 == d.e[1] ? 0 : x1 + 1};
-        const int y2[3] = {x2 == 0 ? d.e[2] - 1 : x2 - 1, x2, x2 + 1 == d.e[2] ? 0 : x2 + 1};
-        const int y0[3] = {x0 == 0 ? d.e[0] - 1 : x0 - 1, x0, x0 + 1 == d.e[0] ? 0 : x0 + 1};
-        bool ready = true;
-        const int n0 = d.ndim == 3 ? 3 : 1;
-        for (int p0 = 0; p0 < n0 && ready; ++p0)
-            for (int p1 = 0; p1 < 3 && ready; ++p1)
-                for (int p2 = 0; p2 < 3; ++p2) {
-                    const int z0 = d.ndim == 3 ? y0[p0] : 0;
-                    const int nb = (int)(((long long)z0 * d.e[1] + y1[p1]) * d.e[2] + y2[p2]);
-                    if (nb < j && crossing[nb] && __ldcg(&done[nb]) >= round) {
-                        ready = false;
-                        break;
-                    }
-                }
-        if (!ready) continue;
-        const int old_label = lab[j], new_label = comp[j];
-        if (cert_local(d, lab, j, old_label, new_label, nullptr)) {
+    if (M == 0) return;
+    __shared__ int s_counts[256];
+    bool falls = false;
+    for (int k = threadIdx.x; k < 256; k += TX_TPB) {
+        s_counts[k] = counts[k];
+        if (crossing_hist[k] && s_counts[k] - crossing_hist[k] < 2) falls = true;
+    }
+    if (__syncthreads_or(falls)) {
+        if (blockIdx.x != 0 || threadIdx.x != 0) return;
+        unsigned long long nd = 0;
+        for (int q = 0; q < M; ++q) {
+            const long long i = list[q];
+            const int old_label = lab[i], new_label = comp[i];
+            if (cert_local(d, lab, i, old_label, new_label, s_counts)) {
+                lab[i] = (int8_t)new_label;
+                alpha[i] = 1.0;
+                s_counts[old_label + 128] -= 1;
+                s_counts[new_label + 128] += 1;
+            } else {
+                ++nd;
+                const double a = alpha[i];
+                alpha[i] = 1.0e-6 > a ? 1.0e-6 : a;  // Python max(a, 1e-6)
+            }
+        }
+        *deferred = nd;
+        return;
+    }
+    const int np = d.ndim == 3 ? 27 : 9;
+    unsigned long long nd = 0;
+    int q = blockIdx.x * TX_TPB + threadIdx.x;
+    int j = 0, x0 = 0, x1 = 0, x2 = 0, old_label = 0, new_label = 0;
+    double a = 0.0;
+    unsigned wait = 0;
+    bool fresh = true;
+    for (int polls = 0; q < M;) {
+        if (fresh) {
+            j = list[q];
+            cell_coords(d, j, x0, x1, x2);
+            old_label = lab[j];  // nobody else writes the cell's own values
+            new_label = comp[j];
+            a = alpha[j];
+            wait = 0;
+            for (int p = 0; p < np; ++p) {
+                const int nb = patch_cell(d, x0, x1, x2, p);
+                if (nb < j && crossing[nb]) wait |= 1u << p;
+            }
+            fresh = false;
+        }
+        for (unsigned m = wait; m; m &= m - 1u) {
+            const int p = __ffs(m) - 1;
+            if (__ldcg(&state[patch_cell(d, x0, x1, x2, p)]) == TX_DONE) wait &= ~(1u << p);
+        }
+        if (wait) {
+            if (++polls > TX_POLLS) {
+                atomicOr(err, 1u);
+                break;
+            }
+            continue;
+        }
+        __threadfence();  // the labels below are read after the states above
+        if (cert_at<true>(d, lab, x0, x1, x2, old_label, new_label, nullptr)) {
             lab[j] = (int8_t)new_label;
             alpha[j] = 1.0;
+            __threadfence();
         } else {
             ++nd;
-            const double a = alpha[j];
-            alpha[j] = 1.0e-6 > a ? 1.0e-6 : a;  // Python max(a, 1e-6)
+            alpha[j] = 1.0e-6 > a ? 1.0e-6 : a;
         }
-        done[j] = round;
-        ++ran;
+        __stcg(&state[j], TX_DONE);
+        polls = 0;
+        q += gridDim.x * TX_TPB;
+        fresh = true;
     }
-    if (ran) atomicAdd(&counters[0], ran);
-    if (nd) atomicAdd(&counters[1], nd);
+    if (nd) atomicAdd(deferred, nd);
 }
 
 // the labels present, ascending (np.unique), at most 8
@@ -1433,19 +1546,17 @@ struct gpk_alcu {
     Phys p{};
     int device = 0;
     int num_sms = 148;
+    int tx_grid = 0;  // resident blocks of the transaction sweep
     int grid = 0;
     cudaStream_t own = nullptr, stream = nullptr;
     long long bytes = 0;
     // transport scratch
     double* f[6] = {};  // six N-double fields
-    // pairwise-sum tree: leaves, then upper levels up to the root
-    int* leaf_start = nullptr;
-    int* leaf_len = nullptr;
-    int n_leaves = 0;
-    std::vector<int*> lvl_n, lvl_first;
-    std::vector<int> lvl_count;
-    std::vector<long long> lvl_below;  // threshold of the level under each
-    double* pw_buf[2] = {};
+    // pairwise-sum tree, and the sums of a partition transfer
+    PwTree tree{};
+    int n_groups = 0;  // nodes of its lowest level
+    void* tree_mem = nullptr;
+    double* sums = nullptr;
     // reductions
     unsigned long long* u64 = nullptr;  // [0] max key, [1] index, [2] changed count
     int* i32 = nullptr;                 // [0] candidates, [1] conflicts, [2] changed flag, [3] max wave, [4] active
@@ -1502,12 +1613,22 @@ void cut(long long lo, long long n, long long t, std::vector<long long>& s, std:
     cut(lo + n2, n - n2, t, s, len);
 }
 
+// slots of the children (subtrees of at most t values) of a node of n values,
+// appended at out[k..]; false when the path needs more than six splits
+bool slots(long long n, long long t, int p, int half, uint8_t* out, int& k) {
+    if (n <= t) {
+        out[k++] = (uint8_t)p;
+        return true;
+    }
+    if (half == 0) return false;
+    long long n2 = n / 2;
+    n2 -= n2 % 8;
+    return slots(n2, t, p, half / 2, out, k) && slots(n - n2, t, p + half, half / 2, out, k);
+}
+
 void free_all(gpk_alcu* h) {
     for (double*& q : h->f) cudaFree(q);
-    cudaFree(h->leaf_start); cudaFree(h->leaf_len);
-    for (int* q : h->lvl_n) cudaFree(q);
-    for (int* q : h->lvl_first) cudaFree(q);
-    cudaFree(h->pw_buf[0]); cudaFree(h->pw_buf[1]);
+    cudaFree(h->tree_mem); cudaFree(h->sums);
     cudaFree(h->u64); cudaFree(h->i32); cudaFree(h->err);
     cudaFree(h->orig); cudaFree(h->parent); cudaFree(h->root); cudaFree(h->size); cudaFree(h->wave);
     cudaFree(h->seg); cudaFree(h->start); cudaFree(h->flag); cudaFree(h->pos); cudaFree(h->cand);
@@ -1533,41 +1654,11 @@ int taps_of(const double* taps, int radius, Taps& t) {
     return GPK_OK;
 }
 
-// np.sum of the values f(0..N-1); waits for the stream
+// np.sum of the values f(0..N-1) into *out on the device
 template <class F>
-int pw_sum(gpk_alcu* h, F f, double* out) {
-    cudaStream_t st = h->stream;
-    const long long threads = 8ll * h->n_leaves;
-    k_pw_leaves<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(f, h->leaf_start, h->leaf_len, h->n_leaves,
-                                                                     h->pw_buf[0]);
+int pw_launch(gpk_alcu* h, F f, double* out) {
+    k_pw_sum<F><<<h->n_groups, PW_TPB, 0, h->stream>>>(f, h->tree, out);
     ALCU_TRY(cudaGetLastError());
-    int cur = 0;
-    size_t k = 0;
-    for (; k < h->lvl_n.size() && h->lvl_count[k] > 1024; ++k) {
-        const int M = h->lvl_count[k];
-        k_pw_nodes<<<(M + 127) / 128, 128, 0, st>>>(h->lvl_n[k], h->lvl_first[k], M, h->lvl_below[k],
-                                                     h->pw_buf[cur], h->pw_buf[cur ^ 1]);
-        ALCU_TRY(cudaGetLastError());
-        cur ^= 1;
-    }
-    if (k < h->lvl_n.size()) {
-        PwTop lv{};
-        for (; k < h->lvl_n.size() && lv.levels < 12; ++k, ++lv.levels) {
-            lv.n[lv.levels] = h->lvl_n[k];
-            lv.first[lv.levels] = h->lvl_first[k];
-            lv.count[lv.levels] = h->lvl_count[k];
-            lv.below[lv.levels] = h->lvl_below[k];
-        }
-        if (k < h->lvl_n.size()) {
-            gpk_set_error("alcu: summation tree deeper than expected");
-            return GPK_ERR_INTERNAL;
-        }
-        k_pw_top<<<1, 1024, 0, st>>>(lv, h->pw_buf[0], h->pw_buf[1], cur);
-        ALCU_TRY(cudaGetLastError());
-        cur ^= lv.levels & 1;
-    }
-    ALCU_TRY(cudaMemcpyAsync(out, h->pw_buf[cur], sizeof(double), cudaMemcpyDeviceToHost, st));
-    ALCU_TRY(cudaStreamSynchronize(st));
     return GPK_OK;
 }
 
@@ -1743,57 +1834,77 @@ extern "C" int gpk_alcu_create(int ndim, const int* shape, const gpk_alcu_params
     };
     for (double*& q : h->f)
         if (!alloc((void**)&q, sizeof(double) * N)) return fail(GPK_ERR_OUT_OF_MEMORY);
-    // pairwise-sum tree
+    // pairwise-sum tree: the levels' nodes, then one allocation for all of it
     {
         std::vector<long long> s, len;
         cut(0, N, 128, s, len);
-        h->n_leaves = (int)s.size();
-        std::vector<int> s32(s.begin(), s.end()), l32(len.begin(), len.end());
-        if (!alloc((void**)&h->leaf_start, sizeof(int) * s32.size()) ||
-            !alloc((void**)&h->leaf_len, sizeof(int) * l32.size()))
-            return fail(GPK_ERR_OUT_OF_MEMORY);
-        if (cudaMemcpy(h->leaf_start, s32.data(), sizeof(int) * s32.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(h->leaf_len, l32.data(), sizeof(int) * l32.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        std::vector<int> leaf_start(s.begin(), s.end()), leaf_len(len.begin(), len.end());
+        std::vector<std::vector<int>> first, parent;
+        std::vector<std::vector<uint8_t>> slot;
+        std::vector<long long> below = s;
+        for (long long t = 128 * 32;; t *= 32) {
+            std::vector<long long> ns, nl;
+            cut(0, N, t < N ? t : N, ns, nl);
+            first.emplace_back();
+            slot.emplace_back(below.size());
+            std::vector<int> up(below.size());
+            size_t k = 0;
+            for (size_t q = 0; q < ns.size(); ++q) {
+                first.back().push_back((int)k);
+                int p = 0;
+                if (!slots(nl[q], t / 32, 0, 32, slot.back().data() + k, p)) {
+                    gpk_set_error("alcu: summation tree deeper than expected");
+                    return fail(GPK_ERR_INTERNAL);
+                }
+                for (int c = 0; c < p; ++c) up[k + c] = (int)q;
+                k += p;
+            }
+            first.back().push_back((int)k);
+            if (!parent.empty() || first.size() > 1) parent.push_back(up);
+            below = ns;
+            if (ns.size() == 1) break;
+        }
+        PwTree& T = h->tree;
+        T.levels = (int)first.size();
+        if (T.levels > PW_LEVELS) {
+            gpk_set_error("alcu: summation tree deeper than expected");
+            return fail(GPK_ERR_INTERNAL);
+        }
+        h->n_groups = (int)first[0].size() - 1;
+        size_t bytes = 0;
+        auto place = [&](size_t b) { const size_t at = bytes; bytes += (b + 15) & ~(size_t)15; return at; };
+        const size_t o_start = place(4 * leaf_start.size()), o_len = place(4 * leaf_len.size());
+        size_t o_first[PW_LEVELS], o_parent[PW_LEVELS], o_slot[PW_LEVELS], o_val[PW_LEVELS], o_ticket[PW_LEVELS];
+        for (int l = 0; l < T.levels; ++l) {
+            const size_t n = first[l].size() - 1;
+            o_first[l] = place(4 * (n + 1));
+            o_slot[l] = place(slot[l].size());
+            o_parent[l] = place(4 * n);
+            o_val[l] = place(8 * n);
+            o_ticket[l] = place(4 * n);
+        }
+        if (!alloc(&h->tree_mem, bytes)) return fail(GPK_ERR_OUT_OF_MEMORY);
+        std::vector<char> host(bytes, 0);
+        char* dev = (char*)h->tree_mem;
+        std::memcpy(host.data() + o_start, leaf_start.data(), 4 * leaf_start.size());
+        std::memcpy(host.data() + o_len, leaf_len.data(), 4 * leaf_len.size());
+        T.leaf_start = (const int*)(dev + o_start);
+        T.leaf_len = (const int*)(dev + o_len);
+        for (int l = 0; l < T.levels; ++l) {
+            std::memcpy(host.data() + o_first[l], first[l].data(), 4 * first[l].size());
+            std::memcpy(host.data() + o_slot[l], slot[l].data(), slot[l].size());
+            if (l + 1 < T.levels) std::memcpy(host.data() + o_parent[l], parent[l].data(), 4 * parent[l].size());
+            T.first[l] = (const int*)(dev + o_first[l]);
+            T.slot[l] = (const uint8_t*)(dev + o_slot[l]);
+            T.parent[l] = (const int*)(dev + o_parent[l]);
+            T.val[l] = (double*)(dev + o_val[l]);
+            T.ticket[l] = (unsigned*)(dev + o_ticket[l]);
+        }
+        if (cudaMemcpy(h->tree_mem, host.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
             gpk_set_error("alcu: upload of the summation tree failed");
             return fail(GPK_ERR_CUDA);
         }
-        std::vector<long long> below_s = s;
-        long long t_below = 128;
-        while (below_s.size() > 1) {
-            const long long t = t_below * 32;
-            std::vector<long long> ns, nl;
-            if (t >= N) {
-                ns.push_back(0);
-                nl.push_back(N);
-            } else {
-                cut(0, N, t, ns, nl);
-            }
-            // first lower-level node of each node: walk both ordered lists
-            std::vector<int> first(ns.size()), n32(ns.size());
-            size_t k = 0;
-            for (size_t q = 0; q < ns.size(); ++q) {
-                while (k < below_s.size() && below_s[k] < ns[q]) ++k;
-                first[q] = (int)k;
-                n32[q] = (int)nl[q];
-            }
-            int *dn = nullptr, *df = nullptr;
-            if (!alloc((void**)&dn, sizeof(int) * ns.size()) || !alloc((void**)&df, sizeof(int) * ns.size()))
-                return fail(GPK_ERR_OUT_OF_MEMORY);
-            h->lvl_n.push_back(dn);
-            h->lvl_first.push_back(df);
-            if (cudaMemcpy(dn, n32.data(), sizeof(int) * ns.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-                cudaMemcpy(df, first.data(), sizeof(int) * ns.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-                gpk_set_error("alcu: upload of the summation tree failed");
-                return fail(GPK_ERR_CUDA);
-            }
-            h->lvl_count.push_back((int)ns.size());
-            h->lvl_below.push_back(t_below);
-            below_s = ns;
-            t_below = t;
-        }
-        if (!alloc((void**)&h->pw_buf[0], sizeof(double) * h->n_leaves) ||
-            !alloc((void**)&h->pw_buf[1], sizeof(double) * h->n_leaves))
-            return fail(GPK_ERR_OUT_OF_MEMORY);
+        if (!alloc((void**)&h->sums, sizeof(double) * PT_SUMS)) return fail(GPK_ERR_OUT_OF_MEMORY);
     }
     if (!alloc((void**)&h->u64, sizeof(unsigned long long) * 4) || !alloc((void**)&h->i32, sizeof(int) * 8) ||
         !alloc((void**)&h->err, sizeof(unsigned) * 2))
@@ -1915,7 +2026,12 @@ extern "C" int gpk_alcu_diffuse(gpk_alcu* h, double* ctot, const double* fprec, 
 
 extern "C" int gpk_alcu_sum(gpk_alcu* h, const double* x, double* out) {
     if (!h || !x || !out) { gpk_set_error("alcu: null argument"); return GPK_ERR_INVALID_ARGUMENT; }
-    return pw_sum(h, LoadF{x}, out);
+    const int rc = pw_launch(h, LoadF{x}, h->sums);
+    if (rc != GPK_OK) return rc;
+    ALCU_TRY(cudaMemcpyAsync(out, h->sums, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    ALCU_TRY(cudaStreamSynchronize(h->stream));
+    *out = 0.0 + *out;  // np.sum starts at +0: a sum of -0 alone is +0
+    return GPK_OK;
 }
 
 extern "C" int gpk_alcu_gaussian_filter(gpk_alcu* h, const double* in, double* out, const double* taps, int radius) {
@@ -1940,12 +2056,14 @@ extern "C" int gpk_alcu_partition_transfer(gpk_alcu* h, double* ctot, const doub
     int rc = taps_of(taps, radius, t);
     if (rc != GPK_OK) return rc;
     const long long N = h->d.N;
-    double *tr = h->f[0], *absd = h->f[1], *g = h->f[2], *w = h->f[3], *cap = h->f[4], *tmp = h->f[5];
-    k_pt_transfer<<<h->grid, 256, 0, h->stream>>>(N, h->p.ct, ctot, old_fraction, new_fraction, matrix_composition, tr,
-                                                  absd);
-    ALCU_TRY(cudaGetLastError());
+    double *absd = h->f[1], *g = h->f[2], *w = h->f[3], *cap = h->f[4], *tmp = h->f[5];
+    double* sums = h->sums;
+    rc = pw_launch(h, TransferF{ctot, old_fraction, new_fraction, matrix_composition, absd, h->p.ct, h->u64},
+                   sums + PT_TOTAL);
+    if (rc != GPK_OK) return rc;
     double total = 0.0;
-    if ((rc = pw_sum(h, LoadF{tr}, &total)) != GPK_OK) return rc;
+    ALCU_TRY(cudaMemcpyAsync(&total, sums + PT_TOTAL, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    ALCU_TRY(cudaStreamSynchronize(h->stream));
     if (std::fabs(total) <= 1.0e-30) return GPK_OK;
     const double correction = -total;
     const int draw = correction < 0.0;
@@ -1963,30 +2081,25 @@ extern "C" int gpk_alcu_partition_transfer(gpk_alcu* h, double* ctot, const doub
                                                               draw);
         ALCU_TRY(cudaGetLastError());
     }
-    if (draw) {
-        double cap_sum = 0.0;
-        if ((rc = pw_sum(h, LoadF{cap}, &cap_sum)) != GPK_OK) return rc;
-        if (cap_sum < -correction * (1.0 - 1.0e-12)) {
-            gpk_set_error("insufficient matrix Cu for partition transfer");
-            return GPK_ERR_INFEASIBLE;
-        }
+    // ctot += (correction w) / wsum, summed as it is added; on the device the
+    // two refusals below leave ctot as it is, and the host reads the sums once
+    if (draw && (rc = pw_launch(h, LoadF{cap}, sums + PT_CAP)) != GPK_OK) return rc;
+    if ((rc = pw_launch(h, WeightF{w, h->u64, 0}, sums + PT_WSUM)) != GPK_OK) return rc;
+    rc = pw_launch(h, CorrApplyF{w, ctot, h->u64, sums, correction, draw, 0.0, 0, 0}, sums + PT_APPLIED);
+    if (rc != GPK_OK) return rc;
+    k_pt_residue<<<1, 1, 0, h->stream>>>(N, ctot, h->u64 + 1, sums, draw);
+    ALCU_TRY(cudaGetLastError());
+    double got[PT_SUMS];
+    ALCU_TRY(cudaMemcpyAsync(got, sums, sizeof(got), cudaMemcpyDeviceToHost, h->stream));
+    ALCU_TRY(cudaStreamSynchronize(h->stream));
+    if (pt_insufficient(got, draw)) {
+        gpk_set_error("insufficient matrix Cu for partition transfer");
+        return GPK_ERR_INFEASIBLE;
     }
-    double wsum = 0.0;
-    if ((rc = pw_sum(h, LoadF{w}, &wsum)) != GPK_OK) return rc;
-    if (wsum <= 0.0) {
+    if (pt_empty(got)) {
         gpk_set_error("empty matrix neighbourhood for partition transfer");
         return GPK_ERR_INFEASIBLE;
     }
-    // ctot += (correction w) / wsum, summed as it is added
-    double s = 0.0;
-    if ((rc = pw_sum(h, CorrApplyF{w, ctot, correction, wsum}, &s)) != GPK_OK) return rc;
-    const double residue = total + s;
-    ALCU_TRY(cudaMemsetAsync(h->u64, 0, sizeof(unsigned long long), h->stream));
-    ALCU_TRY(cudaMemsetAsync(h->u64 + 1, 0xff, sizeof(unsigned long long), h->stream));
-    k_max_key<<<h->grid, 256, 0, h->stream>>>(N, w, h->u64);
-    k_first_at<<<h->grid, 256, 0, h->stream>>>(N, w, h->u64, h->u64 + 1);
-    k_pt_residue<<<1, 1, 0, h->stream>>>(N, ctot, h->u64 + 1, residue);
-    ALCU_TRY(cudaGetLastError());
     return GPK_OK;
 }
 
@@ -2242,44 +2355,31 @@ extern "C" int gpk_alcu_commit_transactions(gpk_alcu* h, int8_t* labels, double*
     k_compact<<<G, 256, 0, st>>>(N, h->flag, h->pos, nullptr, h->cand, n_list);
     k_tx_init<<<G, 256, 0, st>>>(h->cand, n_list, h->wave, xhist, labels);
     ALCU_TRY(cudaGetLastError());
-    int M = 0;
-    int hc[256], hx[256];
-    ALCU_TRY(cudaMemcpyAsync(&M, n_list, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ALCU_TRY(cudaMemcpyAsync(hc, h->cnt256, sizeof(hc), cudaMemcpyDeviceToHost, st));
-    ALCU_TRY(cudaMemcpyAsync(hx, xhist, sizeof(hx), cudaMemcpyDeviceToHost, st));
-    ALCU_TRY(cudaStreamSynchronize(st));
-    if (deferred) *deferred = 0;
-    if (M == 0) return GPK_OK;
-    // the extinction test can only fire for a label that the sweep may
-    // reduce to one cell; then the serial order runs on one thread
-    bool extinction_possible = false;
-    for (int k = 0; k < 256; ++k)
-        if (hx[k] && hc[k] - hx[k] < 2) extinction_possible = true;
-    unsigned long long nd = 0;
-    if (extinction_possible) {
-        k_tx_commit<<<1, 32, 0, st>>>(d, h->cand, n_list, labels, alpha, competitor, h->cnt256, h->u64 + 1);
-        ALCU_TRY(cudaGetLastError());
-        ALCU_TRY(cudaMemcpyAsync(&nd, h->u64 + 1, sizeof(nd), cudaMemcpyDeviceToHost, st));
-        ALCU_TRY(cudaStreamSynchronize(st));
-    } else {
-        const int gb = (M + 255) / 256 < G ? (M + 255) / 256 : G;
-        unsigned long long hcnt[2] = {0, 0};
-        // the earliest pending transaction is always ready: at most M rounds
-        for (int round = 0; hcnt[0] < (unsigned long long)M;) {
-            if (round > M) {
-                gpk_set_error("alcu: transaction rounds did not finish");
-                return GPK_ERR_INTERNAL;
-            }
-            for (int k = 0; k < 8; ++k, ++round)
-                k_tx_round<<<gb, 256, 0, st>>>(d, round, h->cand, n_list, crossing, h->wave, labels, alpha,
-                                                competitor, h->u64);
-            ALCU_TRY(cudaGetLastError());
-            ALCU_TRY(cudaMemcpyAsync(hcnt, h->u64, sizeof(hcnt), cudaMemcpyDeviceToHost, st));
-            ALCU_TRY(cudaStreamSynchronize(st));
-        }
-        nd = hcnt[1];
+    // every block is resident: the grid is what fits, or a thread per cell
+    if (h->tx_grid == 0) {
+        int per_sm = 0;
+        ALCU_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tx_commit, TX_TPB, 0));
+        h->tx_grid = per_sm * h->num_sms;
     }
-    if (deferred) *deferred = (int64_t)nd;
+    const long long want = (N + TX_TPB - 1) / TX_TPB;
+    const int grid = want < h->tx_grid ? (int)want : h->tx_grid;
+    const int* list = h->cand;
+    const int* count = n_list;
+    const int* hist = xhist;
+    unsigned long long* n_def = h->u64 + 1;
+    unsigned* stuck = (unsigned*)(h->u64 + 2);
+    Ext dd = d;
+    void* args[] = {&dd,    &list,       &count,     &crossing, &h->wave, &labels,
+                    &alpha, &competitor, &h->cnt256, &hist,     &n_def,   &stuck};
+    ALCU_TRY(cudaLaunchCooperativeKernel((const void*)k_tx_commit, dim3(grid), dim3(TX_TPB), args, 0, st));
+    unsigned long long got[2];
+    ALCU_TRY(cudaMemcpyAsync(got, n_def, sizeof(got), cudaMemcpyDeviceToHost, st));
+    ALCU_TRY(cudaStreamSynchronize(st));
+    if (got[1]) {
+        gpk_set_error("alcu: topology transactions did not finish");
+        return GPK_ERR_INTERNAL;
+    }
+    if (deferred) *deferred = (int64_t)got[0];
     return GPK_OK;
 }
 
