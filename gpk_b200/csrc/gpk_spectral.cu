@@ -58,8 +58,8 @@ struct SpecConst {
     } while (0)
 
 // wave number of FFT index i on an axis of n points: 2 pi * fftfreq(n, dx)[i]
-__device__ __forceinline__ double wave_number(long long i, int n, double scale) {
-    const long long m = (i <= (n - 1) / 2) ? i : i - n;
+__device__ __forceinline__ double wave_number(int i, int n, double scale) {
+    const int m = (i <= (n - 1) / 2) ? i : i - n;
     return 6.283185307179586 * ((double)m * scale);
 }
 
@@ -169,15 +169,37 @@ __device__ __forceinline__ void strain_at(const SpecConst& c, double kx, double 
 // carries the same Nyquist wave number as the bin, Y(m(k)) is evaluated
 // there explicitly, and H is formed.  The residual sums run over the full
 // spectrum: a stored bin whose mirror is not stored also counts the mirror.
-__global__ void __launch_bounds__(256) k_green(SpecConst c, const double2* __restrict__ e0h, double2* __restrict__ eh,
+//
+// Bound: FP64 issue (some 300 operations a bin, 1.1 M bins at 128^3) over 153 MB.
+// The bins of the halved axis's Nyquist wave number cost twice the others; they
+// are taken last, so that they fill warps of their own (in place, one of 65,
+// they held up every second warp), and 128 registers leave two blocks on an SM
+// (148 left one).  56 -> 46 us at 128^3.
+__global__ void __launch_bounds__(256, 2) k_green(SpecConst c, const double2* __restrict__ e0h, double2* __restrict__ eh,
                                                double* __restrict__ partial) {
     __shared__ double sh[16];
     const long long Nh = c.Nh;
     double r2s = 0.0, b2s = 0.0;
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < Nh;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const long long i2 = idx % c.h2, t = idx / c.h2;
-        const long long i1 = t % c.h1, i0 = t / c.h1;
+    const unsigned h = c.hax == 2 ? c.h2 : c.h1;
+    const unsigned body = (unsigned)(Nh / h) * (h - 1);
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < Nh;
+         q += (long long)gridDim.x * blockDim.x) {
+        // bin q of the order above (fewer than 2^31 bins: 32-bit divisions)
+        unsigned t, ih;
+        if ((unsigned)q < body) {
+            t = (unsigned)q / (h - 1);
+            ih = (unsigned)q - t * (h - 1);
+        } else if (h > 1) {
+            t = (unsigned)q - body;
+            ih = h - 1;
+        } else {
+            t = (unsigned)q;
+            ih = 0;
+        }
+        const long long idx = (long long)t * h + ih;
+        const unsigned t0 = c.hax == 2 ? t / (unsigned)c.h1 : t;
+        const int i0 = (int)t0, i1 = c.hax == 2 ? (int)(t - t0 * (unsigned)c.h1) : (int)ih;
+        const int i2 = c.hax == 2 ? (int)ih : 0;
         const double kx = wave_number(i0, c.e0, c.v0);
         const double ky = wave_number(i1, c.e1, c.v1);
         const double kz = wave_number(i2, c.e2, c.v2);
@@ -188,12 +210,11 @@ __global__ void __launch_bounds__(256) k_green(SpecConst c, const double2* __res
         const bool ny0 = (c.e0 % 2 == 0) && i0 == c.e0 / 2;
         const bool ny1 = (c.e1 % 2 == 0) && i1 == c.e1 / 2;
         const bool ny2 = (c.e2 % 2 == 0) && i2 == c.e2 / 2;
-        const long long ih = c.hax == 2 ? i2 : i1;
         const int eh_n = c.hax == 2 ? c.e2 : c.e1;
-        const bool self_mirror = ih == 0 || ((eh_n % 2 == 0) && ih == eh_n / 2);
+        const bool self_mirror = ih == 0 || ((eh_n % 2 == 0) && (int)ih == eh_n / 2);
         double mr2 = r2, mb2 = b2;
         if (ny0 || ny1 || ny2) {
-            const long long m0 = (c.e0 - i0) % c.e0, m1 = (c.e1 - i1) % c.e1, m2 = (c.e2 - i2) % c.e2;
+            const int m0 = (c.e0 - i0) % c.e0, m1 = (c.e1 - i1) % c.e1, m2 = (c.e2 - i2) % c.e2;
             double2 em[6];
             strain_at(c, wave_number(m0, c.e0, c.v0), wave_number(m1, c.e1, c.v1), wave_number(m2, c.e2, c.v2),
                       conj2(a0), conj2(a1), conj2(a2), em, mr2, mb2);
