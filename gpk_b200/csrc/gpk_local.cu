@@ -246,14 +246,22 @@ __global__ void __launch_bounds__(256) k_projection_tiled(Dims D, const int32_t*
 // 26 x TY x TZ cells has halo rows of exactly 32 cells (R = 3), so for one
 // label a halo row is one 32-bit word; a 7-tap window of a row is a 7-bit
 // pattern, and a table of the weight sums of all 128 patterns per (dy, dz)
-// gives every score in 49 lookups.  Those sums are added in another order
-// than the reference's, so they differ from its sums by far less than
-// 1e-9.  A cell whose screened gain is below -1e-5 and whose best candidate
-// leads the others by more than 1e-9 cannot make a proposal nor pick
+// gives a row's part of a score in one lookup.  Those sums are added in another
+// order than the reference's, so they differ from its sums by far less than
+// 1e-9.  Screening takes the core rows alone (|dy|, |dz| <= 1, 96 % of the
+// weight): a cell whose gain is below -1e-5 even if every tap off the resident
+// label's core were a candidate's, and whose best candidate leads the others
+// by more than the remaining rows weigh, cannot make a proposal nor pick
 // another candidate, whatever the rounding: it keeps the screened values
-// (read only by the proposal test).  Every other cell is queued and summed
-// exactly, tap by tap in z -> y -> x order as the reference adds them
-// (src/gpk_transitions.cpp:67-85), by all threads of the CTA together.
+// (read only by the proposal test).  Every other cell, some 7 % of them, is
+// queued and summed exactly, tap by tap in z -> y -> x order as the reference
+// adds them (src/gpk_transitions.cpp:67-85), by all threads of the CTA together.
+//
+// Bound: latency of a tile's phases (57 k cycles, of them lookups 10 k, exact
+// sums 19 k).  Screening by all 49 rows left 1 % of the cells to the exact sums,
+// which take as long for one cell as for the 30 to 70 of a tile now, but its
+// lookups took 33 k cycles: 0.88 -> 0.66 ms a launch at 256^3.  Bitmaps by one
+// vote per listed label instead of a match per row: 0.70 ms.
 template <bool IS3D> struct BitTile;
 template <> struct BitTile<true> { static constexpr int TY = 8, TZ = 8; };
 template <> struct BitTile<false> { static constexpr int TY = 32, TZ = 1; };
@@ -307,33 +315,26 @@ __device__ __forceinline__ int label_slot_find(const int32_t* keys, int32_t v, i
     return -1;
 }
 
-// screened sums of the resident label and NC candidates: one table lookup
-// per row of 7 taps; li[k] is the bitmap base of label k (0: resident)
-template <bool IS3D, int NC, bool RES = true>
-__device__ __forceinline__ void screen_rows(const uint32_t* __restrict__ bm, const double* __restrict__ rtab,
+// sums over the core rows (|dy|, |dz| <= 1) of the resident label (RES) and NC
+// candidates: one table lookup per row of 7 taps; li[k] is the bitmap base of
+// label k (0: resident)
+template <bool IS3D, int NC, bool RES>
+__device__ __forceinline__ void screen_core(const uint32_t* __restrict__ bm, const double* __restrict__ rtab,
                                             const int li[7], int lx, int ly, int lz, double& resident,
                                             double sup[6]) {
     typedef BitShape<IS3D> S;
     constexpr int R = S::R;
-    const int row0 = (IS3D ? lz * S::HY : 0) + ly;  // halo row of tap (-R, -R) (2-D: (0, -R))
-    // the dz loop stays rolled (code size); the table row of (dy, dz) is
-    // rsum_index(dy^2 + dz^2), with dz^2 in {0, 1, 4, 9}
-#pragma unroll 1
-    for (int dz = (IS3D ? -R : 0); dz <= (IS3D ? R : 0); ++dz) {
-        const int az = dz < 0 ? -dz : dz;
-        // rsum_index(ay^2 + az^2) for ay = 0..3: four bits each, az's 16-bit row of
-        // 0x9876'8543'7421'6310
-        const unsigned idx4 = (unsigned)(0x9876854374216310ull >> (16 * az)) & 0xFFFFu;
+    const int row0 = (IS3D ? (lz + R) * S::HY : 0) + ly + R;  // the cell's own halo row
 #pragma unroll
-        for (int dy = -R; dy <= R; ++dy) {
-            const int row = row0 + (IS3D ? (dz + R) * S::HY : 0) + dy + R;
-            const int ay = dy < 0 ? -dy : dy;
-            const double* t = rtab + ((idx4 >> (4 * ay)) & 0xFu) * 128;
+    for (int dz = (IS3D ? -1 : 0); dz <= (IS3D ? 1 : 0); ++dz)
+#pragma unroll
+        for (int dy = -1; dy <= 1; ++dy) {
+            const int row = row0 + dz * S::HY + dy;
+            const double* t = rtab + (dy * dy + dz * dz) * 128;  // rsum_index is the identity up to 2
             if (RES) resident += t[(bm[li[0] + row] >> lx) & 0x7Fu];
 #pragma unroll
             for (int q = 0; q < NC; ++q) sup[q] += t[(bm[li[q + 1] + row] >> lx) & 0x7Fu];
         }
-    }
 }
 
 // Distinct face-neighbour labels other than pi, in face order, kept in
@@ -383,7 +384,7 @@ __global__ void __launch_bounds__(256) k_bgr_scores_screen(Dims D, const int32_t
     __shared__ int32_t keys[S::HSLOT];
     __shared__ int8_t dense[S::HSLOT];   // bitmap index of a slot, -1 when unused
     __shared__ int s_ncell, s_nl, s_full, s_nexact;
-    __shared__ double s_wtot;  // weight of the whole box
+    __shared__ double s_wtot, s_wrest;  // weight of the whole box, and of its rows off the core
     typedef cub::BlockScan<int, 256> BS;
     __shared__ typename BS::TempStorage scan;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -471,15 +472,20 @@ __global__ void __launch_bounds__(256) k_bgr_scores_screen(Dims D, const int32_t
         }
         if (lane == 0) {
             s_nl = total;
-            double wt = 0.0;
+            double wt = 0.0, wr = 0.0;
             for (int dz = (IS3D ? -R : 0); dz <= (IS3D ? R : 0); ++dz)
-                for (int dy = -R; dy <= R; ++dy) wt += rtab[rsum_index(dy * dy + dz * dz) * 128 + 127];
+                for (int dy = -R; dy <= R; ++dy) {
+                    const double w_row = rtab[rsum_index(dy * dy + dz * dz) * 128 + 127];
+                    wt += w_row;
+                    if (dy * dy > 1 || dz * dz > 1) wr += w_row;
+                }
             s_wtot = wt;
+            s_wrest = wr;
         }
     }
     __syncthreads();
     const int nl = s_nl;
-    const double wtot = s_wtot;
+    const double wtot = s_wtot, wrest = s_wrest;
     const bool screen = !s_full && nl <= (nl_cap < S::NL ? nl_cap : S::NL);
     if (screen) {
         // 4. one word per halo row and listed label (words of absent labels stay 0)
@@ -511,21 +517,20 @@ __global__ void __launch_bounds__(256) k_bgr_scores_screen(Dims D, const int32_t
             for (int q = 0; q < 6; ++q)
                 li[q + 1] = q < nc ? dense[label_slot_find(keys, cand[q], S::HSLOT)] * S::NROWP : li[0];
             double resident = 0.0, sup[6] = {0, 0, 0, 0, 0, 0};
-            screen_rows<IS3D, 0>(bm, rtab, li, lx, ly, lz, resident, sup);
-            // One candidate: it is the best, and its score is at most the
-            // weight of the box outside the resident label, wtot - resident;
-            // when that bound already puts the gain below -1e-5 (with 1e-9 to
-            // spare for the other summation order) its sum is not needed.
-            const bool bounded = nc == 1 && wtot - resident - resident < -1e-5 - 1e-9;
-            const int ncw = __reduce_max_sync(__activemask(), bounded ? 0 : nc);
+            screen_core<IS3D, 0, true>(bm, rtab, li, lx, ly, lz, resident, sup);
+            // No label's score exceeds the box's weight off the resident's
+            // core: where that bound puts every gain below -1e-5 (with 1e-9 to
+            // spare for the order of the sums) there is no proposal, and one
+            // candidate is the best one.  Of several the best has to lead by
+            // more than the rows off the core can hold.
+            const bool bounded = wtot - resident - resident < -1e-5 - 1e-9;
+            const int ncw = __reduce_max_sync(__activemask(), bounded && nc > 1 ? nc : 0);
             switch (ncw) {
             case 0: break;
-            case 1: screen_rows<IS3D, 1, false>(bm, rtab, li, lx, ly, lz, resident, sup); break;
-            case 2: screen_rows<IS3D, 2, false>(bm, rtab, li, lx, ly, lz, resident, sup); break;
-            case 3: screen_rows<IS3D, 3, false>(bm, rtab, li, lx, ly, lz, resident, sup); break;
-            default: screen_rows<IS3D, 6, false>(bm, rtab, li, lx, ly, lz, resident, sup); break;
+            case 2: screen_core<IS3D, 2, false>(bm, rtab, li, lx, ly, lz, resident, sup); break;
+            case 3: screen_core<IS3D, 3, false>(bm, rtab, li, lx, ly, lz, resident, sup); break;
+            default: screen_core<IS3D, 6, false>(bm, rtab, li, lx, ly, lz, resident, sup); break;
             }
-            if (bounded) sup[0] = wtot - resident;
             double best = -1.0, second = -1.0;
             int32_t best_label = pi;
 #pragma unroll
@@ -534,11 +539,11 @@ __global__ void __launch_bounds__(256) k_bgr_scores_screen(Dims D, const int32_t
                 if (sup[q] > best) { second = best; best = sup[q]; best_label = cand[q]; }
                 else if (sup[q] > second) second = sup[q];
             }
-            if (best - resident < -1e-5 && (nc < 2 || best - second > 1e-9)) {
+            if (bounded && (nc < 2 || best - second > wrest + 1e-9)) {
                 settled = true;
                 const int i = D.idx(z0 + lz, y0 + ly, x0 + lx);
                 res_out[i] = (real)resident;
-                best_out[i] = (real)best;
+                best_out[i] = (real)(nc == 1 ? wtot - resident : best);
                 phi_comp[i] = best_label;
             }
         }
