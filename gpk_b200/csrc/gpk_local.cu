@@ -257,11 +257,13 @@ __global__ void __launch_bounds__(256) k_projection_tiled(Dims D, const int32_t*
 // queued and summed exactly, tap by tap in z -> y -> x order as the reference
 // adds them (src/gpk_transitions.cpp:67-85), by all threads of the CTA together.
 //
-// Bound: latency of a tile's phases (57 k cycles, of them lookups 10 k, exact
-// sums 19 k).  Screening by all 49 rows left 1 % of the cells to the exact sums,
-// which take as long for one cell as for the 30 to 70 of a tile now, but its
-// lookups took 33 k cycles: 0.88 -> 0.66 ms a launch at 256^3.  Bitmaps by one
-// vote per listed label instead of a match per row: 0.70 ms.
+// Bound: latency of a tile's phases.  Screening by all 49 rows left 1 % of the
+// cells to the exact sums, whose time a tile pays for one cell as for the 30 to
+// 70 now, but its lookups took 33 k of a tile's 75 k cycles: 0.88 -> 0.66 ms a
+// launch at 256^3.  The exact sums on one thread a cell, every tap's label
+// compared with every candidate, were 19 k of the remaining cycles; on four
+// lanes a cell, one label each, from the bitmaps: 0.66 -> 0.51 ms.  (Bitmaps by
+// one vote per listed label instead of a match per row: 0.04 ms slower.)
 template <bool IS3D> struct BitTile;
 template <> struct BitTile<true> { static constexpr int TY = 8, TZ = 8; };
 template <> struct BitTile<false> { static constexpr int TY = 32, TZ = 1; };
@@ -335,6 +337,28 @@ __device__ __forceinline__ void screen_core(const uint32_t* __restrict__ bm, con
 #pragma unroll
             for (int q = 0; q < NC; ++q) sup[q] += t[(bm[li[q + 1] + row] >> lx) & 0x7Fu];
         }
+}
+
+// the exact sum of one label from its bitmap: the weight of every set tap, z -> y -> x
+template <bool IS3D>
+__device__ __forceinline__ double bitmap_sum(const uint32_t* __restrict__ bml, const double* __restrict__ w, int lx,
+                                             int ly, int lz) {
+    typedef BitShape<IS3D> S;
+    constexpr int R = S::R;
+    double sum = 0.0;
+#pragma unroll 1
+    for (int dz = (IS3D ? -R : 0); dz <= (IS3D ? R : 0); ++dz) {
+        const uint32_t* row = bml + (IS3D ? (lz + dz + R) * S::HY : 0) + ly;
+        const double* wz = w + dz * dz;
+#pragma unroll
+        for (int dy = -R; dy <= R; ++dy) {
+            const uint32_t pat = row[dy + R] >> lx;
+#pragma unroll
+            for (int dx = -R; dx <= R; ++dx)
+                if ((pat >> (dx + R)) & 1u) sum += wz[dy * dy + dx * dx];
+        }
+    }
+    return sum;
 }
 
 // Distinct face-neighbour labels other than pi, in face order, kept in
@@ -555,6 +579,46 @@ __global__ void __launch_bounds__(256) k_bgr_scores_screen(Dims D, const int32_t
     if (tid == 0 && stats) {
         atomicAdd(&stats->score_cells, (unsigned long long)ncell);
         atomicAdd(&stats->score_exact, (unsigned long long)nexact);
+    }
+    if (screen) {
+        // four lanes a cell, one label each (two where more than four are there)
+        const int sub = tid & 3;
+        for (int e0 = 0; e0 < nexact; e0 += 64) {
+            const int e = e0 + (tid >> 2);
+            const bool act = e < nexact;
+            const int lc = cells[exact[act ? e : 0]];
+            const int lx = lc % S::TX, ly = (lc / S::TX) % S::TY, lz = lc / (S::TX * S::TY);
+            const int cb = ((IS3D ? lz + R : 0) * S::HY + ly + R) * S::HX + lx + R;
+            const int32_t pi = lab[cb];
+            int32_t cand[6];
+            const int nc = face_candidates<IS3D>(lab, cb, pi, cand);
+            double sum[2] = {0.0, 0.0};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = sub + 4 * h;  // label 0 is the resident's, k the candidate k - 1
+                if (!act || k > nc) continue;
+                int32_t v = pi;
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    if (q + 1 == k) v = cand[q];
+                sum[h] = bitmap_sum<IS3D>(bm + dense[label_slot_find(keys, v, S::HSLOT)] * S::NROWP, w, lx, ly, lz);
+            }
+            __syncwarp();
+            double best = -1.0;
+            int32_t best_label = pi;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const double v = __shfl_sync(0xffffffffu, sum[(q + 1) >> 2], (q + 1) & 3, 4);
+                if (q < nc && v > best) { best = v; best_label = cand[q]; }
+            }
+            if (act && sub == 0) {
+                const int i = D.idx(z0 + lz, y0 + ly, x0 + lx);
+                res_out[i] = (real)sum[0];
+                best_out[i] = (real)best;
+                phi_comp[i] = best_label;
+            }
+        }
+        return;
     }
     for (int e = tid; e < nexact; e += 256) {
         const int lc = cells[exact[e]];
