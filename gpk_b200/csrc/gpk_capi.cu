@@ -75,6 +75,17 @@ int gpk_alloc(gpk_grid* G, void** p, size_t bytes) {
     return GPK_OK;
 }
 
+bool gpk_alloc_optional(gpk_grid* G, void** p, size_t bytes) {
+    if (cudaMalloc(p, bytes) != cudaSuccess) {
+        cudaGetLastError();  // not the error of the launches that follow
+        *p = nullptr;
+        return false;
+    }
+    G->allocations.push_back(*p);
+    G->device_bytes += bytes;
+    return true;
+}
+
 static void gpk_free(gpk_grid* G, void* p) {
     if (!p) return;
     auto it = std::find(G->allocations.begin(), G->allocations.end(), p);

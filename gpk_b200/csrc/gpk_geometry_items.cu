@@ -875,7 +875,7 @@ static bool for_radius(int R, F f) {
 // capture, which allocates nothing).
 template <typename real>
 int gpk_geometry_items_init(gpk_grid* G) {
-    if (G->item_counters) return GPK_OK;
+    if (G->item_counters || G->item_no_room) return GPK_OK;
     const HostKernels<real>* hk = (const HostKernels<real>*)G->host_kernels;
     const int R = hk->geom_radius;
     const std::vector<real>& taps = hk->geom_table;
@@ -908,7 +908,16 @@ int gpk_geometry_items_init(gpk_grid* G) {
     const size_t slots = ((size_t)D.N + 64 * (size_t)ntiles + 3) & ~(size_t)3;
     const size_t table = sizeof(real) * packed.size();
     unsigned char* base = nullptr;
-    GPK_TRY(gpk_alloc(G, (void**)&base, 16 + table + 12 * slots + 4 * (size_t)G->item_pool));
+    const size_t fixed = 16 + table + 12 * slots;
+    // a full device: the smallest pool (most tiles compare labels), or no items
+    // at all (the per-cell kernel, which needs no memory of its own)
+    if (!gpk_alloc_optional(G, (void**)&base, fixed + 4 * (size_t)G->item_pool)) {
+        G->item_pool = 4096;
+        if (!gpk_alloc_optional(G, (void**)&base, fixed + 4 * (size_t)G->item_pool)) {
+            G->item_no_room = true;
+            return GPK_OK;
+        }
+    }
     // (the interface mask of this step ran before there were counters to clear)
     GPK_CUDA_TRY(cudaMemsetAsync(base, 0, 16, G->stream));
     G->d_geom_packed = base + 16;
@@ -925,11 +934,12 @@ template int gpk_geometry_items_init<float>(gpk_grid*);
 template int gpk_geometry_items_init<double>(gpk_grid*);
 
 // The direct geometry for kernel radii 4..10 (Gaussian radius 2..8); returns
-// -1 for other radii (the caller then uses the per-cell kernel).
+// -1 for other radii and where the device has no room for the items (the caller then uses the per-cell kernel).
 template <typename real>
 int gpk_geometry_items(gpk_grid* G, int R, real inv_dx, real inv_dx2, real dx, real kappa_limit) {
     if (R < 4 || R > 10) return -1;
     GPK_TRY(gpk_geometry_items_init<real>(G));
+    if (!G->item_counters) return -1;
     SumArgs<real> a{};
     a.D = G->d;
     a.phi = G->phi;

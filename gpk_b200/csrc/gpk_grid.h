@@ -88,6 +88,7 @@ struct gpk_grid {
     // separable geometry: label by label over the whole grid, or per label box
     // (gpk_separable.cu: values of the passes; label index and regions)
     void* sep_I = nullptr; void* sep_t1 = nullptr; void* sep_t2 = nullptr; void* sep_S = nullptr;
+    size_t sep_cap[3] = {};
     void* sep_box = nullptr; void* sep_table = nullptr; size_t sep_table_bytes = 0;
     // labels
     int32_t* count = nullptr;              // cells per label
@@ -106,6 +107,7 @@ struct gpk_grid {
     int32_t* item_word = nullptr; int32_t* item_cell = nullptr;
     uint32_t* item_support = nullptr; uint32_t* item_words = nullptr;
     unsigned item_pool = 0;
+    bool item_no_room = false;
     unsigned* item_counters = nullptr;
     gpk_dev::StepScalars* scal = nullptr;  // device scalars
     gpk_dev::StepScalars* h_scal = nullptr;  // pinned host mirror
@@ -172,6 +174,8 @@ template <typename real> int gpk_projection_tiled(gpk_grid* G, int radius);
 int gpk_recount_labels(gpk_grid* G);
 int gpk_topology_simple_move_impl(gpk_grid* G, int cell, int32_t new_label, int* result);
 int gpk_alloc(gpk_grid* G, void** p, size_t bytes);
+// memory the grid can do without: false (and no error) when there is none
+bool gpk_alloc_optional(gpk_grid* G, void** p, size_t bytes);
 int gpk_ensure_label_capacity(gpk_grid* G, int cap);
 int gpk_sync_scalars(gpk_grid* G);
 template <typename real> int gpk_remap_pass_graph(gpk_grid* G, const unsigned long long* gate);

@@ -311,10 +311,17 @@ int gpk_geometry_separable(gpk_grid* G, real dx, real kappa_limit) {
     }
     if (regions.empty()) return GPK_OK;
     // workspace (kept): values of the three passes, taps' run sums, label index and regions
-    const size_t cap1 = 8 * (size_t)D.N, cap2 = 5 * (size_t)D.N, cap3 = 4 * (size_t)D.N;
+    // (many labels' boxes at once; where the device has no room for that, one
+    // label's at least, which is less than the whole-grid passes take)
     if (!G->sep_box) {
+        const size_t extra = (size_t)K * (K + 1);
         void* p = nullptr;
-        GPK_TRY(gpk_alloc(G, &p, sizeof(real) * (cap1 + cap2 + cap3 + (size_t)K * (K + 1))));
+        if (gpk_alloc_optional(G, &p, sizeof(real) * (17 * (size_t)D.N + extra))) {
+            G->sep_cap[0] = 8 * (size_t)D.N; G->sep_cap[1] = 5 * (size_t)D.N; G->sep_cap[2] = 4 * (size_t)D.N;
+        } else {
+            GPK_TRY(gpk_alloc(G, &p, sizeof(real) * (3 * (size_t)D.N + extra)));
+            G->sep_cap[0] = G->sep_cap[1] = G->sep_cap[2] = (size_t)D.N;
+        }
         G->sep_box = p;
         std::vector<real> runs((size_t)K * (K + 1), (real)0);
         for (int s = 0; s < K; ++s) {
@@ -324,10 +331,11 @@ int gpk_geometry_separable(gpk_grid* G, real dx, real kappa_limit) {
                 runs[(size_t)s * (K + 1) + l] = acc;
             }
         }
-        GPK_CUDA_TRY(cudaMemcpyAsync((real*)p + cap1 + cap2 + cap3, runs.data(), sizeof(real) * runs.size(),
+        GPK_CUDA_TRY(cudaMemcpyAsync((real*)p + G->sep_cap[0] + G->sep_cap[1] + G->sep_cap[2], runs.data(), sizeof(real) * runs.size(),
                                      cudaMemcpyHostToDevice, G->stream));
         GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
     }
+    const size_t cap1 = G->sep_cap[0], cap2 = G->sep_cap[1], cap3 = G->sep_cap[2];
     real* t1 = (real*)G->sep_box;
     real* t2 = t1 + cap1;
     real* s = t2 + cap2;
