@@ -41,11 +41,11 @@ SETTLE = 16  # steps evolved while preparing the input state (untimed)
 # single-thread CPU sample: same grain size (4096 cells per grain) on a 128^3 sub-volume
 CPU_SIZE = 128
 CPU_GRAINS = 512
-# DRAM read + write bytes of one k_geometry_tiled launch on the 256^3 / 4096
+# DRAM read + write bytes of one k_geo_prepare and one k_geo_sum launch on the 256^3 / 4096
 # grain / sigma 1.5 workload, measured by ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum, one-pass metrics, the launch of the third warm-up step)
-GEOMETRY_TRAFFIC_256 = 527.80e6
-GEOMETRY_TRAFFIC_NOTE = ("DRAM bytes (read 300.98 MB + write 226.82 MB) of one launch of the kernel on this "
+# dram__bytes_write.sum, one-pass metrics, the launches of the third warm-up step)
+GEOMETRY_TRAFFIC_256 = 1005.04e6
+GEOMETRY_TRAFFIC_NOTE = ("DRAM bytes (read 586.73 MB + write 418.30 MB) of one launch of both kernels on this "
                          "256^3 workload, measured by ncu with the one-pass dram__bytes metrics")
 
 
@@ -685,11 +685,10 @@ def separable_measurement(n: int = 256, grains: int = 32, sigma: float = 5.0, se
     grains, sigma 5 cells (Gaussian radius 18, geometry radius 20 > 18), FP32
     reference arithmetic.  Per step and interface label: the x pass of the
     indicator, the y and z passes, the evaluation on the label's interface
-    cells.  Algorithmic bytes of the geometry stage: the labels read once
-    per interface label (4 B per cell) and the normals and curvature of the
-    interface cells written once (16 B each); the intermediate smoothed
-    fields between the passes are not algorithmic bytes (the traffic they
-    cause is in `intermediate_bytes_per_step`)."""
+    cells, over the box of those cells.  Algorithmic bytes of the geometry
+    stage: the labels read once (4 B per cell) and the normals and curvature
+    of the interface cells written once (16 B each); the intermediate smoothed
+    fields between the passes are not algorithmic bytes."""
     import torch
     from gpk_b200 import GPKGrid, thermo
     g = GPKGrid(n, n, n, 1.0, thermo.isotropic(1.0, 1.0), 0.0, sigma)
@@ -714,17 +713,16 @@ def separable_measurement(n: int = 256, grains: int = 32, sigma: float = 5.0, se
     geo_ms = st["geometry"][0] / max(1, st["geometry"][1])
     cells = n ** 3
     n_active = g.interface_fraction() * cells
-    geo_bytes = grains * cells * 4.0 + n_active * 16.0
-    inter_bytes = grains * cells * 29.0  # x-pass output, y and z passes in/out, evaluation reads
+    geo_bytes = cells * 4.0 + n_active * 16.0
     peak, peak_kind = _peaks()
     res = {"workload": f"3-D isotropic grain growth {n}^3, {grains} Voronoi grains, sigma {sigma} cells "
                        "(separable geometry: per-label x/y/z Gaussian passes + interface evaluation), FP32",
            "steps": steps, "warmup": warmup, "ms_per_step": ms, "value": cells / (ms / 1e3),
            "unit": "cell-updates/s", "geometry_ms_per_step": geo_ms,
            "stages_ms_per_step": {k: v[0] / max(1, v[1]) for k, v in st.items()},
-           "roofline": {"kernels": "k_sep_x_indicator_f2, k_sep_pass (y, z), k_separable_eval per label",
+           "roofline": {"kernels": "k_sep_box_x, k_sep_box_line (y, z), k_sep_box_eval",
                         "bound": "fp32 issue (the reference's unfused multiply + add per tap)",
-                        "algorithmic_bytes_per_step": geo_bytes, "intermediate_bytes_per_step": inter_bytes,
+                        "algorithmic_bytes_per_step": geo_bytes,
                         "achieved": geo_bytes / (geo_ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                         "frac": geo_bytes / (geo_ms / 1e3) / 1e9 / peak, "peak_kind": peak_kind}}
     g.close()
@@ -892,11 +890,11 @@ def run_gpu_arm(args):
     tap_adds = n_active * W ** 3 * 9 / (geo_ms / 1e3)
     separable = (W - 1) // 2 > 18
     if separable:
-        # per interface label the labels once (4 B per cell); the interface
-        # cells' normals and curvature (16 B) once; intermediates excluded
-        geo_bytes = GRAINS * cells * 4.0 + n_active * 16
+        # the labels once (4 B per cell), the interface cells' normals and
+        # curvature (16 B) once; intermediates excluded
+        geo_bytes = cells * 4.0 + n_active * 16
         achieved = geo_bytes / (geo_ms / 1e3) / 1e9
-    roofline = {"kernel": "k_geometry_tiled (label-bitmap Gaussian-Hessian tensor stencil + competitor)",
+    roofline = {"kernel": "k_geo_prepare + k_geo_sum (label-bitmap Gaussian-Hessian tensor stencil + competitor)",
                 "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_kind": peak_kind, "traffic": traffic,
                 "algorithmic_bytes_per_launch": geo_bytes, "ms_per_launch": geo_ms,
@@ -908,7 +906,7 @@ def run_gpu_arm(args):
                             "peak_fp32_adds_per_s": _fp32_add_peak(clocks["sm_mhz"] or 1965.0),
                             "frac": tap_adds / _fp32_add_peak(clocks["sm_mhz"] or 1965.0)}}
     if separable:
-        roofline = {"kernel": "k_sep_pass x3 + k_separable_eval per interface label (separable geometry)",
+        roofline = {"kernel": "k_sep_box_x + k_sep_box_line x2 + k_sep_box_eval, all label boxes per launch (separable geometry)",
                     "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "peak_kind": peak_kind, "traffic": None, "algorithmic_bytes_per_launch": geo_bytes,
                     "ms_per_launch": geo_ms}
