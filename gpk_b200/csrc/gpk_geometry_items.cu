@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "gpk_grid.h"
+#include "gpk_pool.h"
 
 namespace gpk_dev {
 
@@ -230,6 +231,12 @@ struct GeoItems {
     unsigned* counters;  // items, words taken, next item (the interface mask's kernel clears them)
 };
 
+struct PoolCounter {
+    unsigned* p;
+    __device__ __forceinline__ unsigned load() { return *(volatile unsigned*)p; }
+    __device__ __forceinline__ unsigned exchange(unsigned old, unsigned next) { return atomicCAS(p, old, next); }
+};
+
 template <int R, bool IS3D, int TD>
 __global__ void __launch_bounds__(256) k_geo_prepare(Dims D, const int32_t* __restrict__ phi,
                                                      const uint8_t* __restrict__ mask, int ntx, int nty, GeoItems it) {
@@ -389,13 +396,8 @@ __global__ void __launch_bounds__(256) k_geo_prepare(Dims D, const int32_t* __re
     const int nitem = (ncell + 63) / 64;
     if (tid == 0) {
         s_item = atomicAdd(&it.counters[0], (unsigned)nitem);
-        const unsigned need = (unsigned)nl * S::NROW;
-        s_word = 0;
-        // (64-bit test: the sum of all requests may pass 2^32 only where the pool is long full)
-        const unsigned old = need <= it.pool ? atomicAdd(&it.counters[1], need) : it.pool;
-        s_ok = old <= it.pool && it.pool - old >= need;
-        s_word = old;
-        if (!s_ok && need <= it.pool) atomicSub(&it.counters[1], need);
+        PoolCounter taken{it.counters + 1};
+        s_ok = pool_take(taken, (unsigned)nl * S::NROW, it.pool, s_word);
     }
     __syncthreads();
     const bool okw = s_ok != 0;
