@@ -68,6 +68,7 @@ def lib() -> C.CDLL:
         "gpk_grid_run": ([vp, dbl, dbl, i32, C.POINTER(i32)], i32),
         "gpk_grid_sync": ([vp], i32),
         "gpk_grid_geometry": ([vp], i32),
+        "gpk_grid_geometry_stats": ([vp, C.POINTER(u64)], i32),
         "gpk_grid_max_dt": ([vp, C.POINTER(dbl)], i32),
         "gpk_grid_phase_volume": ([vp, C.c_int32, C.POINTER(dbl)], i32),
         "gpk_grid_n_grains": ([vp, C.POINTER(i32)], i32),

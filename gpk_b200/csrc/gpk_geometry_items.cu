@@ -228,7 +228,7 @@ struct GeoItems {
     uint32_t* support;   // per face 5 bits: like labels around the cell, 31 where the face has the cell's own label
     uint32_t* words;     // bitmap pool
     unsigned pool;       // words in the pool
-    unsigned* counters;  // items, words taken, next item (the interface mask's kernel clears them)
+    unsigned* counters;  // items, words taken, next item, tiles without bitmaps (the geometry's mask launch clears them)
 };
 
 struct PoolCounter {
@@ -398,6 +398,7 @@ __global__ void __launch_bounds__(256) k_geo_prepare(Dims D, const int32_t* __re
         s_item = atomicAdd(&it.counters[0], (unsigned)nitem);
         PoolCounter taken{it.counters + 1};
         s_ok = pool_take(taken, (unsigned)nl * S::NROW, it.pool, s_word);
+        if (!s_ok) atomicAdd(&it.counters[3], 1u);
     }
     __syncthreads();
     const bool okw = s_ok != 0;
@@ -883,6 +884,7 @@ int gpk_geometry_items_init(gpk_grid* G) {
     const std::vector<real>& taps = hk->geom_table;
     std::vector<real> packed;
     long long ntiles = 0;
+    double label_words = 0;  // words per cell that one label in every tile takes
     const bool is3d = G->d.is3d();
     const Dims D = G->d;
     if (!for_radius(R, [&](auto r) {
@@ -893,17 +895,21 @@ int gpk_geometry_items_init(gpk_grid* G) {
             if (is3d) {
                 pack_table<real, RR, true>(taps, packed);
                 tiles(ItemTile<RR, true, 1>::TX, ItemTile<RR, true, 1>::TY, ItemTile<RR, true, 1>::TZ);
+                label_words = (double)ItemTile<RR, true, 1>::NROW / ItemTile<RR, true, 1>::NCELL;
             } else {
                 pack_table<real, RR, false>(taps, packed);
                 tiles(ItemTile<RR, false, 4>::TX, ItemTile<RR, false, 4>::TY, 1);
+                label_words = (double)ItemTile<RR, false, 1>::NROW / ItemTile<RR, false, 1>::NCELL;
             }
         }))
         return GPK_OK;
-    // words: a tile of a polycrystal of 16^3-cell grains takes about 2.4 per
-    // cell; smaller grids get room for many more labels per tile, and tiles
-    // that find the pool full compare labels instead
-    const size_t want = is3d ? std::max((size_t)4 * D.N, std::min((size_t)64 * D.N, (size_t)8 << 20))
-                             : std::max((size_t)D.N, std::min((size_t)16 * D.N, (size_t)1 << 20));
+    // words: 20 labels in every tile (0.38 words a cell and label at R = 8, 0.49
+    // at R = 9, 0.66 at R = 10): tiles of a polycrystal with grains of 1500 cells
+    // meet 9 to 11 on average.  Smaller grids get room for more labels per tile, and tiles that find
+    // the pool full compare labels instead (and are counted)
+    const size_t base_words = (size_t)(20 * label_words * (double)D.N);
+    const size_t want = is3d ? std::max(base_words, std::min((size_t)64 * D.N, (size_t)8 << 20))
+                             : std::max(base_words, std::min((size_t)16 * D.N, (size_t)1 << 20));
     // (the padding of an item reads the pool's first words)
     G->item_pool = (unsigned)std::max(std::min(want, (size_t)1 << 31), (size_t)4096);
     // one allocation: counters, table, items, words

@@ -148,7 +148,8 @@ __global__ void __launch_bounds__(MASK_TPB) k_mask_list(Dims D, const int32_t* _
             s->n_cand = 0; s->n_prop = 0; s->waves = 0; s->n_near = 0; s->vmax = 0.0;
         }
         if (job.clear_waves) s->waves = 0;
-        if (job.item_counters) job.item_counters[0] = job.item_counters[1] = job.item_counters[2] = 0u;
+        if (job.item_counters)
+            for (int k = 0; k < 4; ++k) job.item_counters[k] = 0u;
     }
     constexpr int TILE = MASK_TPB * IPT;
     constexpr int G = W4 ? 4 : 1, ROUNDS = IPT / G, CHUNKS = ROUNDS * MASK_WARPS;
@@ -1604,7 +1605,6 @@ static int launch_mask(gpk_grid* G, MaskJob job) {
     const bool large = G->d.N >= 1 << 22;
     const int tile = MASK_TPB * (large ? 32 : 8);
     const int nt = (G->d.N + tile - 1) / tile;
-    job.item_counters = G->item_counters;
     job.rsz = (int)G->rsz;
     ListState* L = (ListState*)G->list_state;
     const Dims D = G->d;
@@ -1628,6 +1628,7 @@ int gpk_interface_mask(gpk_grid* G, const unsigned long long* gate) {
 // the first mask of a step (or of a geometry alone): the geometry's fields start at zero
 static MaskJob geometry_job(gpk_grid* G) {
     MaskJob job;
+    job.item_counters = G->item_counters;
     for (int f : {GPK_FIELD_NX, GPK_FIELD_NY, GPK_FIELD_NZ, GPK_FIELD_KAPPA}) job.zero[job.nzero++] = G->f[f];
     return job;
 }

@@ -293,6 +293,14 @@ class GPKGrid:
         """Mask and geometry of the current labels, without stepping."""
         check(lib().gpk_grid_geometry(self._h))
 
+    def geometry_stats(self) -> dict:
+        """Of the last direct geometry: items of 64 interface cells, tiles
+        without room for their label bitmaps, bitmap words taken and there are."""
+        out = (C.c_uint64 * 4)()
+        check(lib().gpk_grid_geometry_stats(self._h, out))
+        return {"items": int(out[0]), "tiles_without_bitmaps": int(out[1]), "words": int(out[2]),
+                "pool_words": int(out[3])}
+
     def stream_ptr(self) -> int:
         p = C.c_void_p()
         check(lib().gpk_grid_stream(self._h, C.byref(p)))

@@ -247,6 +247,12 @@ int gpk_grid_stage_times(gpk_grid* grid, double ms[GPK_NUM_STAGES], uint64_t cal
  * cells given remap scores, those of them summed tap by tap}, summed since
  * the last read.                                                           */
 int gpk_grid_wave_stats(gpk_grid* grid, uint64_t out[10]);
+/* The direct geometry of the last step or gpk_grid_geometry call: out = {items
+ * of 64 interface cells, tiles that found no room for their label bitmaps
+ * (their rows are compared label by label, many times slower), bitmap words
+ * taken, bitmap words there are}; the first three are zero where another
+ * geometry ran.                                                            */
+int gpk_grid_geometry_stats(gpk_grid* grid, uint64_t out[4]);
 /* Kernel selection (all give identical results): 0 = tiled shared-memory
  * kernels where an instantiation exists (default), 1 = the per-interface-
  * cell kernels, 2 = tiled kernels without label bitmaps in the geometry

@@ -1,5 +1,8 @@
-"""Geometry tiles that ask for very different shares of a pool too small for
-all of them: every repetition equals the per-cell kernel, bit for bit.
+"""The pool of the geometry's label bitmaps.
+
+Tiles that ask for very different shares of a pool too small for all of them:
+every repetition equals the per-cell kernel, bit for bit, and the tiles without
+bitmaps are counted.  A polycrystal of small grains finds room at every radius.
 """
 import numpy as np
 import pytest
@@ -41,4 +44,22 @@ def test_uneven_requests(sigma, precision):
             ref = ref or got
             for f in FIELDS:
                 assert bits_equal(ref[f], got[f]), (kind, rep, f)
+            st = g.geometry_stats()
+            assert st["words"] <= st["pool_words"] and (st["tiles_without_bitmaps"] > 0) == (kind == "tiled"), st
+            assert (st["items"] > 0) == (kind == "tiled"), st
         g.close()
+
+
+@pytest.mark.parametrize("sigma,cells", [(1.5, 1500), (2.0, 1500), (2.2, 1500)])  # radii 8, 9, 10
+def test_small_grains_find_room(sigma, cells):
+    """2.4 M cells in grains of 1500: 9 to 11 labels a tile, 4.4 to 6.6 words a cell."""
+    shape = (128, 136, 136)
+    g = GPKGrid(*shape, 1.0, thermo.isotropic(1.0, 1.0), 0.0, sigma)
+    g.voronoi(int(np.prod(shape)) // cells, 7)
+    g.geometry()
+    st = g.geometry_stats()
+    assert st["tiles_without_bitmaps"] == 0 and st["words"] > 2 * np.prod(shape), st
+    g.set_geometry_kernel("tiled_batched")  # no pool: every tile with interface cells is counted
+    g.geometry()
+    assert g.geometry_stats()["tiles_without_bitmaps"] > 0
+    g.close()
