@@ -675,14 +675,14 @@ extern "C" int gpk_grid_step_n(gpk_grid* G, int n, double dt, double dt_cap, dou
 
 extern "C" int gpk_grid_geometry_stats(gpk_grid* G, uint64_t out[4]) {
     if (!G || !out) return GPK_ERR_INVALID_ARGUMENT;
-    unsigned c[4] = {0, 0, 0, 0};
+    ItemCounters c{};
     if (G->item_counters) {
-        GPK_CUDA_TRY(cudaMemcpyAsync(c, G->item_counters, sizeof(c), cudaMemcpyDeviceToHost, G->stream));
+        GPK_CUDA_TRY(cudaMemcpyAsync(&c, G->item_counters, sizeof(c), cudaMemcpyDeviceToHost, G->stream));
         GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
     }
-    out[0] = c[0];
-    out[1] = c[3];
-    out[2] = c[1];
+    out[0] = c.items;
+    out[1] = c.no_bitmap;
+    out[2] = std::min<uint64_t>(c.words, G->item_pool);
     out[3] = G->item_pool;
     return GPK_OK;
 }

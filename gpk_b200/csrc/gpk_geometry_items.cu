@@ -228,13 +228,13 @@ struct GeoItems {
     uint32_t* support;   // per face 5 bits: like labels around the cell, 31 where the face has the cell's own label
     uint32_t* words;     // bitmap pool
     unsigned pool;       // words in the pool
-    unsigned* counters;  // items, words taken, next item, tiles without bitmaps (the geometry's mask launch clears them)
+    ItemCounters* counters;  // (the geometry's mask launch clears them)
 };
 
 struct PoolCounter {
-    unsigned* p;
-    __device__ __forceinline__ unsigned load() { return *(volatile unsigned*)p; }
-    __device__ __forceinline__ unsigned exchange(unsigned old, unsigned next) { return atomicCAS(p, old, next); }
+    unsigned long long* p;
+    __device__ __forceinline__ unsigned long long load() { return *(volatile unsigned long long*)p; }
+    __device__ __forceinline__ unsigned long long add(unsigned v) { return atomicAdd(p, (unsigned long long)v); }
 };
 
 template <int R, bool IS3D, int TD>
@@ -395,10 +395,10 @@ __global__ void __launch_bounds__(256) k_geo_prepare(Dims D, const int32_t* __re
     // 4. room for the items and the words
     const int nitem = (ncell + 63) / 64;
     if (tid == 0) {
-        s_item = atomicAdd(&it.counters[0], (unsigned)nitem);
-        PoolCounter taken{it.counters + 1};
+        s_item = atomicAdd(&it.counters->items, (unsigned)nitem);
+        PoolCounter taken{&it.counters->words};
         s_ok = pool_take(taken, (unsigned)nl * S::NROW, it.pool, s_word);
-        if (!s_ok) atomicAdd(&it.counters[3], 1u);
+        if (!s_ok) atomicAdd(&it.counters->no_bitmap, 1u);
     }
     __syncthreads();
     const bool okw = s_ok != 0;
@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(geo_warps<real, IS3D>() * 32, IS3D ? 1 : 3) k_
     extern __shared__ __align__(16) unsigned char smem[];
     typedef GeoTable<real, R, IS3D> T;
     real* tab = reinterpret_cast<real*>(smem);
-    const int n = (int)a.it.counters[0];
+    const int n = (int)a.it.counters->items;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = gridDim.x;
     if ((int)blockIdx.x >= 2 * n) return;  // (a CTA may take half an item)
     copy_table(tab, a.table + T::offset(T::S0), (int)T::smem());
@@ -822,7 +822,7 @@ __global__ void __launch_bounds__(geo_warps<real, IS3D>() * 32, IS3D ? 1 : 3) k_
             if (cell[s] >= 0)
                 finish_cell<real>(a, cell[s], acc[s], a.it.support[(size_t)item * 64 + 32 * s + lane]);
         int nx = 0;
-        if (lane == 0) nx = (int)atomicAdd(&a.it.counters[2], 1u) + G * NW;
+        if (lane == 0) nx = (int)atomicAdd(&a.it.counters->next, 1u) + G * NW;
         item = __shfl_sync(0xffffffffu, nx, 0);
     }
 }
@@ -916,7 +916,7 @@ int gpk_geometry_items_init(gpk_grid* G) {
     const size_t slots = ((size_t)D.N + 64 * (size_t)ntiles + 3) & ~(size_t)3;
     const size_t table = sizeof(real) * packed.size();
     unsigned char* base = nullptr;
-    const size_t fixed = 16 + table + 12 * slots;
+    const size_t head = sizeof(ItemCounters), fixed = head + table + 12 * slots;
     // a full device: the smallest pool (most tiles compare labels), or no items
     // at all (the per-cell kernel, which needs no memory of its own)
     if (!gpk_alloc_optional(G, (void**)&base, fixed + 4 * (size_t)G->item_pool)) {
@@ -927,15 +927,15 @@ int gpk_geometry_items_init(gpk_grid* G) {
         }
     }
     // (the interface mask of this step ran before there were counters to clear)
-    GPK_CUDA_TRY(cudaMemsetAsync(base, 0, 16, G->stream));
-    G->d_geom_packed = base + 16;
+    GPK_CUDA_TRY(cudaMemsetAsync(base, 0, head, G->stream));
+    G->d_geom_packed = base + head;
     GPK_CUDA_TRY(cudaMemcpyAsync(G->d_geom_packed, packed.data(), table, cudaMemcpyHostToDevice, G->stream));
     GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
-    G->item_word = (int32_t*)(base + 16 + table);
+    G->item_word = (int32_t*)(base + head + table);
     G->item_cell = G->item_word + slots;
     G->item_support = (uint32_t*)(G->item_cell + slots);
     G->item_words = G->item_support + slots;
-    G->item_counters = (unsigned*)base;
+    G->item_counters = (ItemCounters*)base;
     return GPK_OK;
 }
 template int gpk_geometry_items_init<float>(gpk_grid*);

@@ -108,7 +108,7 @@ struct gpk_grid {
     uint32_t* item_support = nullptr; uint32_t* item_words = nullptr;
     unsigned item_pool = 0;
     bool item_no_room = false;
-    unsigned* item_counters = nullptr;
+    gpk_dev::ItemCounters* item_counters = nullptr;
     gpk_dev::StepScalars* scal = nullptr;  // device scalars
     gpk_dev::StepScalars* h_scal = nullptr;  // pinned host mirror
     void* host_kernels = nullptr;          // HostKernels<real>*

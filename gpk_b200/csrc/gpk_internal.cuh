@@ -53,6 +53,13 @@ template <typename T> __host__ __device__ __forceinline__ T dclamp(T v, T lo, T 
     return (v < lo) ? lo : (hi < v) ? hi : v;
 }
 
+// counters of the direct geometry's items (gpk_geometry_items.cu)
+struct ItemCounters {
+    unsigned items, next;       // items made; items taken by the warps that ran out of their first ones
+    unsigned long long words;   // bitmap words asked for
+    unsigned no_bitmap, pad[3]; // tiles without bitmaps
+};
+
 // ---------------------------------------------------------------------------
 // per-step device scalars (one struct per grid, in device memory)
 // ---------------------------------------------------------------------------

@@ -8,25 +8,21 @@
 #endif
 
 // Takes `need` words of a pool of `pool` words; `at` becomes the first of
-// them.  False where they do not fit.  The counter moves only with a request
-// that fits, and never back: no word is given twice, whatever the order in
-// which requests of different sizes arrive.  (Adding first and subtracting
-// where the request did not fit gives words twice: a subtraction may follow
-// another block's successful addition.)  The loop repeats only where another
-// request was granted in between.
-//   Counter::load()               the words taken so far
-//   Counter::exchange(old, next)  writes next where the value is old; returns
-//                                 the value found
+// them.  False where they do not fit.  The counter never goes back, so no word
+// is given twice, whatever the order in which requests of different sizes
+// arrive.  (Taking an addition back where the request did not fit gives words
+// twice: the subtraction may follow another block's successful addition.)  A
+// request that does not fit adds nothing, unless another one came between its
+// reading and its addition: then the counter stays past the end.
+// One addition, not a compare-and-exchange: that one is granted once per round
+// trip to the L2 and per word of contention, 5.5 ms for the 7875 tiles of
+// 2000 x 2000 cells where this takes 0.2, and 1.4 ms of a 256^3 step.
+//   Counter::load()    the count, 64 bits wide (additions past the end never wrap it)
+//   Counter::add(v)    adds v; returns the count before
 template <class Counter>
 GPK_POOL_FN bool pool_take(Counter& c, unsigned need, unsigned pool, unsigned& at) {
-    unsigned old = c.load();
-    while (old <= pool && pool - old >= need) {
-        const unsigned found = c.exchange(old, old + need);
-        if (found == old) {
-            at = old;
-            return true;
-        }
-        old = found;
-    }
-    return false;
+    if (c.load() + need > pool) return false;
+    const unsigned long long old = c.add(need);
+    at = (unsigned)old;
+    return old + need <= pool;
 }

@@ -111,7 +111,7 @@ struct MaskJob {
     // `gate` (may be null): when it points to zero the launch does nothing
     // (device-side skip of a stage inside a captured step)
     const unsigned long long* gate = nullptr;
-    unsigned* item_counters = nullptr;  // the geometry's item counters, cleared
+    ItemCounters* item_counters = nullptr;  // the geometry's item counters, cleared
     void* zero[7] = {};                 // fields set to zero everywhere
     int nzero = 0, rsz = 4;
     int32_t* copy = nullptr;            // phi copied here (phi_comp before a remap pass) ...
@@ -148,8 +148,7 @@ __global__ void __launch_bounds__(MASK_TPB) k_mask_list(Dims D, const int32_t* _
             s->n_cand = 0; s->n_prop = 0; s->waves = 0; s->n_near = 0; s->vmax = 0.0;
         }
         if (job.clear_waves) s->waves = 0;
-        if (job.item_counters)
-            for (int k = 0; k < 4; ++k) job.item_counters[k] = 0u;
+        if (job.item_counters) *job.item_counters = ItemCounters{};
     }
     constexpr int TILE = MASK_TPB * IPT;
     constexpr int G = W4 ? 4 : 1, ROUNDS = IPT / G, CHUNKS = ROUNDS * MASK_WARPS;

@@ -3,7 +3,8 @@
 gpk_pool.h is compiled for the host and its requests are made from several
 threads at once, of very different sizes and past the end of the pool.  The
 given ranges lie in the pool and do not overlap, and a request is refused only
-where it does not fit behind what was given.
+where it does not fit behind what was asked for (with one thread: behind what
+was given).
 """
 import os
 import subprocess
@@ -23,20 +24,17 @@ SOURCE = r"""
 #include <vector>
 #include "gpk_pool.h"
 
-static std::atomic<unsigned> g_taken;
+static std::atomic<unsigned long long> g_taken;
 static std::atomic<int> g_go;
 
 struct Counter {
-    unsigned load() { return g_taken.load(); }
-    unsigned exchange(unsigned old, unsigned next) {
-        g_taken.compare_exchange_strong(old, next);
-        return old;
-    }
+    unsigned long long load() { return g_taken.load(); }
+    unsigned long long add(unsigned v) { return g_taken.fetch_add(v); }
 };
 
 int main(int argc, char** argv) {
     const unsigned pool = std::atoi(argv[1]);
-    const int rounds = std::atoi(argv[2]), T = 8, per = 40;
+    const int rounds = std::atoi(argv[2]), T = std::atoi(argv[3]), per = 320 / T;
     for (int r = 0; r < rounds; ++r) {
         g_taken = 0;
         g_go = 0;
@@ -66,9 +64,10 @@ int main(int argc, char** argv) {
             end = a.first + a.second;
         }
         if (end > pool) { std::printf("round %d: past the end\n", r); return 1; }
+        const unsigned long long behind = T == 1 ? end : g_taken.load();
         for (auto& q : refused)
             for (unsigned n : q)
-                if (pool - end >= n) { std::printf("round %d: %u refused with %u left\n", r, n, pool - end); return 1; }
+                if (behind + n <= pool) { std::printf("round %d: %u refused with %u left\n", r, n, pool - end); return 1; }
     }
     std::printf("ok\n");
     return 0;
@@ -76,11 +75,11 @@ int main(int argc, char** argv) {
 """
 
 
-@pytest.mark.parametrize("pool", [1, 1000, 3000, 100000])
-def test_no_word_is_given_twice(tmp_path, pool):
+@pytest.mark.parametrize("pool,threads", [(1, 8), (1000, 8), (3000, 8), (100000, 8), (1000, 1), (3000, 1)])
+def test_no_word_is_given_twice(tmp_path, pool, threads):
     src, exe = tmp_path / "pool.cpp", tmp_path / "pool"
     src.write_text(SOURCE)
     inc = os.path.join(ROOT, "gpk_b200", "csrc")
     subprocess.run(["g++", "-O2", "-std=c++17", "-pthread", "-I", inc, str(src), "-o", str(exe)], check=True)
-    r = subprocess.run([str(exe), str(pool), "300"], capture_output=True, text=True, timeout=120)
+    r = subprocess.run([str(exe), str(pool), "300", str(threads)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout
