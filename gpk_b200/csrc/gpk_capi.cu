@@ -367,24 +367,11 @@ extern "C" int gpk_grid_create(int Nz, int Ny, int Nx, double dx, const gpk_ther
     ALLOC(G->active, 4 * N);
     const size_t list_bytes = 16 + 8 * ((N + 2047) / 2048);
     ALLOC(G->list_state, list_bytes);
-    ALLOC(G->alpha_new_a, rb + 16);
-    ALLOC(G->cand, 4 * N);
-    ALLOC(G->cand_info, 16 * N);
     ALLOC(G->pmap, 4 * N);
     ALLOC(G->stamp, 4 * N);
     ALLOC(G->stamp_rev, 4 * N);
-    ALLOC(G->ff_stack, 4 * (5 * N + 64));  // flood-fill queues: cells + search ids
     ALLOC(G->near_list, 4 * (size_t)N);    // near-threshold cells of the last step
-    ALLOC(G->bgr_res, rb);
-    ALLOC(G->bgr_best, rb);
-    ALLOC(G->key_a, 8 * N);
-    ALLOC(G->key_b, 8 * N);
-    ALLOC(G->val_a, 4 * N);
-    ALLOC(G->val_b, 4 * N);
     ALLOC(G->upload_check, 2 * sizeof(unsigned));
-    ALLOC(G->exch, 16 * N);
-    ALLOC(G->ero_target, 4 * N);
-    ALLOC(G->ero_g, rb);
     ALLOC(G->scal, sizeof(StepScalars));
     {
         size_t b1 = 0, b2 = 0;
@@ -393,8 +380,33 @@ extern "C" int gpk_grid_create(int Nz, int Ny, int Nx, double dx, const gpk_ther
         cub::DeviceRadixSort::SortPairs(nullptr, b2, (const int32_t*)nullptr, (int32_t*)nullptr,
                                         (const unsigned long long*)nullptr, (unsigned long long*)nullptr, (int)N, 0, 32);
         G->cub_tmp_bytes = std::max(b1, b2) + 256;
-        ALLOC(G->cub_tmp, G->cub_tmp_bytes);
     }
+    rc = precision == GPK_PREC_F32 ? gpk_build_tables<float>(G) : gpk_build_tables<double>(G);
+    if (rc != GPK_OK) return fail(rc);
+    {
+        // the scratch's parts (see gpk_grid), each on a 256-byte boundary
+        const int R = precision == GPK_PREC_F32 ? ((HostKernels<float>*)G->host_kernels)->geom_radius
+                                                : ((HostKernels<double>*)G->host_kernels)->geom_radius;
+        struct Part { void** p; size_t bytes; };
+        const Part parts[] = {{(void**)&G->cand_info, 16 * N}, {(void**)&G->exch, 16 * N},
+                              {(void**)&G->key_a, 8 * N}, {(void**)&G->key_b, 8 * N},
+                              {(void**)&G->val_a, 4 * N}, {(void**)&G->val_b, 4 * N},
+                              {(void**)&G->ff_stack, 4 * (5 * N + 64)}, {(void**)&G->cand, 4 * N},
+                              {&G->alpha_new_a, rb + 16}, {&G->bgr_res, rb}, {&G->bgr_best, rb},
+                              {(void**)&G->ero_target, 4 * N}, {&G->ero_g, rb}, {&G->cub_tmp, G->cub_tmp_bytes}};
+        auto padded = [](size_t b) { return (b + 255) & ~(size_t)255; };
+        size_t bytes = 0;
+        for (const Part& q : parts) bytes += padded(q.bytes);
+        G->scratch_bytes = std::max(bytes, gpk_geometry_items_scratch(G, R));
+        ALLOC(G->scratch, G->scratch_bytes);
+        bytes = 0;
+        for (const Part& q : parts) {
+            *q.p = G->scratch + bytes;
+            bytes += padded(q.bytes);
+        }
+    }
+    rc = precision == GPK_PREC_F32 ? gpk_geometry_items_init<float>(G) : gpk_geometry_items_init<double>(G);
+    if (rc != GPK_OK) return fail(rc);
 #undef ALLOC
     if (cudaMallocHost((void**)&G->h_scal, sizeof(StepScalars)) != cudaSuccess) {
         gpk_set_error("cudaMallocHost failed");
@@ -404,8 +416,6 @@ extern "C" int gpk_grid_create(int Nz, int Ny, int Nx, double dx, const gpk_ther
     if (cudaMemsetAsync(G->scal, 0, sizeof(StepScalars), G->stream) != cudaSuccess ||
         cudaMemsetAsync(G->list_state, 0, list_bytes, G->stream) != cudaSuccess)
         return fail(GPK_ERR_CUDA);
-    rc = precision == GPK_PREC_F32 ? gpk_build_tables<float>(G) : gpk_build_tables<double>(G);
-    if (rc != GPK_OK) return fail(rc);
     rc = precision == GPK_PREC_F32 ? init_fields<float>(G) : init_fields<double>(G);
     if (rc != GPK_OK) return fail(rc);
     if ((rc = gpk_ensure_label_capacity(G, 64)) != GPK_OK) return fail(rc);
@@ -592,7 +602,6 @@ int gpk_grid_graph_prepare(gpk_grid* G, double dt, double dt_cap) {
     const std::vector<uint64_t> sig = graph_signature(G, dt, dt_cap);
     if (G->step_graph && sig == G->graph_sig) return GPK_OK;
     gpk_grid_graph_release(G);
-    GPK_TRY(G->precision == GPK_PREC_F64 ? gpk_geometry_items_init<double>(G) : gpk_geometry_items_init<float>(G));
     GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
     const uint64_t step0 = G->step_id, launches0 = G->launches;
     GPK_CUDA_TRY(cudaStreamBeginCapture(G->stream, cudaStreamCaptureModeThreadLocal));

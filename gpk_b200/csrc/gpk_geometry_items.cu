@@ -873,68 +873,62 @@ static bool for_radius(int R, F f) {
     }
 }
 
-// The packed tap table, the item arrays and the bitmap pool of a grid (kernel
-// radii 4..10), made when a grid first takes this geometry (and before a
-// capture, which allocates nothing).
+// item slots of a grid: its cells, and for every tile the padding of its last item
+static size_t item_slots(const Dims& D, int R) {
+    long long ntiles = 0;
+    for_radius(R, [&](auto r) {
+        constexpr int RR = decltype(r)::value;
+        auto tiles = [&](int tx, int ty, int tz) {
+            ntiles = (long long)((D.Nx + tx - 1) / tx) * ((D.Ny + ty - 1) / ty) * ((D.Nz + tz - 1) / tz);
+        };
+        // (the lowest 2-D tile: the most tiles)
+        if (D.is3d()) tiles(ItemTile<RR, true, 1>::TX, ItemTile<RR, true, 1>::TY, ItemTile<RR, true, 1>::TZ);
+        else tiles(ItemTile<RR, false, 4>::TX, ItemTile<RR, false, 4>::TY, 1);
+    });
+    return ((size_t)D.N + 64 * (size_t)ntiles + 3) & ~(size_t)3;
+}
+
+// Scratch that a grid's items and bitmaps need at the least (the padding of an
+// item reads the pool's first words)
+size_t gpk_geometry_items_scratch(const gpk_grid* G, int R) { return 12 * item_slots(G->d, R) + 4 * 4096; }
+
+// The packed tap table and the counters of a grid (kernel radii 4..10), and
+// where in its scratch the items and the bitmap pool lie: made with the grid,
+// so that no step allocates.  The scratch holds the crossing and remap records,
+// which nothing reads while the geometry runs.  (As an allocation of their own,
+// 28 bytes a cell and more, the items cost a grid's first step 1 to 120 ms,
+// and the 48 instances of a sweep 20 to 700.)
 template <typename real>
 int gpk_geometry_items_init(gpk_grid* G) {
-    if (G->item_counters || G->item_no_room) return GPK_OK;
     const HostKernels<real>* hk = (const HostKernels<real>*)G->host_kernels;
-    const int R = hk->geom_radius;
     const std::vector<real>& taps = hk->geom_table;
     std::vector<real> packed;
-    long long ntiles = 0;
-    double label_words = 0;  // words per cell that one label in every tile takes
-    const bool is3d = G->d.is3d();
     const Dims D = G->d;
-    if (!for_radius(R, [&](auto r) {
+    if (!for_radius(hk->geom_radius, [&](auto r) {
             constexpr int RR = decltype(r)::value;
-            auto tiles = [&](int tx, int ty, int tz) {
-                ntiles = std::max(ntiles, (long long)((D.Nx + tx - 1) / tx) * ((D.Ny + ty - 1) / ty) * ((D.Nz + tz - 1) / tz));
-            };
-            if (is3d) {
-                pack_table<real, RR, true>(taps, packed);
-                tiles(ItemTile<RR, true, 1>::TX, ItemTile<RR, true, 1>::TY, ItemTile<RR, true, 1>::TZ);
-                label_words = (double)ItemTile<RR, true, 1>::NROW / ItemTile<RR, true, 1>::NCELL;
-            } else {
-                pack_table<real, RR, false>(taps, packed);
-                tiles(ItemTile<RR, false, 4>::TX, ItemTile<RR, false, 4>::TY, 1);
-                label_words = (double)ItemTile<RR, false, 1>::NROW / ItemTile<RR, false, 1>::NCELL;
-            }
+            if (D.is3d()) pack_table<real, RR, true>(taps, packed);
+            else pack_table<real, RR, false>(taps, packed);
         }))
         return GPK_OK;
-    // words: 20 labels in every tile (0.38 words a cell and label at R = 8, 0.49
-    // at R = 9, 0.66 at R = 10): tiles of a polycrystal with grains of 1500 cells
-    // meet 9 to 11 on average.  Smaller grids get room for more labels per tile, and tiles that find
-    // the pool full compare labels instead (and are counted)
-    const size_t base_words = (size_t)(20 * label_words * (double)D.N);
-    const size_t want = is3d ? std::max(base_words, std::min((size_t)64 * D.N, (size_t)8 << 20))
-                             : std::max(base_words, std::min((size_t)16 * D.N, (size_t)1 << 20));
-    // (the padding of an item reads the pool's first words)
-    G->item_pool = (unsigned)std::max(std::min(want, (size_t)1 << 31), (size_t)4096);
-    // one allocation: counters, table, items, words
-    const size_t slots = ((size_t)D.N + 64 * (size_t)ntiles + 3) & ~(size_t)3;
+    const size_t slots = item_slots(D, hk->geom_radius);
     const size_t table = sizeof(real) * packed.size();
     unsigned char* base = nullptr;
-    const size_t head = sizeof(ItemCounters), fixed = head + table + 12 * slots;
-    // a full device: the smallest pool (most tiles compare labels), or no items
-    // at all (the per-cell kernel, which needs no memory of its own)
-    if (!gpk_alloc_optional(G, (void**)&base, fixed + 4 * (size_t)G->item_pool)) {
-        G->item_pool = 4096;
-        if (!gpk_alloc_optional(G, (void**)&base, fixed + 4 * (size_t)G->item_pool)) {
-            G->item_no_room = true;
-            return GPK_OK;
-        }
-    }
-    // (the interface mask of this step ran before there were counters to clear)
-    GPK_CUDA_TRY(cudaMemsetAsync(base, 0, head, G->stream));
+    constexpr size_t head = sizeof(ItemCounters);
+    static_assert(head % 16 == 0, "the table is copied in 16-byte units");
+    GPK_TRY(gpk_alloc(G, (void**)&base, head + table));
+    GPK_CUDA_TRY(cudaMemset(base, 0, head));
+    GPK_CUDA_TRY(cudaMemcpy(base + head, packed.data(), table, cudaMemcpyHostToDevice));
     G->d_geom_packed = base + head;
-    GPK_CUDA_TRY(cudaMemcpyAsync(G->d_geom_packed, packed.data(), table, cudaMemcpyHostToDevice, G->stream));
-    GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
-    G->item_word = (int32_t*)(base + head + table);
+    G->item_word = (int32_t*)G->scratch;
     G->item_cell = G->item_word + slots;
     G->item_support = (uint32_t*)(G->item_cell + slots);
     G->item_words = G->item_support + slots;
+    // words: what is left, 25 a cell (FP64: 29): 66 labels in every tile at R = 8,
+    // 50 at R = 9 and 38 at R = 10 (0.38, 0.49 and 0.66 words a cell and label;
+    // tiles of a polycrystal with grains of 1500 cells meet 9 to 11 on average).
+    // Tiles that find the pool full compare labels instead, and are counted
+    const size_t words = (G->scratch_bytes - 12 * slots) / 4;
+    G->item_pool = (unsigned)std::min(words, (size_t)1 << 31);
     G->item_counters = (ItemCounters*)base;
     return GPK_OK;
 }
@@ -942,11 +936,9 @@ template int gpk_geometry_items_init<float>(gpk_grid*);
 template int gpk_geometry_items_init<double>(gpk_grid*);
 
 // The direct geometry for kernel radii 4..10 (Gaussian radius 2..8); returns
-// -1 for other radii and where the device has no room for the items (the caller then uses the per-cell kernel).
+// -1 for other radii (the caller then uses the per-cell kernel).
 template <typename real>
 int gpk_geometry_items(gpk_grid* G, int R, real inv_dx, real inv_dx2, real dx, real kappa_limit) {
-    if (R < 4 || R > 10) return -1;
-    GPK_TRY(gpk_geometry_items_init<real>(G));
     if (!G->item_counters) return -1;
     SumArgs<real> a{};
     a.D = G->d;

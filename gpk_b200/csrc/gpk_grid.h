@@ -70,21 +70,26 @@ struct gpk_grid {
     int have_solid_old = 0;
     int32_t* active = nullptr;             // sorted interface cells
     void* list_state = nullptr;            // ordered compactions: tickets and tile counts
-    void* alpha_new_a = nullptr;           // per active position
-    int32_t* cand = nullptr;               // candidate active positions
-    int32_t* cand_info = nullptr;          // packed per-candidate wave state
+    // one block for all that is marked (s) below: it holds nothing from one step
+    // to the next, and the geometry keeps its own work there before it is used
+    unsigned char* scratch = nullptr; size_t scratch_bytes = 0;
+    void* alpha_new_a = nullptr;           // (s) per active position
+    int32_t* cand = nullptr;               // (s) candidate active positions
+    int32_t* cand_info = nullptr;          // (s) packed per-candidate wave state
     int32_t* pmap = nullptr;               // pending map (cell -> item) or -1
     int32_t* minF = nullptr; int32_t* minL = nullptr;
-    uint32_t* stamp = nullptr; uint32_t* stamp_rev = nullptr; int32_t* ff_stack = nullptr;
-    // remap
+    uint32_t* stamp = nullptr; uint32_t* stamp_rev = nullptr;
+    int32_t* ff_stack = nullptr;           // (s) flood-fill queues: cells + search ids
+    // remap (s)
     void* bgr_res = nullptr; void* bgr_best = nullptr;   // per active position (real)
     unsigned long long* key_a = nullptr; unsigned long long* key_b = nullptr;
     int32_t* val_a = nullptr; int32_t* val_b = nullptr;
-    unsigned* upload_check = nullptr;      // label range check of an upload
     int32_t* exch = nullptr;               // exchange slots: a, b, low, high, state
     void* cub_tmp = nullptr; size_t cub_tmp_bytes = 0;
     // extinction
-    uint8_t* unres = nullptr; int32_t* ero_target = nullptr; void* ero_g = nullptr;
+    uint8_t* unres = nullptr;
+    int32_t* ero_target = nullptr; void* ero_g = nullptr;  // (s)
+    unsigned* upload_check = nullptr;      // label range check of an upload
     // separable geometry: label by label over the whole grid, or per label box
     // (gpk_separable.cu: values of the passes; label index and regions)
     void* sep_I = nullptr; void* sep_t1 = nullptr; void* sep_t2 = nullptr; void* sep_S = nullptr;
@@ -101,13 +106,13 @@ struct gpk_grid {
     // remap screening: weight sums of the 128 patterns of a 7-tap row, for the
     // ten distinct dy^2 + dz^2 of a 7 x 7 row block (radius 3 only)
     double* d_remap_rtab = nullptr;
-    // direct geometry (gpk_geometry_items.cu): packed tap table, items of 64
-    // interface cells, bitmap pool
+    // direct geometry (gpk_geometry_items.cu): packed tap table and counters
+    // (null: radius without this form), items of 64 interface cells and bitmap
+    // pool in the scratch
     void* d_geom_packed = nullptr;
     int32_t* item_word = nullptr; int32_t* item_cell = nullptr;
     uint32_t* item_support = nullptr; uint32_t* item_words = nullptr;
     unsigned item_pool = 0;
-    bool item_no_room = false;
     gpk_dev::ItemCounters* item_counters = nullptr;
     gpk_dev::StepScalars* scal = nullptr;  // device scalars
     gpk_dev::StepScalars* h_scal = nullptr;  // pinned host mirror
@@ -164,6 +169,7 @@ template <typename real> int gpk_phase_volume_impl(gpk_grid* G, int32_t label, d
 template <typename real>
 int gpk_geometry_items(gpk_grid* G, int R, real inv_dx, real inv_dx2, real dx, real kappa_limit);
 template <typename real> int gpk_geometry_items_init(gpk_grid* G);
+size_t gpk_geometry_items_scratch(const gpk_grid* G, int R);
 template <typename real> int gpk_geometry_separable(gpk_grid* G, real dx, real kappa_limit);
 // FP64 separable tiles (throughput geometry); -1 when they do not apply
 int gpk_geometry_sep_tiles(gpk_grid* G, int R, const double* gauss, int gauss_radius, double dx,
