@@ -75,17 +75,6 @@ int gpk_alloc(gpk_grid* G, void** p, size_t bytes) {
     return GPK_OK;
 }
 
-bool gpk_alloc_optional(gpk_grid* G, void** p, size_t bytes) {
-    if (cudaMalloc(p, bytes) != cudaSuccess) {
-        cudaGetLastError();  // not the error of the launches that follow
-        *p = nullptr;
-        return false;
-    }
-    G->allocations.push_back(*p);
-    G->device_bytes += bytes;
-    return true;
-}
-
 static void gpk_free(gpk_grid* G, void* p) {
     if (!p) return;
     auto it = std::find(G->allocations.begin(), G->allocations.end(), p);
@@ -406,6 +395,8 @@ extern "C" int gpk_grid_create(int Nz, int Ny, int Nx, double dx, const gpk_ther
         }
     }
     rc = precision == GPK_PREC_F32 ? gpk_geometry_items_init<float>(G) : gpk_geometry_items_init<double>(G);
+    if (rc != GPK_OK) return fail(rc);
+    rc = precision == GPK_PREC_F32 ? gpk_geometry_separable_init<float>(G) : gpk_geometry_separable_init<double>(G);
     if (rc != GPK_OK) return fail(rc);
 #undef ALLOC
     if (cudaMallocHost((void**)&G->h_scal, sizeof(StepScalars)) != cudaSuccess) {

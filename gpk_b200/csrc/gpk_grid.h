@@ -90,11 +90,8 @@ struct gpk_grid {
     uint8_t* unres = nullptr;
     int32_t* ero_target = nullptr; void* ero_g = nullptr;  // (s)
     unsigned* upload_check = nullptr;      // label range check of an upload
-    // separable geometry: label by label over the whole grid, or per label box
-    // (gpk_separable.cu: values of the passes; label index and regions)
-    void* sep_I = nullptr; void* sep_t1 = nullptr; void* sep_t2 = nullptr; void* sep_S = nullptr;
-    size_t sep_cap[3] = {};
-    void* sep_box = nullptr; void* sep_table = nullptr; size_t sep_table_bytes = 0;
+    // separable geometry (gpk_separable.cu): sums of the runs of taps (null: whole-grid passes)
+    void* d_sep_runs = nullptr;
     // labels
     int32_t* count = nullptr;              // cells per label
     int32_t* count0 = nullptr;             // cells per label when the crossing sweep started
@@ -171,6 +168,7 @@ int gpk_geometry_items(gpk_grid* G, int R, real inv_dx, real inv_dx2, real dx, r
 template <typename real> int gpk_geometry_items_init(gpk_grid* G);
 size_t gpk_geometry_items_scratch(const gpk_grid* G, int R);
 template <typename real> int gpk_geometry_separable(gpk_grid* G, real dx, real kappa_limit);
+template <typename real> int gpk_geometry_separable_init(gpk_grid* G);
 // FP64 separable tiles (throughput geometry); -1 when they do not apply
 int gpk_geometry_sep_tiles(gpk_grid* G, int R, const double* gauss, int gauss_radius, double dx,
                            double kappa_limit);
@@ -180,8 +178,6 @@ template <typename real> int gpk_projection_tiled(gpk_grid* G, int radius);
 int gpk_recount_labels(gpk_grid* G);
 int gpk_topology_simple_move_impl(gpk_grid* G, int cell, int32_t new_label, int* result);
 int gpk_alloc(gpk_grid* G, void** p, size_t bytes);
-// memory the grid can do without: false (and no error) when there is none
-bool gpk_alloc_optional(gpk_grid* G, void** p, size_t bytes);
 int gpk_ensure_label_capacity(gpk_grid* G, int cap);
 int gpk_sync_scalars(gpk_grid* G);
 template <typename real> int gpk_remap_pass_graph(gpk_grid* G, const unsigned long long* gate);

@@ -265,6 +265,28 @@ static void arc_of(const uint8_t* m, int n, int& start, int& len) {
 
 using namespace gpk_dev;
 
+// The sums of the runs of taps (radii to 31), made with the grid: the first step
+// allocates nothing.
+template <typename real>
+int gpk_geometry_separable_init(gpk_grid* G) {
+    const HostKernels<real>* hk = (const HostKernels<real>*)G->host_kernels;
+    const int R = hk->gauss_radius, K = 2 * R + 1;
+    if (!hk->global_separable || R > SEP_MAX_R) return GPK_OK;
+    std::vector<real> runs((size_t)K * (K + 1), (real)0);
+    for (int s = 0; s < K; ++s) {
+        real acc = (real)0;
+        for (int l = 1; s + l <= K; ++l) {
+            acc += hk->gauss_w[s + l - 1];
+            runs[(size_t)s * (K + 1) + l] = acc;
+        }
+    }
+    GPK_TRY(gpk_alloc(G, &G->d_sep_runs, sizeof(real) * runs.size()));
+    GPK_CUDA_TRY(cudaMemcpy(G->d_sep_runs, runs.data(), sizeof(real) * runs.size(), cudaMemcpyHostToDevice));
+    return GPK_OK;
+}
+template int gpk_geometry_separable_init<float>(gpk_grid*);
+template int gpk_geometry_separable_init<double>(gpk_grid*);
+
 // Smoothing and differences of every interface label into nx, ny, nz, kappa
 // (zero on entry); -1 where this form does not apply (the caller then smooths
 // label by label over the whole grid).
@@ -272,10 +294,10 @@ template <typename real>
 int gpk_geometry_separable(gpk_grid* G, real dx, real kappa_limit) {
     HostKernels<real>* hk = (HostKernels<real>*)G->host_kernels;
     const Dims D = G->d;
-    const int R = hk->gauss_radius, K = 2 * R + 1, span = D.Nx + D.Ny + D.Nz;
+    const int R = hk->gauss_radius, span = D.Nx + D.Ny + D.Nz;
     // (the marks lie in the proposal keys' buffer, free until the remap)
     const size_t mark_bytes = (size_t)G->label_cap * span;
-    if (R > SEP_MAX_R || !D.is3d() || D.Nx < 2 || D.Ny < 2 || mark_bytes > 8 * (size_t)D.N) return -1;
+    if (!G->d_sep_runs || !D.is3d() || D.Nx < 2 || D.Ny < 2 || mark_bytes > 8 * (size_t)D.N) return -1;
     uint8_t* marks = (uint8_t*)G->key_a;
     GPK_CUDA_TRY(cudaMemsetAsync(marks, 0, mark_bytes, G->stream));
     k_sep_marks<<<G->num_sms * 8, 256, 0, G->stream>>>(D, G->active, &G->scal->n_active, G->phi, marks);
@@ -310,43 +332,20 @@ int gpk_geometry_separable(gpk_grid* G, real dx, real kappa_limit) {
         regions.push_back(g);
     }
     if (regions.empty()) return GPK_OK;
-    // workspace (kept): values of the three passes, taps' run sums, label index and regions
-    // (many labels' boxes at once; where the device has no room for that, one
-    // label's at least, which is less than the whole-grid passes take)
-    if (!G->sep_box) {
-        const size_t extra = (size_t)K * (K + 1);
-        void* p = nullptr;
-        if (gpk_alloc_optional(G, &p, sizeof(real) * (17 * (size_t)D.N + extra))) {
-            G->sep_cap[0] = 8 * (size_t)D.N; G->sep_cap[1] = 5 * (size_t)D.N; G->sep_cap[2] = 4 * (size_t)D.N;
-        } else {
-            GPK_TRY(gpk_alloc(G, &p, sizeof(real) * (3 * (size_t)D.N + extra)));
-            G->sep_cap[0] = G->sep_cap[1] = G->sep_cap[2] = (size_t)D.N;
-        }
-        G->sep_box = p;
-        std::vector<real> runs((size_t)K * (K + 1), (real)0);
-        for (int s = 0; s < K; ++s) {
-            real acc = (real)0;
-            for (int l = 1; s + l <= K; ++l) {
-                acc += hk->gauss_w[s + l - 1];
-                runs[(size_t)s * (K + 1) + l] = acc;
-            }
-        }
-        GPK_CUDA_TRY(cudaMemcpyAsync((real*)p + G->sep_cap[0] + G->sep_cap[1] + G->sep_cap[2], runs.data(), sizeof(real) * runs.size(),
-                                     cudaMemcpyHostToDevice, G->stream));
-        GPK_CUDA_TRY(cudaStreamSynchronize(G->stream));
-    }
-    const size_t cap1 = G->sep_cap[0], cap2 = G->sep_cap[1], cap3 = G->sep_cap[2];
-    real* t1 = (real*)G->sep_box;
+    // in the grid's scratch (the marks have been read): label index and regions,
+    // then the values of the three passes
+    const size_t head = ((sizeof(int32_t) * (size_t)G->label_cap + 15) & ~(size_t)15);
+    const size_t table = head + sizeof(SepRegion) * regions.size();
+    const size_t values = (table + 255) & ~(size_t)255;
+    if (values + 3 * sizeof(real) * (size_t)D.N > G->scratch_bytes) return -1;
+    const size_t room = (G->scratch_bytes - values) / sizeof(real);
+    // (a region needs at most N values of each pass; the x-smoothed box is the largest, by its halo)
+    const size_t cap1 = (size_t)D.N + (room - 3 * (size_t)D.N) / 2;
+    const size_t cap2 = (size_t)D.N + (room - 3 * (size_t)D.N) / 4, cap3 = cap2;
+    real* t1 = (real*)(G->scratch + values);
     real* t2 = t1 + cap1;
     real* s = t2 + cap2;
-    const real* runs = s + cap3;
-    const size_t table = ((sizeof(int32_t) * (size_t)G->label_cap + 15) & ~(size_t)15) + sizeof(SepRegion) * regions.size();
-    if (table > G->sep_table_bytes) {
-        // (an outgrown table stays allocated until the grid goes: it may still be read)
-        const size_t room = table + table / 2;
-        GPK_TRY(gpk_alloc(G, &G->sep_table, room));
-        G->sep_table_bytes = room;
-    }
+    const real* runs = (const real*)G->d_sep_runs;
     std::vector<unsigned char> host(table);
     for (size_t r0 = 0; r0 < regions.size();) {
         size_t n = 0, u1 = 0, u2 = 0, u3 = 0;
@@ -365,12 +364,11 @@ int gpk_geometry_separable(gpk_grid* G, real dx, real kappa_limit) {
         int32_t* index = (int32_t*)host.data();
         std::fill(index, index + G->label_cap, -1);
         for (size_t k = 0; k < n; ++k) index[regions[r0 + k].label] = (int32_t)k;
-        const size_t head = (sizeof(int32_t) * (size_t)G->label_cap + 15) & ~(size_t)15;
         std::copy((const unsigned char*)&regions[r0], (const unsigned char*)(&regions[r0] + n), host.data() + head);
         // (pageable memory: staged when the call returns, so `host` may be filled again)
-        GPK_CUDA_TRY(cudaMemcpyAsync(G->sep_table, host.data(), head + sizeof(SepRegion) * n, cudaMemcpyHostToDevice,
+        GPK_CUDA_TRY(cudaMemcpyAsync(G->scratch, host.data(), head + sizeof(SepRegion) * n, cudaMemcpyHostToDevice,
                                      G->stream));
-        const SepRegion* dr = (const SepRegion*)((unsigned char*)G->sep_table + head);
+        const SepRegion* dr = (const SepRegion*)(G->scratch + head);
         const int words = (max_x + 2 * R + 31) / 32 + 1;
         auto blocks = [&](long long work) { return (unsigned)std::max(1LL, std::min(work, 4096LL)); };
         const size_t smem = sizeof(uint32_t) * 8 * (size_t)(words + 2);
@@ -382,7 +380,7 @@ int gpk_geometry_separable(gpk_grid* G, real dx, real kappa_limit) {
         k_sep_box_line<real, 2><<<dim3(blocks((max_z + 255) / 256), (unsigned)n), 256, 0, G->stream>>>(
             D, dr, R, (const real*)G->d_gauss, t2, s);
         k_sep_box_eval<real><<<G->num_sms * 8, 256, 0, G->stream>>>(
-            D, G->active, &G->scal->n_active, G->phi, (const int32_t*)G->sep_table, dr, s, dx, kappa_limit,
+            D, G->active, &G->scal->n_active, G->phi, (const int32_t*)G->scratch, dr, s, dx, kappa_limit,
             (real*)G->f[GPK_FIELD_NX], (real*)G->f[GPK_FIELD_NY], (real*)G->f[GPK_FIELD_NZ],
             (real*)G->f[GPK_FIELD_KAPPA]);
         G->launches += 4;

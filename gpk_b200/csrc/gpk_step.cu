@@ -1693,12 +1693,9 @@ static int geometry(gpk_grid* G) {
     if (box != GPK_OK && box != -1) return box;
     if (box == -1) {
         // (kernels of a radius above 31 cells, more labels than there is room for their boxes' marks)
-        if (!G->sep_S) {
-            GPK_TRY(gpk_alloc(G, &G->sep_I, nb));
-            GPK_TRY(gpk_alloc(G, &G->sep_t1, nb));
-            GPK_TRY(gpk_alloc(G, &G->sep_t2, nb));
-            GPK_TRY(gpk_alloc(G, &G->sep_S, nb));
-        }
+        const size_t pad = (nb + 255) & ~(size_t)255;
+        real *I = (real*)G->scratch, *t1 = (real*)(G->scratch + pad), *t2 = (real*)(G->scratch + 2 * pad),
+             *S = (real*)(G->scratch + 3 * pad);
         uint8_t* present = G->unres;  // label-indexed scratch
         GPK_CUDA_TRY(cudaMemsetAsync(present, 0, G->label_cap, G->stream));
         k_label_flags<<<grid_for(G, D.N), 256, 0, G->stream>>>(D.N, G->phi, G->mask, present, G->label_cap);
@@ -1709,12 +1706,11 @@ static int geometry(gpk_grid* G) {
         for (int p = 0; p < G->label_cap; ++p) {
             if (!hp[p]) continue;
             cudaError_t ce = cudaSuccess;
-            const int nl = sep_gauss3<real>(D, nullptr, G->phi, p, (real*)G->sep_t1, (real*)G->sep_t2,
-                                            (real*)G->sep_S, (real*)G->sep_I, (const real*)G->d_gauss,
+            const int nl = sep_gauss3<real>(D, nullptr, G->phi, p, t1, t2, S, I, (const real*)G->d_gauss,
                                             hk->gauss_radius, gN, G->stream, &ce);
             GPK_CUDA_TRY(ce);
             k_separable_eval<real><<<gN, 256, 0, G->stream>>>(D, G->active, &G->scal->n_active, G->phi, p,
-                                                              (const real*)G->sep_S, dx, kappa_limit, nx, ny, nz, kp);
+                                                              S, dx, kappa_limit, nx, ny, nz, kp);
             G->launches += nl + 1;
         }
         G->launches++;

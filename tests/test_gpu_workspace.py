@@ -1,11 +1,11 @@
 """The geometry's workspace comes with the grid: no step, geometry call or
-capture of any kernel kind adds device memory, and what the geometry leaves in
+capture of any kernel kind or kernel width adds device memory, and what the geometry leaves in
 the shared scratch changes no later step.
 """
 import numpy as np
 import pytest
 
-from gpk_b200 import GPKGrid, sweep, thermo
+from gpk_b200 import GPKGrid, sweep, thermo, voronoi
 
 pytestmark = pytest.mark.gpu
 KINDS = ("tiled", "per_cell", "tiled_batched", "tiled_exact_scores")
@@ -26,6 +26,25 @@ def test_no_memory_at_the_first_step(shape, precision, per_cell):
         g.step_n(2)
         assert g.device_bytes() == held, kind
         g.close()
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("sigma,labels", [(5.0, 12), (9.0, 12), (5.0, 20000)])  # boxes; radius 32 and many labels: whole grid
+def test_no_memory_at_the_first_separable_step(sigma, labels, precision):
+    shape = (40, 44, 48)
+    g = GPKGrid(*shape, 1.0, thermo.isotropic(1.0, 1.0), 0.0, sigma, precision=precision)
+    # bytes a cell, and twelve products for every tap of the direct form's table
+    cell, real = (200, 4) if precision == "f32" else (273, 8)
+    taps = (2 * (int(np.ceil(3.5 * sigma)) + 2) + 1) ** 3
+    assert g.device_bytes() < cell * np.prod(shape) + 12 * real * taps + (2 << 20)
+    phi = voronoi(*shape, 12, 3)[0]
+    g.set("phi", np.where(phi == 12, labels, phi).astype(np.int32))
+    g.set("alpha", 0.3)
+    held = g.device_bytes()
+    g.geometry()
+    g.step_n(2)
+    assert g.device_bytes() == held
+    g.close()
 
 
 def test_no_memory_at_a_capture():
