@@ -1710,9 +1710,11 @@ int gpk_crossings(gpk_grid* G, int m) {
     if (m == 0) return GPK_OK;
     const int B = 256;
     int8_t* cres = (int8_t*)G->val_a;  // candidate results, scratch until the remap
-    k_cross_setup<<<(m + B - 1) / B, B, 0, G->stream>>>(G->active, G->cand, m, G->phi, G->phi_comp,
-                                                        (int4*)G->cand_info, G->pmap, cres, G->n_old, G->count, G->count0,
-                                                        G->label_cap, G->scal);
+    // a thread per candidate, and enough of them for the label counts: a few
+    // candidates' blocks alone took 61 ms a step for 512^2 with ids up to 40 M
+    const int setup = std::max((m + B - 1) / B, std::min((G->label_cap + 4 * B - 1) / (4 * B), 8 * G->num_sms));
+    k_cross_setup<<<setup, B, 0, G->stream>>>(G->active, G->cand, m, G->phi, G->phi_comp, (int4*)G->cand_info, G->pmap,
+                                              cres, G->n_old, G->count, G->count0, G->label_cap, G->scal);
     G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     CrossArgs a;
