@@ -1896,7 +1896,7 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
     U* vbits = (U*)&G->scal->vmax;
     k_vmax<real><<<ga, 256, 0, G->stream>>>(G->active, &G->scal->n_active, (const real*)G->f[GPK_FIELD_VN], vbits,
                                             G->scal, (real)G->dx, (real)G->D, D.is3d() ? 1 : 0, dt_req, dt_cap);
-    G->launches += 4;
+    G->launches += prc == -1 ? 3 : 2;  // (the tiled projection counts itself)
     GPK_TRY(gpk_stage_end(G, GPK_STAGE_PROJECTION));
     GPK_TRY(gpk_stage_begin(G, GPK_STAGE_ALPHA));
     if (th.solute_rejection) {
@@ -1916,7 +1916,7 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
         (const real*)G->f[GPK_FIELD_T], (real*)G->f[GPK_FIELD_ALPHA], (real*)G->alpha_new_a, G->cand, G->scal,
         (ListState*)G->list_state, (real)G->dx, th.stochastic, (real)th.M0, (real)th.kB, (real)th.noise_scale,
         G->step_id, (real)G->near_tol, G->near_list, D.N);
-    G->launches += 4;
+    G->launches++;
     GPK_CUDA_TRY(cudaGetLastError());
     GPK_TRY(gpk_stage_end(G, GPK_STAGE_ALPHA));
     GPK_TRY(gpk_sync_scalars(G));
@@ -2151,7 +2151,7 @@ int gpk_step_graph_body(gpk_grid* G, double dt_req, double dt_cap) {
     U* vbits = (U*)&G->scal->vmax;
     k_vmax<real><<<ga, 256, 0, G->stream>>>(G->active, &G->scal->n_active, (const real*)G->f[GPK_FIELD_VN], vbits,
                                             G->scal, (real)G->dx, (real)G->D, D.is3d() ? 1 : 0, dt_req, dt_cap);
-    G->launches += 4;
+    G->launches += prc == -1 ? 3 : 2;
     if (th.solute_rejection) {
         if (!G->solid_old) {
             gpk_set_error("captured step: solute buffers are made by a first ordinary step");
@@ -2172,7 +2172,7 @@ int gpk_step_graph_body(gpk_grid* G, double dt_req, double dt_cap) {
         G->active, G->cand, -1, G->phi, G->phi_comp, (real*)G->f[GPK_FIELD_G], (const real*)G->f[GPK_FIELD_G_COMP],
         (real*)G->f[GPK_FIELD_ALPHA], (real*)G->f[GPK_FIELD_RHO], G->count, G->scal, th.dislocation_enabled,
         (real)th.rho_rex);
-    G->launches += 5;
+    G->launches += 2;
     GPK_CUDA_TRY(cudaGetLastError());
     // balanced remap under the accepted-crossings gate; a second 3-D pass
     // under the first pass's exchanges

@@ -1764,6 +1764,7 @@ int gpk_remap_pass(gpk_grid* G, const unsigned long long* gate) {
         k_bgr_scores<real><<<grid, B, 0, G->stream>>>(D, G->active, &G->scal->n_active, G->phi, G->phi_comp,
                                                       (real*)G->bgr_res, (real*)G->bgr_best, G->d_remap_w,
                                                       hk->remap_radius);
+        G->launches++;
     } else if (rc != GPK_OK) {
         return rc;
     }

@@ -191,7 +191,9 @@ int gpk_grid_topology_simple_move(gpk_grid* grid, int cell, int32_t new_label,
  * Not counted: the 16 MiB static array of gpk_gaussian_filter_3d_noalloc,
  * resident on every GPU that loads the library.                           */
 int gpk_grid_device_bytes(gpk_grid* grid, size_t* out);
-/* Cumulative kernel-launch count issued by this grid (instrumentation).   */
+/* Launches of this library's own kernels issued by this grid, those of
+ * captured steps among them (instrumentation; radix sorts, copies and
+ * memsets are not counted).                                                */
 int gpk_grid_launch_count(gpk_grid* grid, uint64_t* out);
 
 /* gaussian_filter_3d (src/gpk_gaussian.cpp:9-72 of the reference): periodic
