@@ -67,6 +67,7 @@ int gpk_alloc(gpk_grid* G, void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
         gpk_set_error("cudaMalloc of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e));
+        cudaGetLastError();  // not the error of the launches that follow
         *p = nullptr;
         return GPK_ERR_OUT_OF_MEMORY;
     }

@@ -1730,6 +1730,26 @@ static ThermoDev make_thermo_dev(const gpk_thermo_desc& t) {
     return TD;
 }
 
+// The buffers a step's model needs beside the grid's own, made before the step
+// launches anything: a step that finds no memory leaves the labels, the fields
+// and the time as they were.
+template <typename real>
+static int step_buffers(gpk_grid* G) {
+    const size_t rb = G->rsz * (size_t)G->d.N;
+    auto need = [&](void** p, size_t bytes) { return *p ? (int)GPK_OK : gpk_alloc(G, p, bytes); };
+    if (elastic_proxy<real>(G)) {
+        GPK_TRY(need(&G->eps_star, rb));
+        GPK_TRY(need(&G->eps_smooth, rb));
+        GPK_TRY(need(&G->eps_tmp, rb));
+    }
+    if (G->th.solute_rejection) {
+        GPK_TRY(need(&G->solid_old, rb));
+        GPK_TRY(need(&G->s_new, rb));
+        GPK_TRY(need((void**)&G->grew, G->d.N));
+    }
+    return GPK_OK;
+}
+
 template <typename real>
 static int elastic(gpk_grid* G) {
     const gpk_thermo_desc& th = G->th;
@@ -1737,11 +1757,6 @@ static int elastic(gpk_grid* G) {
     real* E = (real*)G->f[GPK_FIELD_E_EL];
     // E_el as the caller supplied it, or zero (the step's first mask launch)
     if (!elastic_proxy<real>(G)) return GPK_OK;
-    if (!G->eps_star) {
-        GPK_TRY(gpk_alloc(G, &G->eps_star, G->rsz * D.N));
-        GPK_TRY(gpk_alloc(G, &G->eps_smooth, G->rsz * D.N));
-        GPK_TRY(gpk_alloc(G, &G->eps_tmp, G->rsz * D.N));
-    }
     const int gN = grid_for(G, D.N);
     const ThermoDev TD = make_thermo_dev(th);
     k_elastic_init<real><<<gN, 256, 0, G->stream>>>(D.N, TD, (const real*)G->f[GPK_FIELD_C], (const real*)G->f[GPK_FIELD_G],
@@ -1855,6 +1870,7 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
     HostKernels<real>* hk = (HostKernels<real>*)G->host_kernels;
     const Dims D = G->d;
     const gpk_thermo_desc& th = G->th;
+    GPK_TRY(step_buffers<real>(G));
     // grid-stride launches over at most N items
     const int ga = grid_for(G, D.N);
     // flood-fill stamps: restart before the 32-bit cursor can wrap
@@ -1900,11 +1916,6 @@ int gpk_step_impl(gpk_grid* G, double dt_req, double dt_cap) {
     GPK_TRY(gpk_stage_end(G, GPK_STAGE_PROJECTION));
     GPK_TRY(gpk_stage_begin(G, GPK_STAGE_ALPHA));
     if (th.solute_rejection) {
-        if (!G->solid_old) {
-            GPK_TRY(gpk_alloc(G, &G->solid_old, G->rsz * D.N));
-            GPK_TRY(gpk_alloc(G, &G->s_new, G->rsz * D.N));
-            GPK_TRY(gpk_alloc(G, (void**)&G->grew, D.N));
-        }
         k_solid_fraction<real><<<grid_for(G, D.N), 256, 0, G->stream>>>(D.N, G->phi, (const real*)G->f[GPK_FIELD_ALPHA],
                                                                          (real*)G->solid_old);
         G->have_solid_old = 1;
@@ -2128,6 +2139,10 @@ int gpk_step_graph_body(gpk_grid* G, double dt_req, double dt_cap) {
     const gpk_thermo_desc& th = G->th;
     // grid-stride launches over at most N items, sized for the grid's cells
     const int ga = (int)std::max(1LL, std::min((long long)G->num_sms * 8, ((long long)D.N + 255) / 256));
+    if (elastic_proxy<real>(G) && !(G->eps_star && G->eps_smooth && G->eps_tmp)) {
+        gpk_set_error("captured step: elastic buffers are made by a first ordinary step");
+        return GPK_ERR_INVALID_ARGUMENT;
+    }
     GPK_TRY(launch_mask(G, step_job<real>(G)));
     GPK_TRY(geometry<real>(G));
     GPK_TRY(elastic<real>(G));
@@ -2153,7 +2168,7 @@ int gpk_step_graph_body(gpk_grid* G, double dt_req, double dt_cap) {
                                             G->scal, (real)G->dx, (real)G->D, D.is3d() ? 1 : 0, dt_req, dt_cap);
     G->launches += prc == -1 ? 3 : 2;
     if (th.solute_rejection) {
-        if (!G->solid_old) {
+        if (!(G->solid_old && G->s_new && G->grew)) {
             gpk_set_error("captured step: solute buffers are made by a first ordinary step");
             return GPK_ERR_INVALID_ARGUMENT;
         }
