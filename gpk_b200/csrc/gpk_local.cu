@@ -962,8 +962,8 @@ static int launch_projection_bits(gpk_grid* G) {
     constexpr size_t smem = sizeof(typename ProjStage<real, R>::T) * S::NH +
                             4 * (size_t)(S::NL * S::NROWP + (S::NL * S::NROWP & 1)) +
                             (R > 3 ? sizeof(double) * (S::R2MAX + 1) : 0);
-    // (8 KB: the static lists)
-    if (smem + 8 * 1024 > 227 * 1024) return -1;
+    // at most 192 KB (FP64 at R = 9) and 8 KB of static lists
+    static_assert(smem + 8 * 1024 <= 227 * 1024, "halo and bitmaps of a tile in shared memory");
     // set once per process (thread-safe initialisation of a function-local static)
     static const cudaError_t attr_rc = cudaFuncSetAttribute(
         k_projection_bits<real, IS3D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1042,9 +1042,9 @@ int gpk_bgr_scores_tiled(gpk_grid* G, int radius, real* res, real* best, const u
 }
 
 // Projection on pair bitmaps for the radii ceil(3 s) of the velocity kernel (s =
-// clamp(0.375 sigma, 0.85, 3) in 3-D, 0.85 in 2-D: radii 3 to 9, and 3); -1
-// where the halo does not fit in shared memory (FP64 at R = 9: the per-cell
-// kernel runs).  Kind 3 keeps the pair-compare tiles at R = 3 (comparison runs).
+// clamp(0.375 sigma, 0.85, 3) in 3-D, 0.85 in 2-D: radii 3 to 9, and 3); -1 for
+// other radii (the per-cell kernel runs).  Kind 3 keeps the pair-compare tiles at
+// R = 3 (comparison runs).
 template <typename real, int R>
 static int projection_r(gpk_grid* G) {
     if constexpr (R == 3) {

@@ -63,3 +63,15 @@ def test_lamellar(call):
     g = sweep.lamellar_grid(5000)[0]
     g.step_n(1)
     _check(g, lambda: getattr(g, call)(6), 48)
+
+
+@pytest.mark.parametrize("precision,real", [("f32", "float"), ("f64", "double")])
+@pytest.mark.parametrize("sigma,radius", [(1.5, 3), (3.0, 4), (4.0, 5), (5.0, 6), (6.0, 7), (7.0, 8), (8.0, 9)])
+def test_projection_on_bitmaps(sigma, radius, precision, real):
+    """Every projection radius runs on pair bitmaps, in both precisions."""
+    g = GPKGrid(30, 34, 41, 1.0, thermo.isotropic(1.0, 1.0), 0.0, sigma, precision=precision)
+    g.set("phi", voronoi(30, 34, 41, 14, 8)[0])
+    g.set("alpha", 1.0)
+    names = [n for n in _profiled(g.step) if "k_projection" in n]
+    assert len(names) == 1 and f"k_projection_bits<{real}, true, {radius}>" in names[0], names
+    g.close()
