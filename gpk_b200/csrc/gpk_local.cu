@@ -291,10 +291,6 @@ __device__ __forceinline__ int rsum_index(int r2) {
     case 8: return 5; case 9: return 6; case 10: return 7; case 13: return 8; default: return 9;
     }
 }
-__host__ __device__ constexpr int rsum_value(int k) {
-    return k == 0 ? 0 : k == 1 ? 1 : k == 2 ? 2 : k == 3 ? 4 : k == 4 ? 5 : k == 5 ? 8 : k == 6 ? 9 : k == 7 ? 10
-           : k == 8 ? 13 : 18;
-}
 
 // the hash slot of label v, inserting it when absent (-1: table full)
 __device__ __forceinline__ int label_slot_insert(int32_t* keys, int32_t v, int nslot) {

@@ -149,66 +149,11 @@ __device__ __forceinline__ int topological_number(const Dims& D, const Lab& lab,
 // ---------------------------------------------------------------------------
 // 5^d bounded branch connectivity (src/gpk_connectivity.cpp:124-173)
 // ---------------------------------------------------------------------------
-typedef unsigned __int128 u128;
-
-__device__ __forceinline__ u128 bit128(int b) { return ((u128)1) << b; }
-
-template <class Lab>
-__device__ __forceinline__ bool bounded_branches_connected(const Dims& D, const Lab& lab, int cell, int32_t label,
-                                                           bool exclude_centre) {
-    int z0, y0, x0;
-    D.decode(cell, z0, y0, x0);
-    const bool is3d = D.is3d();
-    const int zcount = is3d ? 5 : 1, zc = is3d ? 2 : 0;
-    const int centre = zc * 25 + 12;
-    u128 occ = 0;
-    u128 lx0 = 0, lx4 = 0, ly0 = 0, ly4 = 0;
-    for (int lz = 0; lz < zcount; ++lz) {
-        const int z = is3d ? wrap_any(z0 + lz - 2, D.Nz) : z0;
-        for (int ly = 0; ly < 5; ++ly) {
-            const int y = wrap_any(y0 + ly - 2, D.Ny);
-            for (int lx = 0; lx < 5; ++lx) {
-                const int x = wrap_any(x0 + lx - 2, D.Nx);
-                const int b = lz * 25 + ly * 5 + lx;
-                if (lab(D.idx(z, y, x)) == label) occ |= bit128(b);
-                if (lx == 0) lx0 |= bit128(b);
-                if (lx == 4) lx4 |= bit128(b);
-                if (ly == 0) ly0 |= bit128(b);
-                if (ly == 4) ly4 |= bit128(b);
-            }
-        }
-    }
-    if (exclude_centre) occ &= ~bit128(centre);
-    const int branch_bit[6] = {centre - 1, centre + 1, centre - 5, centre + 5, centre - 25, centre + 25};
-    const int nf = D.nface();
-    int branches[6], nb = 0;
-    for (int k = 0; k < nf; ++k)
-        if (occ & bit128(branch_bit[k])) branches[nb++] = branch_bit[k];
-    if (nb <= 1) return true;
-    const u128 all = is3d ? ((((u128)1) << 125) - 1) : ((((u128)1) << 25) - 1);
-    u128 comp = bit128(branches[0]);
-    for (;;) {
-        u128 r = comp;
-        r |= (comp << 1) & ~lx0;
-        r |= (comp >> 1) & ~lx4;
-        r |= (comp << 5) & ~ly0;
-        r |= (comp >> 5) & ~ly4;
-        if (is3d) { r |= (comp << 25); r |= (comp >> 25); }
-        r &= all & occ;
-        if (r == comp) break;
-        comp = r;
-    }
-    for (int k = 1; k < nb; ++k)
-        if (!(comp & bit128(branches[k]))) return false;
-    return true;
-}
-
-// The same two tests from a 5^d occupancy mask already gathered as ballots
-// (bit b = lz*25 + ly*5 + lx, lz = 0 in 2-D): the topological number of the
-// inner 3^d box (centre removed) and the bounded branch connectivity.  The
-// mask is held as planes of 25 bits, all shifts and masks compile-time
-// constants (with the dimension a run-time value, 128-bit shifts in loops took
-// a lane thousands of cycles).
+// From a 5^d occupancy mask gathered as ballots (bit b = lz*25 + ly*5 + lx,
+// lz = 0 in 2-D): the topological number of the inner 3^d box (centre removed)
+// and the bounded branch connectivity.  The mask is held as planes of 25 bits,
+// all shifts and masks compile-time constants (with the dimension a run-time
+// value, 128-bit shifts in loops took a lane thousands of cycles).
 template <bool IS3D>
 struct Box5 {
     static constexpr int NP = IS3D ? 5 : 1, PC = IS3D ? 2 : 0;
@@ -458,19 +403,9 @@ __device__ __forceinline__ void cross_commit(const CrossArgs& a, int k, int4 ci,
     a.cres[k] = accept ? 2 : 1;
 }
 
-// Exact count of `label` at candidate k's serial time; every earlier
-// candidate touching the label has been decided.
-__device__ int serial_count(const CrossArgs& a, int k, int32_t label) {
-    int c = a.count0[label];
-    for (int j = 0; j < k; ++j) {
-        if (a.cres[j] != 2) continue;
-        const int4 cj = a.cinfo[j];
-        c += (cj.z == label) - (cj.y == label);
-    }
-    return c;
-}
-
-// The same count with the 32 lanes of a warp splitting the earlier candidates.
+// Exact count of `label` at candidate k's serial time (every earlier candidate
+// touching the label has been decided), the lanes of a warp splitting the
+// earlier candidates.
 __device__ int warp_serial_count(const CrossArgs& a, int k, int32_t label) {
     const int lane = threadIdx.x & 31;
     int c = 0;
@@ -1529,10 +1464,6 @@ __global__ void k_topology_simple_move(Dims D, const int32_t* __restrict__ phi, 
         }
     }
     *out = r ? 1 : 0;
-}
-
-__global__ void k_fill_i32(int32_t* p, int n, int32_t v) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
 }
 
 // ---------------------------------------------------------------------------
