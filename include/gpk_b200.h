@@ -317,8 +317,11 @@ int gpk_grid_set_solid_diffusivity_ratio(gpk_grid* grid, double ratio);
  * gpk_grid_step_graph returns GPK_ERR_UNSUPPORTED_MODEL otherwise.       */
 int gpk_grid_step_graph(gpk_grid* grid, int n, double dt, double dt_cap, double* time_out);
 /* Height of the 2-D geometry tiles at kernel radius 8 (sigma 1.5): the
- * tile's 32 rows divided by 1, 2 or 4 (512, 256 or 128 cells per CTA).  Results do not depend on it; small grids get more CTAs from
- * smaller tiles.  gpk_batch_autotune_tiles picks it per instance size.     */
+ * tile's 32 rows divided by 1, 2 or 4 (512, 256 or 128 cells per CTA).
+ * Results do not depend on it.  1, the default, is the fastest from 256^2
+ * cells on (512^2: 47, 49 and 57 us; 2048^2: 180, 222 and 322) and in sweeps
+ * of any size; at 64^2 and 128^2 the three differ by 2 us of 40.
+ * gpk_batch_autotune_tiles picks it per instance size.                     */
 int gpk_grid_set_tile_rows(gpk_grid* grid, int divisor);
 int gpk_grid_graph_supported(gpk_grid* grid, int* supported);
 
